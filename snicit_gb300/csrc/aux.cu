@@ -62,19 +62,21 @@ void launch_sum_piece_counts(const int32_t* piece_counts, int pieces, int stride
 }
 
 __global__ void begin_rows_kernel(const int32_t* nrows, int32_t* list, int32_t* count,
-                                  int32_t* zero_a, int32_t* zero_b, int32_t* neg) {
+                                  int32_t* zero_a, int32_t* zero_b, int32_t* zero_c,
+                                  int32_t* neg) {
   const int n = *nrows;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     list[i] = i;
     if (zero_a) zero_a[i] = 0;
     if (zero_b) zero_b[i] = 0;
+    if (zero_c) zero_c[i] = 0;
     if (neg) neg[i] = -1;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) *count = n;
 }
 void launch_begin_rows(const int32_t* nrows, int32_t* list, int32_t* count, int32_t* zero_a,
-                       int32_t* zero_b, int32_t* neg, cudaStream_t s) {
-  begin_rows_kernel<<<264, 256, 0, s>>>(nrows, list, count, zero_a, zero_b, neg);
+                       int32_t* zero_b, int32_t* zero_c, int32_t* neg, cudaStream_t s) {
+  begin_rows_kernel<<<264, 256, 0, s>>>(nrows, list, count, zero_a, zero_b, zero_c, neg);
 }
 
 __global__ void zero_rows_kernel(const int32_t* nrows, int32_t* a, int32_t* b) {

@@ -39,6 +39,7 @@ struct DevLayer {
   uint2* idx = nullptr;
   float4* val = nullptr;
   int32_t* grp = nullptr;
+  int2* lists = nullptr;  // per (group, chunk): first block, slots up to the last edge
   float* bias = nullptr;
   float* sums = nullptr;  // layer 0 with one common value: w added k times, k < 128
   // transposed layer for the sparse residue update: out-edges of every input
@@ -138,8 +139,9 @@ struct sdnn_engine {
   int32_t* d_rlist[2] = {nullptr, nullptr};
   int32_t* d_counts = nullptr;   // [L + 2]
   int32_t* d_rcounts = nullptr;  // [L + 2]
-  uint32_t* d_tmask = nullptr;
+  uint32_t* d_tmask = nullptr;   // tile masks and tickets of the chunked binary layer 0
   int32_t* d_ticket = nullptr;
+  int32_t* d_stamp = nullptr;    // [cap] marks of the layer launches that listed a row
   int32_t* d_clist = nullptr;
   int32_t* d_ccount = nullptr;
   int32_t* d_cand = nullptr;
@@ -273,6 +275,7 @@ void free_weights(sdnn_engine* e) {
     dfree(d.idx);
     dfree(d.val);
     dfree(d.grp);
+    dfree(d.lists);
     dfree(d.bias);
     dfree(d.sums);
     dfree(d.tr_off);
@@ -293,6 +296,7 @@ void free_buffers(sdnn_engine* e) {
   dfree(e->d_rcounts);
   dfree(e->d_tmask);
   dfree(e->d_ticket);
+  dfree(e->d_stamp);
   dfree(e->d_clist);
   dfree(e->d_ccount);
   dfree(e->d_cand);
@@ -412,6 +416,9 @@ int choose_kernel(sdnn_engine* e) {
     const size_t smem = (size_t)k.T * (size_t)(e->Q + 32) * 4;
     if (smem > kMaxSmem) continue;
     if (!layer_instance_exists(k)) continue;
+    // a tile that leaves room for one CTA per SM wants all its warps: 6000 rows
+    // of 16384 neurons took 832 us with 512 threads (T = 2), 572 with 1024 (T = 3)
+    if (e->cfg.threads == 0 && k.kg == 1) threads = smem > kMaxSmem / 2 ? 1024 : 512;
     LayerKernelKey kc = k, kg = k;
     kc.constw = true;
     kg.constw = false;
@@ -460,6 +467,7 @@ int ensure_buffers(sdnn_engine* e, int64_t rows) {
   T(A(&e->d_rcounts, (size_t)(e->L + 4) * 4));
   T(A(&e->d_tmask, (size_t)(cap + 1) * 4));
   T(A(&e->d_ticket, (size_t)(cap + 1) * 4));
+  T(A(&e->d_stamp, (size_t)cap * 4));
   T(A(&e->d_clist, (size_t)K * 4));
   T(A(&e->d_ccount, 16));
   T(A(&e->d_cand, (size_t)K * 4));
@@ -643,10 +651,27 @@ int upload_layer(sdnn_engine* e, int l, const PackedView& p, std::string& err) {
   };
   T(cudaMalloc((void**)&d.idx, std::max<size_t>(nslot * 2, 16)));
   T(cudaMalloc((void**)&d.grp, ngrp * 4));
+  // slots in use of every list: its last block of 4 is rarely full
+  std::vector<int2> lists(ngrp - 1);
+  for (size_t i = 0; i + 1 < ngrp; ++i) {
+    const int32_t first = p.grp_blk[i];
+    int32_t slots = (p.grp_blk[i + 1] - first) * 4;
+    for (; slots > 0; --slots) {
+      const uint16_t* lane0 = p.idx + (size_t)(first + (slots - 1) / 4) * 128 + (slots - 1) % 4;
+      bool used = false;
+      for (int lane = 0; lane < 32 && !used; ++lane)
+        used = lane0[lane * 4] / (slot_index_in_bytes(e->Q) ? 4 : 1) < e->Q;
+      if (used) break;
+    }
+    lists[i] = make_int2(first, slots);
+  }
+  T(cudaMalloc((void**)&d.lists, lists.size() * sizeof(int2)));
   if (!p.constw) T(cudaMalloc((void**)&d.val, std::max<size_t>(nslot * 4, 16)));
   if (p.bias) T(cudaMalloc((void**)&d.bias, (size_t)e->N * 4));
   if (rc == cudaSuccess && nslot) T(cudaMemcpy(d.idx, p.idx, nslot * 2, cudaMemcpyHostToDevice));
   if (rc == cudaSuccess) T(cudaMemcpy(d.grp, p.grp_blk, ngrp * 4, cudaMemcpyHostToDevice));
+  if (rc == cudaSuccess)
+    T(cudaMemcpy(d.lists, lists.data(), lists.size() * sizeof(int2), cudaMemcpyHostToDevice));
   if (rc == cudaSuccess && d.val && nslot)
     T(cudaMemcpy(d.val, p.val, nslot * 4, cudaMemcpyHostToDevice));
   if (rc == cudaSuccess && p.bias) {
@@ -860,6 +885,7 @@ int finalize_weights(sdnn_engine* e) {
       table[l].idx = d.idx;
       table[l].val = d.val;
       table[l].grp_blk = d.grp;
+      table[l].lists = d.lists;
       table[l].bias_vec = d.bias;
       table[l].bias = e->cfg.bias;
       table[l].wconst = d.wconst;
@@ -891,6 +917,7 @@ int layer_launch(sdnn_engine* e, int l, int epi, const float* in, float* out, co
   a.w.idx = d.idx;
   a.w.val = d.val;
   a.w.grp_blk = d.grp;
+  a.w.lists = d.lists;
   a.w.bias_vec = d.bias;
   a.w.bias = e->cfg.bias;
   a.w.wconst = d.wconst;
@@ -900,8 +927,8 @@ int layer_launch(sdnn_engine* e, int l, int epi, const float* in, float* out, co
   a.count_in = cin;
   a.list_out = lout;
   a.count_out = cout;
-  a.tile_mask = e->d_tmask;
-  a.tile_ticket = e->d_ticket;
+  a.stamp = e->d_stamp;
+  a.stamp_id = l + 1;
   a.pre_out = e->d_pre;
   a.pre_in = e->d_pre;
   a.cslot = e->d_cslot;
@@ -1102,7 +1129,8 @@ int enqueue(sdnn_engine* e, int phase, int64_t rows, const float* d_in, int32_t*
     if (e->pipe_start == 0) {
       if ((rc = record(e, 0, capturing))) return rc;
       CK(cudaMemsetAsync(e->d_counts, 0, (size_t)(L + 4) * 4, s));
-      launch_begin_rows(e->d_rows, e->d_list[0], e->d_counts, d_flags, e->d_state, e->d_alias, s);
+      launch_begin_rows(e->d_rows, e->d_list[0], e->d_counts, d_flags, e->d_state, e->d_stamp,
+                        e->d_alias, s);
       e->launches++;
     }
     if ((rc = enqueue_plain_layers(e, d_in, T, capturing))) return rc;
@@ -1947,7 +1975,8 @@ int run_streamed(sdnn_engine* e, const float* Y0, int64_t n, int m, int P) {
   CK(cudaMemsetAsync(e->d_counts, 0, (size_t)(e->L + 4) * 4, s));
   CK(cudaMemsetAsync(e->d_pcounts, 0, (size_t)P * (e->L + 2) * 4, s));  // the layers append
   // identity rows into the pieces' layer-0 lists
-  launch_begin_rows(e->d_rows, e->d_plist[0], e->d_counts, e->d_flags, e->d_state, e->d_alias, s);
+  launch_begin_rows(e->d_rows, e->d_plist[0], e->d_counts, e->d_flags, e->d_state, e->d_stamp,
+                    e->d_alias, s);
   e->launches += 2;
   // two lanes: even and odd pieces
   const bool two = true;
@@ -2383,6 +2412,7 @@ int engine_layer_setup(sdnn_engine* e, int layer, LayerArgs* a, LayerKernelKey* 
   a->w.idx = d.idx;
   a->w.val = d.val;
   a->w.grp_blk = d.grp;
+  a->w.lists = d.lists;
   a->w.bias_vec = d.bias;
   a->w.bias = e->cfg.bias;
   a->w.wconst = d.wconst;

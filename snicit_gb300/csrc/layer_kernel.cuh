@@ -13,7 +13,7 @@
 //    (cp.async.bulk + mbarrier) of the T input rows (or one input chunk of
 //    them) into shared memory, row stride RS = chunk + 32 floats; the last 32
 //    floats of every row are zero and serve the padding slots;
-//  * warp w takes output groups of 32 neurons, lane i owns output 32g+i and
+//  * a warp takes output groups of 32 neurons, lane i owns output 32g+i and
 //    keeps T accumulators in registers (one per row of the tile);
 //  * the in-edges of a group are pre-arranged into slots whose 32 indices hit
 //    32 distinct banks, so every shared load of a slot is one wavefront;
@@ -21,7 +21,7 @@
 //    time, so results are bitwise reproducible (no atomics on values);
 //  * bias + ReLU + clamp (or the residue update) are fused in the epilogue;
 //    the CTA compacts surviving rows into the next row list with one atomic
-//    per tile (a ticket when several CTAs share a tile).
+//    per tile (and a mark per row when several CTAs share a tile).
 #pragma once
 #include "sdnn_internal.h"
 
@@ -79,33 +79,123 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
 __device__ __forceinline__ float clampf(float v, float hi) { return fminf(hi, fmaxf(0.f, v)); }
 
 
-// Applies NB blocks of slots (indices in iv, values in vv) to acc[T].
+// Adds one slot (index j of the packed word, weight w) to acc[T].
+template <int T, int RSW>
+__device__ __forceinline__ void apply_slot(float (&acc)[T], uint32_t j, float w,
+                                           const float* __restrict__ ys, int RS) {
+  // byte offset or float index, fixed by the packer for this row stride
+  const float* p = rsw_in_bytes(RSW)
+                       ? reinterpret_cast<const float*>(reinterpret_cast<const char*>(ys) + j)
+                       : ys + j;
+#pragma unroll
+  for (int t = 0; t < T; ++t) {
+    const int off = (RSW > 0 ? RSW : RS) * t;
+    acc[t] = fmaf(w, p[off], acc[t]);
+  }
+}
+
+// Applies the first n slots of a block (1 <= n <= 4, the same for the whole
+// warp); n is a compile-time 4 for full blocks.
+template <int T, int RSW, bool CONSTW>
+__device__ __forceinline__ void apply_block(float (&acc)[T], uint2 iv, const float4& vv, float wc,
+                                            const float* __restrict__ ys, int RS, int n) {
+  apply_slot<T, RSW>(acc, iv.x & 0xffffu, CONSTW ? wc : vv.x, ys, RS);
+  if (n > 1) apply_slot<T, RSW>(acc, iv.x >> 16, CONSTW ? wc : vv.y, ys, RS);
+  if (n > 2) apply_slot<T, RSW>(acc, iv.y & 0xffffu, CONSTW ? wc : vv.z, ys, RS);
+  if (n > 3) apply_slot<T, RSW>(acc, iv.y >> 16, CONSTW ? wc : vv.w, ys, RS);
+}
+
+// Blocks of a list held in registers ahead of their use (per lane 2 registers
+// a block, 4 more for per-edge values).
+template <int T, bool CONSTW>
+constexpr int kAhead = CONSTW ? (T <= 8 ? 4 : 2) : (T <= 4 ? 2 : 1);
+
+// The groups gbeg + warp, + nwarps, ... below gend of a tile in shared memory:
+// accumulates each group's list and hands (acc, group) to done().  The slot
+// lists are walked as one stream: a block's registers are refilled with the
+// block NB further on -- of this group or the next -- as soon as it has been
+// applied, so a warp never waits for a round trip to L2 between batches or
+// groups (the kernel before this one did, and shared memory stood idle a
+// quarter of the time).  A list ends at its last used slot, not at the end of
+// its last block of 4 (1.5 of 38 slots).
+template <int T, int RSW, bool CONSTW, typename Done>
+__device__ __forceinline__ void walk_groups(const LayerDev& wl, const float* __restrict__ ys, int RS,
+                                            int gbeg, int gend, int warp, int nwarps, int lane,
+                                            Done done) {
+  constexpr int NB = kAhead<T, CONSTW>;
+  const float wc = wl.wconst;
+  const uint2* __restrict__ idx = wl.idx + lane;
+  const float4* __restrict__ val = CONSTW ? nullptr : wl.val + lane;
+  for (int base = gbeg + warp; base < gend; base += 32 * nwarps) {
+    // lane i holds the list (first block, slots) of the warp's i-th group
+    int2 mine = make_int2(0, 0);
+    if (base + lane * nwarps < gend) mine = __ldg(wl.lists + base + lane * nwarps);
+    const int n = min(32, (gend - base + nwarps - 1) / nwarps);
+    int b = __shfl_sync(0xffffffffu, mine.x, 0), slots = __shfl_sync(0xffffffffu, mine.y, 0);
+    uint2 iv[NB];
+    float4 vv[CONSTW ? 1 : NB];
+#pragma unroll
+    for (int k = 0; k < NB; ++k) {
+      if (4 * k < slots) {
+        iv[k] = __ldg(idx + (size_t)(b + k) * 32);
+        if constexpr (!CONSTW) vv[k] = __ldg(val + (size_t)(b + k) * 32);
+      }
+    }
+    for (int i = 0; i < n; ++i) {
+      float acc[T];
+#pragma unroll
+      for (int t = 0; t < T; ++t) acc[t] = 0.f;
+      bool last;
+      do {
+        last = slots <= 4 * NB;
+        // where the refills come from: the rest of this list, or the next one
+        const int fb = last ? __shfl_sync(0xffffffffu, mine.x, (i + 1) & 31) : b + NB;
+        int fs = slots - 4 * NB;
+        if (last) fs = i + 1 < n ? __shfl_sync(0xffffffffu, mine.y, (i + 1) & 31) : 0;
+        if (slots >= 4 * NB) {  // a whole batch: one straight run of gathers
+#pragma unroll
+          for (int k = 0; k < NB; ++k) {
+            apply_block<T, RSW, CONSTW>(acc, iv[k], vv[CONSTW ? 0 : k], wc, ys, RS, 4);
+            if (4 * k < fs) {
+              iv[k] = __ldg(idx + (size_t)(fb + k) * 32);
+              if constexpr (!CONSTW) vv[k] = __ldg(val + (size_t)(fb + k) * 32);
+            }
+          }
+        } else {
+          const int full = slots >> 2, part = slots & 3;
+          uint2 ti = iv[0];
+          float4 tv = vv[0];
+#pragma unroll
+          for (int k = 0; k < NB; ++k) {
+            if (k > 0 && k == full) {
+              ti = iv[k];
+              if constexpr (!CONSTW) tv = vv[k];
+            }
+            if (k < full)
+              apply_block<T, RSW, CONSTW>(acc, iv[k], vv[CONSTW ? 0 : k], wc, ys, RS, 4);
+            if (4 * k < fs) {
+              iv[k] = __ldg(idx + (size_t)(fb + k) * 32);
+              if constexpr (!CONSTW) vv[k] = __ldg(val + (size_t)(fb + k) * 32);
+            }
+          }
+          if (part) apply_block<T, RSW, CONSTW>(acc, ti, tv, wc, ys, RS, part);
+        }
+        b = fb;
+        slots = fs;
+      } while (!last);
+      done(acc, base + i * nwarps);
+    }
+  }
+}
+
+// Applies one block of slots of an input chunk to acc[T].
 template <int T, int RSW, bool CONSTW, int NB>
 __device__ __forceinline__ void apply_blocks(float (&acc)[T], const uint2 (&iv)[NB],
                                              const float4 (&vv)[CONSTW ? 1 : NB], float wc,
                                              const float* __restrict__ ys, int RS) {
 #pragma unroll
-  for (int k = 0; k < NB; ++k) {
-    const uint32_t words[2] = {iv[k].x, iv[k].y};
-    float wv[4];
-    if constexpr (!CONSTW) {
-      wv[0] = vv[k].x; wv[1] = vv[k].y; wv[2] = vv[k].z; wv[3] = vv[k].w;
-    }
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const uint32_t j = (words[s >> 1] >> ((s & 1) * 16)) & 0xffffu;
-      // byte offset or float index, fixed by the packer for this row stride
-      const float* p = rsw_in_bytes(RSW)
-                           ? reinterpret_cast<const float*>(reinterpret_cast<const char*>(ys) + j)
-                           : ys + j;
-      const float w = CONSTW ? wc : wv[s];
-#pragma unroll
-      for (int t = 0; t < T; ++t) {
-        const int off = (RSW > 0 ? RSW : RS) * t;
-        acc[t] = fmaf(w, p[off], acc[t]);
-      }
-    }
-  }
+  for (int k = 0; k < NB; ++k)
+    apply_block<T, RSW, CONSTW>(acc, iv[k], vv[CONSTW ? 0 : k], wc, ys, RS, 4);
 }
 
 // Loads NB blocks starting at block b (indices and, for general layers, values).
@@ -117,42 +207,6 @@ __device__ __forceinline__ void load_blocks(uint2 (&iv)[NB], float4 (&vv)[CONSTW
   for (int k = 0; k < NB; ++k) {
     iv[k] = __ldg(ip + (size_t)(b + k) * 32);
     if constexpr (!CONSTW) vv[k] = __ldg(vp + (size_t)(b + k) * 32);
-  }
-}
-
-// Accumulates the in-edges of group g from input chunk q into acc[T].
-// Slot blocks are fetched in batches of 8, then 2, then 1 (no predicated
-// tail): all indices of a batch are in registers before the first is used,
-// so a warp waits for one memory round trip per batch (the post-threshold
-// launches have one warp per group and nothing else to hide that latency).
-template <int T, int RSW, bool CONSTW>
-__device__ __forceinline__ void accumulate_group(float (&acc)[T], const LayerDev& wl, int nq,
-                                                 const float* __restrict__ ys, int RS, int g,
-                                                 int q, int lane) {
-  const int32_t b0 = __ldg(wl.grp_blk + g * nq + q);
-  const int32_t b1 = __ldg(wl.grp_blk + g * nq + q + 1);
-  const uint2* __restrict__ ip = wl.idx + (size_t)b0 * 32 + lane;
-  const float4* __restrict__ vp = CONSTW ? nullptr : wl.val + (size_t)b0 * 32 + lane;
-  const float wc = wl.wconst;
-  const int nb = b1 - b0;
-  int b = 0;
-  for (; b + 8 <= nb; b += 8) {
-    uint2 iv[8];
-    float4 vv[CONSTW ? 1 : 8];
-    load_blocks<CONSTW, 8>(iv, vv, ip, vp, b);
-    apply_blocks<T, RSW, CONSTW, 8>(acc, iv, vv, wc, ys, RS);
-  }
-  for (; b + 2 <= nb; b += 2) {
-    uint2 iv[2];
-    float4 vv[CONSTW ? 1 : 2];
-    load_blocks<CONSTW, 2>(iv, vv, ip, vp, b);
-    apply_blocks<T, RSW, CONSTW, 2>(acc, iv, vv, wc, ys, RS);
-  }
-  if (b < nb) {
-    uint2 iv[1];
-    float4 vv[1];
-    load_blocks<CONSTW, 1>(iv, vv, ip, vp, b);
-    apply_blocks<T, RSW, CONSTW, 1>(acc, iv, vv, wc, ys, RS);
   }
 }
 
@@ -228,8 +282,9 @@ __device__ __forceinline__ void accumulate_chunk(float (&acc)[KG][T], const Laye
   }
 }
 
-// Epilogue of one group for the rows of the tile; returns the row mask of
-// rows flagged by this warp (alive for PLAIN, non-empty for RESIDUE).
+// Epilogue of one group for the rows of the tile; returns this lane's mask of
+// flagged rows (alive for PLAIN, non-empty for RESIDUE), merged over the warp
+// once per tile.
 template <int T>
 __device__ __forceinline__ uint32_t epilogue_group(const float (&acc)[T], const LayerArgs& a,
                                                    const int32_t* s_rows, int nrows, int g,
@@ -243,25 +298,22 @@ __device__ __forceinline__ uint32_t epilogue_group(const float (&acc)[T], const 
     if (t < nrows) {
       const int row = s_rows[t];
       float* dst = a.y_out + (size_t)row * a.N + c;
-      bool flag;
       if (a.epi == EPI_PLAIN) {
         const float v = acc[t] + bc;
         *dst = clampf(v, hi);
-        flag = v > 0.f;
+        if (v > 0.f) m |= 1u << t;
       } else if (a.epi == EPI_CENTROID) {
         const int k = a.cslot[row];
         const float v = acc[t] + bc;
         a.pre_out[(size_t)k * a.N + c] = v;
         *dst = clampf(v, hi);
-        flag = false;
       } else {
         const int k = a.cslot[row];
         const float pc = __ldg(a.pre_in + (size_t)k * a.N + c);
         const float y = clampf(pc + acc[t], hi) - clampf(pc, hi);
         *dst = y;
-        flag = y != 0.f;
+        if (y != 0.f) m |= 1u << t;
       }
-      if (__any_sync(0xffffffffu, flag)) m |= 1u << t;
     }
   }
   return m;
@@ -282,7 +334,190 @@ __device__ __forceinline__ void load_tile(const LayerArgs& a, float* buf, int RS
   }
 }
 
-// Work split shared by all CTAs of a launch (same count, same grid).
+// Appends the rows of a finished piece of a tile that are flagged in m to the
+// next list (called by one warp).  When other CTAs hold the tile's other
+// groups, a row may be found by several of them: the first to put this
+// launch's mark on the row appends it (a.stamp; marks differ between the
+// launches of an inference and are cleared at its start).
+__device__ __forceinline__ void publish_rows(const LayerArgs& a, uint32_t m, bool shared,
+                                             const int32_t* rows, int lane) {
+  if (a.epi == EPI_CENTROID || m == 0) return;
+  bool mine = (m >> lane) & 1u;
+  const int row = mine ? rows[lane] : 0;
+  if (shared && mine) mine = atomicExch(a.stamp + row, a.stamp_id) != a.stamp_id;
+  const uint32_t w = __ballot_sync(0xffffffffu, mine);
+  if (!w) return;
+  int at = 0;
+  if (lane == 0) at = atomicAdd(a.count_out, __popc(w));
+  at = __shfl_sync(0xffffffffu, at, 0) + __popc(w & ((1u << lane) - 1u));
+  if (mine) a.list_out[at] = row;
+}
+
+// ---------------------------------------------------------------------------
+// Whole rows in shared memory (N <= 32768).
+//
+// Split of the work: the tiles' groups are cut into units of one group per
+// warp, and the units of all tiles, in order, are divided evenly over the
+// CTAs, so a CTA gets a contiguous run of units that may begin and end inside
+// a tile.  With one item per (tile, part) the last wave was nearly empty for
+// row counts between the grid's size and a few times that: 329 rows of 16384
+// neurons took two rounds of half-tile items, 104 us, for 21 us of gathers.
+// With fewer units than CTAs the tiles are cut finer, at most one piece per
+// CTA.  Small row counts use smaller tiles (TE < T): what bounds them is the
+// time to fetch rows and lists, which the CTAs then share.
+struct Cut {
+  int count, TE, unit, per_tile;  // rows, rows per tile, groups per unit, units per tile
+  long long units;
+};
+// Largest tile size <= T, then halved from the power of 2 below it, that
+// still gives every CTA a unit.
+template <int T>
+__device__ __forceinline__ Cut make_cut(int count, int G, int nwarps) {
+  Cut c;
+  c.count = count;
+  c.unit = nwarps;
+  c.per_tile = (G + nwarps - 1) / nwarps;
+  c.TE = T;
+  int p2 = 1;
+  while (2 * p2 < T) p2 *= 2;
+  const long long grid = gridDim.x;
+  while (c.TE > 1 && (long long)((count + c.TE - 1) / c.TE) * c.per_tile < grid) {
+    c.TE = c.TE == T ? p2 : c.TE / 2;
+  }
+  const long long tiles = (count + c.TE - 1) / c.TE;
+  if (tiles * c.per_tile < grid && tiles > 0) {
+    const int parts = (int)(grid / tiles);
+    c.unit = (G + parts - 1) / parts;
+    c.per_tile = (G + c.unit - 1) / c.unit;
+  }
+  c.units = tiles * c.per_tile;
+  return c;
+}
+
+// One piece of a tile: groups [gbeg, gend) of the rows in shared memory.
+template <int T, int RSW, bool CONSTW>
+__device__ __forceinline__ uint32_t run_piece(const LayerArgs& a, const float* ys, int RS,
+                                              const int32_t* rows, int nrows, int gbeg, int gend,
+                                              int warp, int nwarps, int lane) {
+  uint32_t m = 0;
+  walk_groups<T, RSW, CONSTW>(a.w, ys, RS, gbeg, gend, warp, nwarps, lane,
+                              [&](const float (&acc)[T], int g) {
+                                m |= epilogue_group<T>(acc, a, rows, nrows, g, lane);
+                              });
+  return m;
+}
+// ... with the code of the smallest tile size that holds TE rows.
+template <int T, int P2, int RSW, bool CONSTW>
+__device__ __forceinline__ uint32_t run_sized(int TE, const LayerArgs& a, const float* ys, int RS,
+                                              const int32_t* rows, int nrows, int gbeg, int gend,
+                                              int warp, int nwarps, int lane) {
+  if constexpr (P2 >= 1) {
+    if (TE <= P2)
+      return run_sized<P2, P2 / 2, RSW, CONSTW>(TE, a, ys, RS, rows, nrows, gbeg, gend, warp,
+                                                nwarps, lane);
+  }
+  return run_piece<T, RSW, CONSTW>(a, ys, RS, rows, nrows, gbeg, gend, warp, nwarps, lane);
+}
+__host__ __device__ constexpr int pow2_below(int t) {
+  int p = 1;
+  while (2 * p < t) p *= 2;
+  return t > 1 ? p : 0;
+}
+
+template <int T, int RSW, bool CONSTW>
+__global__ void __launch_bounds__(1024, 1) layer_rows_kernel(const LayerArgs a) {
+  extern __shared__ __align__(128) float ys[];
+  __shared__ __align__(8) uint64_t bar;
+  __shared__ int32_t s_rows[2][32];
+  __shared__ uint32_t s_mask[2];
+  __shared__ int32_t s_fail;
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  const int RS = RSW > 0 ? RSW : a.Q + 32;
+  // Launched with programmatic stream serialization: the next launch may be
+  // scheduled now, and this one may have started before its predecessor
+  // ended -- so only CTA-local setup comes before griddepcontrol.wait, which
+  // returns once the predecessor has completed and its writes are visible.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // One tile buffer, reloaded per tile: the load of one CTA overlaps the
+  // compute of the other CTAs on the SM (up to four).
+  for (int i = tid; i < T * 32; i += blockDim.x) ys[(i >> 5) * RS + a.Q + (i & 31)] = 0.f;
+  if (tid == 0) {
+    mbar_init(&bar, 1);
+    s_mask[0] = s_mask[1] = 0;
+    s_fail = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const Cut cut = make_cut<T>(*a.count_in, a.G, nwarps);
+  const long long grid = gridDim.x;
+  const long long lo = cut.units >= grid ? cut.units * blockIdx.x / grid : (long long)blockIdx.x;
+  const long long hi = cut.units >= grid ? cut.units * (blockIdx.x + 1) / grid
+                                         : min(cut.units, (long long)blockIdx.x + 1);
+  if (lo >= hi) return;
+
+  int tile = (int)(lo / cut.per_tile), first = (int)(lo % cut.per_tile);
+  int left = (int)min(hi - lo, (long long)0x7fffffff);
+  // the row ids of the tile after the current one are fetched while it runs
+  int next_row = -1;
+  if (warp == 0 && lane < cut.TE && tile * cut.TE + lane < cut.count)
+    next_row = a.list_in[tile * cut.TE + lane];
+  uint32_t phase = 0;
+  int buf = 0;
+  bool pending = false, pending_shared = false;
+  while (left > 0) {
+    const int take = min(left, cut.per_tile - first);
+    const int nrows = min(cut.TE, cut.count - tile * cut.TE);
+    const int gbeg = first * cut.unit, gend = min(a.G, (first + take) * cut.unit);
+    __syncthreads();  // every warp is done with the previous tile
+    if (warp == 0) {
+      s_rows[buf][lane] = next_row;
+      // one lane per row issues its copies (a long row in pieces of 32 KB)
+      const uint32_t row_bytes = (uint32_t)a.Q * 4u;
+      if (lane == 0) mbar_expect_tx(&bar, row_bytes * (uint32_t)nrows);
+      __syncwarp();
+      if (lane < nrows) {
+        const char* src = reinterpret_cast<const char*>(a.y_in + (size_t)next_row * a.N);
+        char* dst = reinterpret_cast<char*>(ys + (size_t)lane * RS);
+        for (uint32_t off = 0; off < row_bytes; off += 32768u)
+          bulk_g2s(dst + off, src + off, min(32768u, row_bytes - off), &bar);
+      }
+      const int nt = tile + 1;
+      next_row = -1;
+      if (take < left && lane < cut.TE && nt * cut.TE + lane < cut.count)
+        next_row = a.list_in[nt * cut.TE + lane];
+      if (lane == 0 && !mbar_wait_bounded(&bar, phase, a.err)) s_fail = 1;
+    }
+    // the rows of the previous piece are published while this tile loads
+    if (warp == nwarps - 1 && pending) {
+      publish_rows(a, s_mask[buf ^ 1], pending_shared, s_rows[buf ^ 1], lane);
+      __syncwarp();
+      if (lane == 0) s_mask[buf ^ 1] = 0;
+    }
+    __syncthreads();
+    if (s_fail) return;
+    mbar_try_wait(&bar, phase);
+    phase ^= 1u;
+    uint32_t m = run_sized<T, pow2_below(T), RSW, CONSTW>(cut.TE, a, ys, RS, s_rows[buf], nrows,
+                                                          gbeg, gend, warp, nwarps, lane);
+    m = __reduce_or_sync(0xffffffffu, m);
+    if (lane == 0 && m) atomicOr(&s_mask[buf], m);
+    pending = true;
+    pending_shared = take < cut.per_tile;
+    left -= take;
+    first = 0;
+    ++tile;
+    buf ^= 1;
+  }
+  __syncthreads();
+  if (warp == nwarps - 1)
+    publish_rows(a, s_mask[buf ^ 1], pending_shared, s_rows[buf ^ 1], lane);
+}
+
+// ---------------------------------------------------------------------------
+// Input chunks (rows too wide for shared memory): an item is (tile, part of
+// the groups), parts sized to the registers that hold the accumulators.
 struct Split {
   int count, n_tiles, spl;
   long items;
@@ -300,53 +535,22 @@ __device__ __forceinline__ Split make_split(const LayerArgs& a) {
   return sp;
 }
 
-// Publishes the flagged rows of a finished item: straight to the next list,
-// or through the per-tile mask and ticket when several CTAs share the tile.
-template <int T>
-__device__ __forceinline__ void publish_rows(const LayerArgs& a, uint32_t m, int tile, int spl,
-                                             const int32_t* rows) {
-  if (a.epi == EPI_CENTROID) return;
-  bool emit = true;
-  if (spl > 1) {
-    atomicOr(a.tile_mask + tile, m);
-    __threadfence();
-    const int tk = atomicAdd(a.tile_ticket + tile, 1);
-    emit = (tk == spl - 1);
-    if (emit) {
-      __threadfence();
-      m = atomicExch(a.tile_mask + tile, 0u);
-      a.tile_ticket[tile] = 0;
-    }
-  }
-  if (emit && m) {
-    const int base = atomicAdd(a.count_out, __popc(m));
-    int i = 0;
-    for (int t = 0; t < T; ++t)
-      if (m & (1u << t)) a.list_out[base + i++] = rows[t];
-  }
-}
-
 template <int T, int RSW, int KG, bool CONSTW>
 // (instances with up to 8 groups per warp may run 1024 threads; 16 groups per
 // warp keep 512 so their KG x T accumulators stay in registers)
-__global__ void __launch_bounds__(KG <= 8 ? 1024 : 512) layer_kernel(const LayerArgs a) {
+__global__ void __launch_bounds__(KG <= 8 ? 1024 : 512) layer_chunk_kernel(const LayerArgs a) {
   extern __shared__ __align__(128) float ys[];
   __shared__ __align__(8) uint64_t bar[1];
   __shared__ int32_t s_rows[2][T];
   __shared__ int32_t s_next[T];
   __shared__ uint32_t s_mask, s_pmask;
-  __shared__ int32_t s_ptile, s_pbuf;
+  __shared__ int32_t s_ppending, s_pbuf;
   __shared__ int32_t s_fail;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
   const int RS = RSW > 0 ? RSW : a.Q + 32;
-  // Launched with programmatic stream serialization: the next launch may be
-  // scheduled now, and this one may have started before its predecessor
-  // ended -- so only CTA-local setup comes before griddepcontrol.wait, which
-  // returns once the predecessor has completed and its writes are visible.
+  // (programmatic stream serialization, see layer_rows_kernel)
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  // One tile buffer, reloaded per item (and input chunk): the load of one CTA
-  // overlaps the compute of the other CTAs on the SM (up to four).
   for (int i = tid; i < T * 32; i += blockDim.x) ys[(i >> 5) * RS + a.Q + (i & 31)] = 0.f;
   if (tid == 0) {
     mbar_init(&bar[0], 1);
@@ -361,20 +565,18 @@ __global__ void __launch_bounds__(KG <= 8 ? 1024 : 512) layer_kernel(const Layer
   __syncthreads();
 
   // Per item: row ids of the item after it are fetched while it runs, and the
-  // rows it flags are published (tile mask, ticket, list append: a chain of
-  // global atomics) during the next item, while the other warps already work
-  // on it -- both by the CTA's last warp (its lane 31 publishes); s_rows is
-  // double-buffered, and the pending state lives in shared memory so that it
-  // costs the compute warps no registers.
+  // rows it flags are published (a chain of global atomics) during the next
+  // item, while the other warps already work on it -- both by the CTA's last
+  // warp; s_rows is double-buffered, and the pending state lives in shared
+  // memory so that it costs the compute warps no registers.
   const bool last_warp = warp == nwarps - 1;
   auto item_row = [&](long it, int t) -> int {
     const int r0 = (int)(it / sp.spl) * T;
     return t < min(T, sp.count - r0) ? a.list_in[r0 + t] : -1;
   };
   if (last_warp && lane < T) s_next[lane] = item_row(blockIdx.x, lane);
-  if (last_warp && lane == 31) s_ptile = -1;
+  if (last_warp && lane == 31) s_ppending = 0;
   uint32_t phase = 0;
-  int loaded_tile = -1;
   int b = 0;
   for (long item = blockIdx.x; item < sp.items; item += gridDim.x, b ^= 1) {
     const int tile = (int)(item / sp.spl), part = (int)(item % sp.spl);
@@ -386,72 +588,51 @@ __global__ void __launch_bounds__(KG <= 8 ? 1024 : 512) layer_kernel(const Layer
     __syncthreads();
     if (last_warp) {
       if (lane < T && item + gridDim.x < sp.items) s_next[lane] = item_row(item + gridDim.x, lane);
-      if (lane == 31 && s_ptile >= 0) {
-        publish_rows<T>(a, s_pmask, s_ptile, sp.spl, s_rows[s_pbuf]);
-        s_ptile = -1;
-      }
+      if (s_ppending) publish_rows(a, s_pmask, sp.spl > 1, s_rows[s_pbuf], lane);
     }
     uint32_t m = 0;
-    if constexpr (KG == 1) {
-      // one buffer, whole rows (one chunk): reloaded when the tile changes
-      if (tile != loaded_tile) {
-        if (tid == 0) {
-          load_tile(a, ys, RS, s_rows[b], nrows, 0, &bar[0]);
-          s_fail = mbar_wait_bounded(&bar[0], phase, a.err) ? 0 : 1;
-        }
-        __syncthreads();
-        if (s_fail) return;
-        mbar_try_wait(&bar[0], phase);
-        phase ^= 1u;
-        loaded_tile = tile;
-      }
-      for (int g = gbeg + warp; g < gend; g += nwarps) {
-        float acc[T];
+    // accumulators of KG groups per warp live across chunks
+    float acc[KG][T];
 #pragma unroll
-        for (int t = 0; t < T; ++t) acc[t] = 0.f;
-        accumulate_group<T, RSW, CONSTW>(acc, a.w, a.nq, ys, RS, g, 0, lane);
-        m |= epilogue_group<T>(acc, a, s_rows[b], nrows, g, lane);
-      }
-    } else {
-      // input chunks (nq > 1): accumulators of KG groups per warp live across chunks
-      float acc[KG][T];
+    for (int kk = 0; kk < KG; ++kk)
 #pragma unroll
-      for (int kk = 0; kk < KG; ++kk)
-#pragma unroll
-        for (int t = 0; t < T; ++t) acc[kk][t] = 0.f;
-      for (int q = 0; q < a.nq; ++q) {
-        if (q > 0) __syncthreads();
-        if (tid == 0) {
-          load_tile(a, ys, RS, s_rows[b], nrows, q, &bar[0]);
-          s_fail = mbar_wait_bounded(&bar[0], phase, a.err) ? 0 : 1;
-        }
-        __syncthreads();
-        if (s_fail) return;
-        mbar_try_wait(&bar[0], phase);
-        phase ^= 1u;
-        accumulate_chunk<T, RSW, CONSTW, KG>(acc, a.w, a.nq, ys, RS, gbeg, gend, warp, nwarps, q,
-                                             lane);
+      for (int t = 0; t < T; ++t) acc[kk][t] = 0.f;
+    for (int q = 0; q < a.nq; ++q) {
+      if (q > 0) __syncthreads();
+      if (tid == 0) {
+        load_tile(a, ys, RS, s_rows[b], nrows, q, &bar[0]);
+        s_fail = mbar_wait_bounded(&bar[0], phase, a.err) ? 0 : 1;
       }
-#pragma unroll
-      for (int kk = 0; kk < KG; ++kk) {
-        const int g = gbeg + warp + kk * nwarps;
-        if (g < gend) m |= epilogue_group<T>(acc[kk], a, s_rows[b], nrows, g, lane);
-      }
+      __syncthreads();
+      if (s_fail) return;
+      mbar_try_wait(&bar[0], phase);
+      phase ^= 1u;
+      accumulate_chunk<T, RSW, CONSTW, KG>(acc, a.w, a.nq, ys, RS, gbeg, gend, warp, nwarps, q,
+                                           lane);
     }
+#pragma unroll
+    for (int kk = 0; kk < KG; ++kk) {
+      const int g = gbeg + warp + kk * nwarps;
+      if (g < gend) m |= epilogue_group<T>(acc[kk], a, s_rows[b], nrows, g, lane);
+    }
+    m = __reduce_or_sync(0xffffffffu, m);
     if (lane == 0 && m) atomicOr(&s_mask, m);
     __syncthreads();
     if (last_warp && lane == 31) {
       s_pmask = s_mask;
       s_mask = 0;
-      s_ptile = tile;
+      s_ppending = 1;
       s_pbuf = b;
     }
+    __syncwarp();
   }
-  if (last_warp && lane == 31 && s_ptile >= 0)
-    publish_rows<T>(a, s_pmask, s_ptile, sp.spl, s_rows[s_pbuf]);
+  if (last_warp && s_ppending) publish_rows(a, s_pmask, sp.spl > 1, s_rows[s_pbuf], lane);
 }
 
-#define SDNN_LAYER_INSTANCE(T, RSW, KG, CW) template __global__ void layer_kernel<T, RSW, KG, CW>(const LayerArgs);
+#define SDNN_ROWS_INSTANCE(T, RSW, CW) \
+  template __global__ void layer_rows_kernel<T, RSW, CW>(const LayerArgs);
+#define SDNN_CHUNK_INSTANCE(T, RSW, KG, CW) \
+  template __global__ void layer_chunk_kernel<T, RSW, KG, CW>(const LayerArgs);
 
 // Registry entry used by the dispatcher.
 struct LayerInstance {

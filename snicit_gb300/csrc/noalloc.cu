@@ -7,7 +7,7 @@
 // owned by another framework.  The engine's own inference paths allocate
 // their row buffers on first use; this entry point allocates nothing: the
 // caller passes the rows in and out, and the per-row scratch the layer kernel
-// needs (row lists, counters, per-tile masks and tickets) lives in one
+// needs (row lists, counters, a mark per row) lives in one
 // file-scope __device__ array of fixed size, kNoAllocMaxRows rows (about
 // 1 MB), held by every GPU that loads the library until the process exits.
 //
@@ -38,8 +38,7 @@ constexpr int kMaxDevices = 64;
 struct NoAllocScratch {
   int32_t list_in[kNoAllocMaxRows];
   int32_t list_out[kNoAllocMaxRows];
-  uint32_t tile_mask[kNoAllocMaxRows + 1];
-  int32_t tile_ticket[kNoAllocMaxRows + 1];
+  int32_t stamp[kNoAllocMaxRows];
   int32_t counts[4];  // [0] rows in, [1] survivors
   int32_t err[4];
 };
@@ -53,12 +52,10 @@ NoAllocScratch* g_addr[kMaxDevices] = {};
 
 // Resets the parts of the scratch that must start at zero for this call and
 // lists every row.
-__global__ void noalloc_prepare_kernel(NoAllocScratch* s, int32_t rows, int32_t tiles) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x)
+__global__ void noalloc_prepare_kernel(NoAllocScratch* s, int32_t rows) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x) {
     s->list_in[i] = i;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= tiles; i += gridDim.x * blockDim.x) {
-    s->tile_mask[i] = 0u;
-    s->tile_ticket[i] = 0;
+    s->stamp[i] = 0;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     s->counts[0] = rows;
@@ -147,16 +144,15 @@ extern "C" int sdnn_layer_noalloc(sdnn_engine* e, int32_t layer, const float* d_
   rc = scratch_address(e, &scratch);
   if (rc) return rc;
   cudaStream_t s = stream ? (cudaStream_t)stream : sdnn::engine_stream(e);
-  const int tiles = (int)((rows + key.T - 1) / key.T);
-  noalloc_prepare_kernel<<<64, 256, 0, s>>>(scratch, (int32_t)rows, tiles);
+  noalloc_prepare_kernel<<<64, 256, 0, s>>>(scratch, (int32_t)rows);
   a.y_in = d_y_in;
   a.y_out = d_y_out;
   a.list_in = scratch->list_in;
   a.count_in = &scratch->counts[0];
   a.list_out = scratch->list_out;
   a.count_out = &scratch->counts[1];
-  a.tile_mask = scratch->tile_mask;
-  a.tile_ticket = scratch->tile_ticket;
+  a.stamp = scratch->stamp;
+  a.stamp_id = 1;
   a.err = &scratch->err[0];
   cudaError_t ce = sdnn::launch_layer(key, a, grid, threads, smem, s);
   if (ce == cudaSuccess) ce = cudaMemsetAsync(d_alive, 0, (size_t)rows * sizeof(int32_t), s);
@@ -190,7 +186,7 @@ extern "C" int sdnn_selftest_noalloc_timeout(sdnn_engine* e, int32_t* d_alive, i
   rc = scratch_address(e, &scratch);
   if (rc) return rc;
   cudaStream_t s = stream ? (cudaStream_t)stream : sdnn::engine_stream(e);
-  noalloc_prepare_kernel<<<64, 256, 0, s>>>(scratch, (int32_t)rows, 0);
+  noalloc_prepare_kernel<<<64, 256, 0, s>>>(scratch, (int32_t)rows);
   cudaError_t ce = sdnn::launch_wait_selftest(&scratch->err[0], (uint64_t)limit_us * 1000ull, s);
   if (ce == cudaSuccess) ce = cudaMemsetAsync(d_alive, 0, (size_t)rows * sizeof(int32_t), s);
   if (ce == cudaSuccess) {

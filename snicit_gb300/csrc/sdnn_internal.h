@@ -27,6 +27,7 @@ struct LayerDev {
   const uint2* idx;        // [blocks][32] uint2 (4 x u16)
   const float4* val;       // [blocks][32] float4, nullptr when const_w
   const int32_t* grp_blk;  // [G*nq + 1] block offsets, entry g*nq + q
+  const int2* lists;       // [G*nq] (first block, slots up to the last edge)
   const float* bias_vec;   // [N] per-neuron bias or nullptr
   float bias;              // scalar bias when bias_vec == nullptr
   float wconst;            // common value when val == nullptr
@@ -40,8 +41,8 @@ struct LayerArgs {
   const int32_t* count_in;  // number of ids (device scalar)
   int32_t* list_out;        // surviving ids (PLAIN) / non-empty residues (RESIDUE)
   int32_t* count_out;       // device scalar, must start at 0
-  uint32_t* tile_mask;      // scratch per tile, zero between launches
-  int32_t* tile_ticket;     // scratch per tile, zero between launches
+  int32_t* stamp;           // [rows] mark of the launch that last listed the row
+  int32_t stamp_id;         // this launch's mark (> 0, unlike any other since the clearing)
   float* pre_out;           // CENTROID: [K][N] pre-activations
   const float* pre_in;      // RESIDUE:  [K][N] pre-activations of this layer
   const int32_t* cslot;     // row -> centroid slot
@@ -183,10 +184,10 @@ void launch_post_choice(const PostChoiceArgs& a, cudaGraphConditionalHandle h, c
 // (row counts of the layers run piece by piece).
 void launch_sum_piece_counts(const int32_t* piece_counts, int pieces, int stride, int layers,
                              int32_t* counts, cudaStream_t s);
-// list[i] = i, zero_a[i] = zero_b[i] = 0 and neg[i] = -1 for i < *nrows;
+// list[i] = i, zero_a[i] = zero_b[i] = zero_c[i] = 0 and neg[i] = -1 for i < *nrows;
 // *count = *nrows
 void launch_begin_rows(const int32_t* nrows, int32_t* list, int32_t* count, int32_t* zero_a,
-                       int32_t* zero_b, int32_t* neg, cudaStream_t s);
+                       int32_t* zero_b, int32_t* zero_c, int32_t* neg, cudaStream_t s);
 void launch_zero_rows(const int32_t* nrows, int32_t* a, int32_t* b, cudaStream_t s);
 void launch_copy_rows(const int32_t* nrows, const float* src, float* dst, int32_t N, cudaStream_t s);
 void launch_identify(const float* y, const int32_t* list, const int32_t* count, int32_t N,
