@@ -53,6 +53,7 @@ struct DevLayer {
   int64_t slots = 0;
   int32_t max_depth = 0;
   uint32_t chain_slice8 = 0, chain_slice16 = 0;  // largest per-CTA weight slices (chain)
+  ResidentPlan res{};  // layer kernel with the lists in tensor memory (fn null: not this layer)
 };
 
 struct GraphKey {
@@ -640,6 +641,7 @@ int upload_layer(sdnn_engine* e, int l, const PackedView& p, std::string& err) {
   d.slots = p.slots;
   d.max_depth = p.max_depth;
   if (e->nq == 1) {
+    d.res = resident_plan(e->N, p.constw, p.max_depth);
     d.chain_slice8 = chain_slice_bytes(p.grp_blk, e->G, !p.constw, 8);
     d.chain_slice16 = chain_slice_bytes(p.grp_blk, e->G, !p.constw, 16);
   }
@@ -910,6 +912,13 @@ int finalize_weights(sdnn_engine* e) {
   return SDNN_OK;
 }
 
+// Whether layer l runs on the kernel that keeps its slot lists in tensor
+// memory: wherever that kernel applies, unless the caller asked for a tile
+// shape (tile_rows, threads) of the streaming kernel.
+bool resident_on(const sdnn_engine* e, int l) {
+  return e->cfg.tile_rows == 0 && e->cfg.threads == 0 && e->dl[l].res.fn;
+}
+
 int layer_launch(sdnn_engine* e, int l, int epi, const float* in, float* out, const int32_t* lin,
                  const int32_t* cin, int32_t* lout, int32_t* cout) {
   const DevLayer& d = e->dl[l];
@@ -941,9 +950,13 @@ int layer_launch(sdnn_engine* e, int l, int epi, const float* in, float* out, co
   a.max_split = e->G;
   a.min_split = e->min_split;
   a.clampv = e->cfg.clamp;
-  LayerKernelKey k = e->key;
-  k.constw = d.constw;
-  CK(launch_layer(k, a, d.constw ? e->grid : e->grid_general, e->threads, e->smem, e->stream));
+  if (resident_on(e, l)) {
+    CK(launch_layer_resident(d.res, a, e->num_sms, e->stream));
+  } else {
+    LayerKernelKey k = e->key;
+    k.constw = d.constw;
+    CK(launch_layer(k, a, d.constw ? e->grid : e->grid_general, e->threads, e->smem, e->stream));
+  }
   e->launches++;
   return SDNN_OK;
 }
@@ -1589,6 +1602,11 @@ int prepare(sdnn_engine* e, int64_t rows) {
   }
   CK(layer_prepare(LayerKernelKey{e->key.T, e->key.rsw, e->key.kg, true}, e->smem));
   CK(layer_prepare(LayerKernelKey{e->key.T, e->key.rsw, e->key.kg, false}, e->smem));
+  if (e->nq == 1)
+    for (bool constw : {true, false}) {
+      const ResidentPlan p = resident_plan(e->N, constw, 0);
+      if (p.fn) CK(resident_prepare(p));
+    }
   if (e->sparse_built) CK(sparse_residue_prepare(e->N));
   e->bits_chunked = e->nq > 1 && !(e->cfg.flags & SDNN_FLAG_NO_BINARY_FIRST_LAYER) &&
                     layer0_bits_chunked_supported(e->N, e->Q);
@@ -1655,8 +1673,9 @@ int collect_stats(sdnn_engine* e) {
   st.weight_nnz = e->total_nnz;
   st.launches = e->launches;
   st.threshold = T;
-  st.tile_rows = e->key.T;
-  st.threads = e->threads;
+  const bool resident = resident_on(e, L - 1);
+  st.tile_rows = resident ? e->dl[L - 1].res.T : e->key.T;
+  st.threads = resident ? 512 : e->threads;
   st.input_pieces = e->last_pieces;
   st.centroid_candidates = e->cfg.num_centroids;
   st.merge_start = merging_on(e) ? (e->cfg.merge_start > 0 ? e->cfg.merge_start : kMergeStart) : 0;
@@ -2395,7 +2414,7 @@ sdnn_config engine_config(const sdnn_engine* e) { return e->cfg; }
 // launch shape, without allocating anything: the weights must already be on
 // the device (sdnn_finalize_weights or an earlier inference).
 int engine_layer_setup(sdnn_engine* e, int layer, LayerArgs* a, LayerKernelKey* key, int* grid,
-                       int* threads, size_t* smem) {
+                       int* threads, size_t* smem, ResidentPlan* res, int* num_sms) {
   if (layer < 0 || layer >= e->L) return fail(e, SDNN_ERR_INVALID, "bad layer");
   if (!e->stream || e->weights_dirty || (int)e->dl.size() != e->L)
     return fail(e, SDNN_ERR_STATE, "weights are not on the device: call sdnn_finalize_weights first");
@@ -2407,7 +2426,10 @@ int engine_layer_setup(sdnn_engine* e, int layer, LayerArgs* a, LayerKernelKey* 
   const DevLayer& d = e->dl[layer];
   LayerKernelKey k = e->key;
   k.constw = d.constw;
-  CK(layer_prepare(k, e->smem));
+  *res = resident_on(e, layer) ? d.res : ResidentPlan{};
+  *num_sms = e->num_sms;
+  if (res->fn) CK(resident_prepare(*res));
+  else CK(layer_prepare(k, e->smem));
   *a = LayerArgs{};
   a->w.idx = d.idx;
   a->w.val = d.val;

@@ -1,0 +1,431 @@
+// Layer kernel with the slot lists resident in tensor memory (N <= 4096).
+//
+// The same step, epilogues, slots and summation order as layer_rows_kernel
+// (layer_kernel.cuh): bitwise the same rows.  What bounds both is the shared
+// memory port (a gather of 32 operands is one wavefront); layer_rows_kernel
+// fetches every slot list again for every tile, through the same port: two
+// wavefronts to fill L1 and two to read a block of 4 slots, for 4 T wavefronts
+// of gathers -- 17 % at T = 6 rows of 4096 neurons, twice that with a value
+// per edge.  Here a CTA keeps its groups' lists for the whole launch in tensor
+// memory (256 KB per SM, its own read path, no use of the port), 128 columns
+// per warp, and streams row tiles past them:
+//
+//  * one CTA of 16 warps per SM; a warp owns up to 4 groups of 32 outputs (2
+//    when the layer has a value per edge: 6 bytes per slot instead of 2), deep
+//    ones and shallow ones together so that the warps stay level; layers of
+//    more groups than a CTA holds are split over `split` CTAs that read the
+//    same rows;
+//  * row tiles arrive by TMA bulk copies in a ring of stages; a warp waits for
+//    its stage's copies only, and the last warp to finish a tile lists the
+//    tile's surviving rows and reloads the stage, so no barrier ties the warps
+//    together and the copies run a few tiles ahead;
+//  * the lists are loaded before griddepcontrol.wait (weights do not depend on
+//    the previous launch), so their latency hides behind its end.
+//
+// One layer, us with lists streamed per tile (best tile) -> kept: 60000 rows of
+// 1024 neurons 334 -> 290, of 4096 1292 -> 1119 (the gathers alone need 239
+// and 956 at one wavefront per clock); 3001 rows of 4096 with values 104 -> 93.
+// The port is then 85 % busy, tile copies and stores included.
+#include <algorithm>
+#include <cstdint>
+#include "layer_kernel.cuh"
+
+namespace sdnn {
+
+namespace {
+
+constexpr int kWarps = 16;
+constexpr int kCols = 128;  // tensor memory columns of a warp
+constexpr int kMaxStages = 6;
+// groups a warp owns and the blocks of 4 slots it keeps of each: 2 words of
+// indices a block, then 4 words of values a block in general layers
+template <bool CONSTW>
+constexpr int kGroups = CONSTW ? 4 : 2;
+template <bool CONSTW>
+constexpr int kResBlocks = CONSTW ? 16 : 10;
+template <bool CONSTW>
+constexpr int kGroupCols = kCols / kGroups<CONSTW>;
+constexpr size_t kResSmem = 225 * 1024;
+
+__device__ __forceinline__ void tmem_st2(uint32_t addr, uint2 v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(v.x), "r"(v.y)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st4(uint32_t addr, float4 v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr),
+               "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)),
+               "r"(__float_as_uint(v.w))
+               : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() {
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_ld4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t (&r)[8], uint32_t addr) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+                 "=r"(r[7])
+               : "r"(addr));
+}
+// The registers of the loads before it are valid after this wait (they are
+// operands so that their uses stay behind it).
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[8]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]),
+                 "+r"(r[7])::"memory");
+}
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[4], uint32_t (&v)[8]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(v[0]), "+r"(v[1]), "+r"(v[2]),
+                 "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7])::"memory");
+}
+
+// A batch of a list in registers: 16 slots of a layer with one weight value,
+// or 8 slots and their values.
+template <bool CONSTW>
+struct Batch;
+template <>
+struct Batch<true> {
+  static constexpr int kSlots = 16;
+  uint32_t w[8];
+  // block words from column `col` on, b the first block
+  __device__ __forceinline__ void load(uint32_t col, int b) { tmem_ld8(w, col + 2 * b); }
+  __device__ __forceinline__ void wait() { tmem_wait_ld(w); }
+  __device__ __forceinline__ float val(int, float wc) const { return wc; }
+  __device__ __forceinline__ void drop(int pairs) {  // the first pairs are used up
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (k + pairs < 8) w[k] = w[k + pairs];
+  }
+};
+template <>
+struct Batch<false> {
+  static constexpr int kSlots = 8;
+  uint32_t w[4], v[8];
+  __device__ __forceinline__ void load(uint32_t col, int b) {
+    tmem_ld4(w, col + 2 * b);
+    tmem_ld8(v, col + 2 * kResBlocks<false> + 4 * b);
+  }
+  __device__ __forceinline__ void wait() { tmem_wait_ld(w, v); }
+  __device__ __forceinline__ float val(int slot, float) const { return __uint_as_float(v[slot]); }
+  __device__ __forceinline__ void drop(int pairs) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (k + pairs < 4) w[k] = w[k + pairs];
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (k + 2 * pairs < 8) v[k] = v[k + 2 * pairs];
+  }
+};
+
+template <int PAIRS, int T, int RSW, bool CONSTW>
+__device__ __forceinline__ void apply_pairs(float (&acc)[T], const Batch<CONSTW>& b, float wc,
+                                            const float* ys, int RS) {
+#pragma unroll
+  for (int k = 0; k < PAIRS; ++k) {
+    apply_slot<T, RSW>(acc, b.w[k] & 0xffffu, b.val(2 * k, wc), ys, RS);
+    apply_slot<T, RSW>(acc, b.w[k] >> 16, b.val(2 * k + 1, wc), ys, RS);
+  }
+}
+
+// acc[T] over the first `slots` slots of the list in tensor memory from column
+// `col` on.  cur holds the list's first batch on entry and that of the list at
+// `next` on return: the next batch is always on its way while one is applied.
+// The last batch is taken in runs of 8, 4, 2 and 1 slots.
+template <int T, int RSW, bool CONSTW>
+__device__ __forceinline__ void gather(float (&acc)[T], Batch<CONSTW>& cur, uint32_t col,
+                                       uint32_t next, int slots, float wc, const float* ys, int RS) {
+  constexpr int S = Batch<CONSTW>::kSlots;
+  Batch<CONSTW> nxt;
+  int b = 0;
+  while (slots > S) {
+    b += S / 4;
+    nxt.load(col, b);
+    apply_pairs<S / 2, T, RSW, CONSTW>(acc, cur, wc, ys, RS);
+    nxt.wait();
+    cur = nxt;
+    slots -= S;
+  }
+  nxt.load(next, 0);
+  if (slots == S) {
+    apply_pairs<S / 2, T, RSW, CONSTW>(acc, cur, wc, ys, RS);
+  } else {
+    if (S == 16 && (slots & 8)) {
+      apply_pairs<4, T, RSW, CONSTW>(acc, cur, wc, ys, RS);
+      cur.drop(4);
+    }
+    if (slots & 4) {
+      apply_pairs<2, T, RSW, CONSTW>(acc, cur, wc, ys, RS);
+      cur.drop(2);
+    }
+    if (slots & 2) {
+      apply_pairs<1, T, RSW, CONSTW>(acc, cur, wc, ys, RS);
+      cur.drop(1);
+    }
+    if (slots & 1) apply_slot<T, RSW>(acc, cur.w[0] & 0xffffu, cur.val(0, wc), ys, RS);
+  }
+  nxt.wait();
+  cur = nxt;
+}
+
+// Outputs of one group for a full tile in plain mode: no per-row tests.
+template <int T>
+__device__ __forceinline__ uint32_t plain_outputs(const float (&acc)[T], const LayerArgs& a,
+                                                  float* const (&dst)[T], int g, int lane) {
+  const int c = g * 32 + lane;
+  const float bc = a.w.bias_vec ? __ldg(a.w.bias_vec + c) : a.w.bias;
+  uint32_t m = 0;
+#pragma unroll
+  for (int t = 0; t < T; ++t) {
+    const float v = acc[t] + bc;
+    dst[t][c] = clampf(v, a.clampv);
+    if (v > 0.f) m |= 1u << t;
+  }
+  return m;
+}
+
+// One warp's groups over the rows of a stage; returns the lane's row mask.
+template <int T, int RSW, bool CONSTW>
+__device__ __forceinline__ uint32_t run_groups(const LayerArgs& a, const float* ys, int RS,
+                                               const int32_t* rows, int nrows, uint32_t col,
+                                               Batch<CONSTW>& cur, const int2* lists, int first_grp,
+                                               int step0, int step1, int n, int lane) {
+  constexpr int kHeld = 4 * kResBlocks<CONSTW>;
+  const bool plain = a.epi == EPI_PLAIN && nrows == T;
+  float* dst[T];
+#pragma unroll
+  for (int t = 0; t < T; ++t) dst[t] = plain ? a.y_out + (size_t)rows[t] * a.N : nullptr;
+  uint32_t m = 0;
+  int g = first_grp;
+#pragma unroll 1
+  for (int i = 0; i < n; ++i) {
+    const int2 list = lists[i];
+    float acc[T];
+#pragma unroll
+    for (int t = 0; t < T; ++t) acc[t] = 0.f;
+    const uint32_t here = col + i * kGroupCols<CONSTW>;
+    gather<T, RSW, CONSTW>(acc, cur, here, i + 1 < n ? here + kGroupCols<CONSTW> : col,
+                           min(list.y, kHeld), a.w.wconst, ys, RS);
+    // slots past the resident ones (few groups of a layer, if any)
+    for (int s = kHeld; s < list.y; s += 4) {
+      const size_t at = (size_t)(list.x + (s >> 2)) * 32 + lane;
+      const uint2 iv = __ldg(a.w.idx + at);
+      float4 vv = make_float4(0.f, 0.f, 0.f, 0.f);
+      if constexpr (!CONSTW) vv = __ldg(a.w.val + at);
+      apply_block<T, RSW, CONSTW>(acc, iv, vv, a.w.wconst, ys, RS, min(4, list.y - s));
+    }
+    m |= plain ? plain_outputs<T>(acc, a, dst, g, lane)
+               : epilogue_group<T>(acc, a, rows, nrows, g, lane);
+    g += (i & 1) ? step1 : step0;
+  }
+  return m;
+}
+
+// ... with the code of the smallest tile size that holds TE rows.
+template <int T, int RSW, bool CONSTW>
+__device__ __forceinline__ uint32_t run_stage(int TE, const LayerArgs& a, const float* ys, int RS,
+                                              const int32_t* rows, int nrows, uint32_t col,
+                                              Batch<CONSTW>& cur, const int2* lists, int first_grp,
+                                              int step0, int step1, int n, int lane) {
+  if constexpr (T > 1) {
+    if (TE <= pow2_below(T))
+      return run_stage<pow2_below(T), RSW, CONSTW>(TE, a, ys, RS, rows, nrows, col, cur, lists, first_grp,
+                                           step0, step1, n, lane);
+  }
+  return run_groups<T, RSW, CONSTW>(a, ys, RS, rows, nrows, col, cur, lists, first_grp, step0, step1,
+                                    n, lane);
+}
+
+template <int T, int RSW, bool CONSTW>
+__global__ void __launch_bounds__(kWarps * 32, 1)
+    layer_resident_kernel(const LayerArgs a, int split, int stages) {
+  extern __shared__ __align__(128) float ring[];  // [stages][T][RS]
+  __shared__ __align__(8) uint64_t full[kMaxStages];
+  __shared__ int32_t s_rows[kMaxStages][T];
+  __shared__ uint32_t s_mask[kMaxStages];
+  __shared__ int32_t s_done[kMaxStages];
+  __shared__ uint32_t s_tmem;
+  __shared__ int2 s_lists[kWarps][kGroups<CONSTW>];
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int RS = RSW > 0 ? RSW : a.Q + 32;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // ---- before the previous launch has ended: nothing it writes is read
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+                     smem_u32(&s_tmem))
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  for (int i = warp; i < T * stages; i += kWarps) ring[(size_t)i * RS + a.Q + lane] = 0.f;
+  if (tid < kMaxStages) {
+    mbar_init(&full[tid], 1);
+    s_mask[tid] = 0;
+    s_done[tid] = 0;
+  }
+  if (tid == 0) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  // the warp's columns: its quarter of the lanes, 128 of the 512 columns
+  const uint32_t tmem = s_tmem;
+  const uint32_t col = tmem + ((uint32_t)(warp & 3) << 21) + (uint32_t)(warp >> 2) * kCols;
+  const int part = blockIdx.x % split, team = blockIdx.x / split, teams = gridDim.x / split;
+  // Groups come in order of depth (degree order), so the warps take them there
+  // and back: warp w the w-th, the (31 - w)-th, the (32 + w)-th, ...
+  const int first_grp = warp * split + part;
+  const int step0 = (2 * kWarps - 1 - 2 * warp) * split, step1 = (2 * warp + 1) * split;
+  int n = 0;
+  for (int g = first_grp; n < kGroups<CONSTW> && g < a.G; ++n) {
+    const int2 list = __ldg(a.w.lists + g);
+    if (lane == 0) s_lists[warp][n] = list;
+    const int nb = min((list.y + 3) >> 2, kResBlocks<CONSTW>);
+    const size_t at = (size_t)list.x * 32 + lane;
+    const uint32_t to = col + n * kGroupCols<CONSTW>;
+#pragma unroll 4
+    for (int b = 0; b < nb; ++b) {
+      tmem_st2(to + 2 * b, __ldg(a.w.idx + at + (size_t)b * 32));
+      if constexpr (!CONSTW)
+        tmem_st4(to + 2 * kResBlocks<false> + 4 * b, __ldg(a.w.val + at + (size_t)b * 32));
+    }
+    g += (n & 1) ? step1 : step0;
+  }
+  tmem_wait_st();
+  __syncwarp();
+  Batch<CONSTW> cur;
+  cur.load(col, 0);
+  cur.wait();
+
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int count = *a.count_in;
+  // Rows per tile: as many as still give every team a tile, the last round of
+  // tiles full (TE = 1 .. T).
+  const int rounds = max(1, (int)(((long long)count + (long long)T * teams - 1) / ((long long)T * teams)));
+  const int TE = min(T, max(1, (int)(((long long)count + (long long)rounds * teams - 1) /
+                                     ((long long)rounds * teams))));
+  const int tiles = (int)(((long long)count + TE - 1) / TE);
+  const int mine = team < tiles ? (tiles - team + teams - 1) / teams : 0;
+  // Lists the rows of this CTA's k-th tile and starts their copies into stage s
+  // (one warp).
+  auto load = [&](int k, int s) {
+    const long long r0 = (long long)(team + (long long)k * teams) * TE;
+    const int nrows = (int)min((long long)TE, count - r0);
+    const int row = lane < nrows ? a.list_in[r0 + lane] : -1;
+    if (lane < T) s_rows[s][lane] = row;
+    __syncwarp();
+    const uint32_t bytes = (uint32_t)a.N * 4u;
+    if (lane == 0) mbar_expect_tx(&full[s], bytes * (uint32_t)nrows);
+    __syncwarp();
+    if (lane < nrows)
+      bulk_g2s(ring + (size_t)(s * T + lane) * RS, a.y_in + (size_t)row * a.N, bytes, &full[s]);
+  };
+  if (warp < stages && warp < mine) load(warp, warp);
+  int s = 0;
+  uint32_t phase = 0;
+  bool ok = true;
+  for (int k = 0; k < mine; ++k) {
+    ok = mbar_wait_bounded(&full[s], phase, a.err);
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) break;
+    const long long r0 = (long long)(team + (long long)k * teams) * TE;
+    const int nrows = (int)min((long long)TE, count - r0);
+    uint32_t m = run_stage<T, RSW, CONSTW>(TE, a, ring + (size_t)s * T * RS, RS, s_rows[s], nrows,
+                                           col, cur, s_lists[warp], first_grp, step0, step1, n, lane);
+    m = __reduce_or_sync(0xffffffffu, m);
+    int before = 0;
+    if (lane == 0) {
+      if (m) atomicOr(&s_mask[s], m);
+      __threadfence_block();
+      before = atomicAdd(&s_done[s], 1);
+    }
+    before = __shfl_sync(0xffffffffu, before, 0);
+    if (before == kWarps - 1) {
+      // every warp is done with the tile
+      __threadfence_block();
+      const uint32_t mask = s_mask[s];
+      publish_rows(a, mask, split > 1, s_rows[s], lane);
+      __syncwarp();
+      if (lane == 0) {
+        s_mask[s] = 0;
+        s_done[s] = 0;
+      }
+      __syncwarp();
+      if (k + stages < mine) load(k + stages, s);
+    }
+    if (++s == stages) {
+      s = 0;
+      phase ^= 1u;
+    }
+  }
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+}
+
+struct Instance {
+  int T, rsw;
+  bool constw;
+  const void* fn;
+};
+#define SDNN_RESIDENT(T, RSW) \
+  {T, RSW, true, (const void*)&layer_resident_kernel<T, RSW, true>}, \
+      {T, RSW, false, (const void*)&layer_resident_kernel<T, RSW, false>}
+const Instance kInstances[] = {SDNN_RESIDENT(8, 1056), SDNN_RESIDENT(6, 4128), SDNN_RESIDENT(8, 0),
+                               SDNN_RESIDENT(6, 0)};
+
+const void* find_instance(int T, int rsw, bool constw) {
+  for (const Instance& e : kInstances)
+    if (e.T == T && e.rsw == rsw && e.constw == constw) return e.fn;
+  return nullptr;
+}
+
+}  // namespace
+
+ResidentPlan resident_plan(int N, bool constw, int max_depth) {
+  ResidentPlan p{};
+  const int G = N / 32;
+  const int per_cta = kWarps * (constw ? kGroups<true> : kGroups<false>);
+  const int held = 4 * (constw ? kResBlocks<true> : kResBlocks<false>);
+  if (N % 32 != 0 || N < 1024 || N > 4096 || max_depth > 2 * held) return p;
+  p.split = (G + per_cta - 1) / per_cta;
+  p.rsw = N == 1024 ? 1056 : N == 4096 ? 4128 : 0;
+  const size_t row = (size_t)(N + 32) * 4;
+  // 8 rows where three stages of them fit (N <= 2300), else two stages of 6:
+  // at N = 4096 three stages of 4 rows took 1208 us for 60000 rows, two of 6
+  // 1119 (fewer list words and group turns per row); at N = 1024 16 rows are no
+  // faster than 8 (285 against 290 us) and leave more of the last round empty
+  // (10000 rows: 76 against 64 us).
+  p.T = 3 * 8 * row <= kResSmem ? 8 : 6;
+  p.stages = (int)std::min<size_t>(kMaxStages, kResSmem / (p.T * row));
+  p.smem = p.stages * p.T * row;
+  p.fn = find_instance(p.T, p.rsw, constw);
+  return p;
+}
+
+cudaError_t resident_prepare(const ResidentPlan& p) {
+  return cudaFuncSetAttribute(p.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+}
+
+cudaError_t launch_layer_resident(const ResidentPlan& p, const LayerArgs& a, int num_sms,
+                                  cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(std::max(1, num_sms / p.split) * p.split);
+  cfg.blockDim = dim3(kWarps * 32);
+  cfg.dynamicSmemBytes = p.smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int split = p.split, stages = p.stages;
+  void* args[] = {const_cast<LayerArgs*>(&a), &split, &stages};
+  return cudaLaunchKernelExC(&cfg, p.fn, args);
+}
+
+}  // namespace sdnn

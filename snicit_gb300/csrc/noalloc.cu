@@ -25,7 +25,7 @@
 
 namespace sdnn {
 int engine_layer_setup(sdnn_engine* e, int layer, LayerArgs* a, LayerKernelKey* key, int* grid,
-                       int* threads, size_t* smem);
+                       int* threads, size_t* smem, ResidentPlan* res, int* num_sms);
 cudaStream_t engine_stream(const sdnn_engine* e);
 void engine_set_error(sdnn_engine* e, const std::string& msg);
 }  // namespace sdnn
@@ -128,9 +128,11 @@ extern "C" int sdnn_layer_noalloc(sdnn_engine* e, int32_t layer, const float* d_
   DeviceGuard guard;  // engine_layer_setup makes the engine's device current
   sdnn::LayerArgs a;
   sdnn::LayerKernelKey key;
-  int grid = 0, threads = 0;
+  sdnn::ResidentPlan res;
+  int grid = 0, threads = 0, num_sms = 0;
   size_t smem = 0;
-  int rc = sdnn::engine_layer_setup(e, layer, &a, &key, &grid, &threads, &smem);
+  int rc = sdnn::engine_layer_setup(e, layer, &a, &key, &grid, &threads, &smem, &res,
+                                    &num_sms);
   if (rc) return rc;
   // CTAs that share a tile write one row's outputs while others may still be
   // loading that row: input and output must not overlap
@@ -154,7 +156,8 @@ extern "C" int sdnn_layer_noalloc(sdnn_engine* e, int32_t layer, const float* d_
   a.stamp = scratch->stamp;
   a.stamp_id = 1;
   a.err = &scratch->err[0];
-  cudaError_t ce = sdnn::launch_layer(key, a, grid, threads, smem, s);
+  cudaError_t ce = res.fn ? sdnn::launch_layer_resident(res, a, num_sms, s)
+                          : sdnn::launch_layer(key, a, grid, threads, smem, s);
   if (ce == cudaSuccess) ce = cudaMemsetAsync(d_alive, 0, (size_t)rows * sizeof(int32_t), s);
   if (ce == cudaSuccess) {
     noalloc_flags_kernel<<<64, 256, 0, s>>>(scratch, d_alive, (int32_t)rows);
@@ -178,9 +181,11 @@ extern "C" int sdnn_selftest_noalloc_timeout(sdnn_engine* e, int32_t* d_alive, i
   DeviceGuard guard;
   sdnn::LayerArgs a;
   sdnn::LayerKernelKey key;
-  int grid = 0, threads = 0;
+  sdnn::ResidentPlan res;
+  int grid = 0, threads = 0, num_sms = 0;
   size_t smem = 0;
-  int rc = sdnn::engine_layer_setup(e, 0, &a, &key, &grid, &threads, &smem);  // engine's device
+  int rc = sdnn::engine_layer_setup(e, 0, &a, &key, &grid, &threads, &smem, &res,
+                                    &num_sms);  // engine's device
   if (rc) return rc;
   NoAllocScratch* scratch = nullptr;
   rc = scratch_address(e, &scratch);

@@ -79,6 +79,19 @@ bool layer_instance_exists(const LayerKernelKey& key);
 // Sets the max dynamic shared memory attribute of an instance.
 cudaError_t layer_prepare(const LayerKernelKey& key, size_t smem);
 
+// Layer kernel with the slot lists in tensor memory (layer_resident.cu): the
+// plan for a layer, fn == nullptr where it does not apply (N outside 1024 ..
+// 4096, or lists too deep to keep).
+struct ResidentPlan {
+  const void* fn;
+  int T, rsw, split, stages;
+  size_t smem;
+};
+ResidentPlan resident_plan(int N, bool constw, int max_depth);
+cudaError_t resident_prepare(const ResidentPlan& p);
+cudaError_t launch_layer_resident(const ResidentPlan& p, const LayerArgs& a, int num_sms,
+                                  cudaStream_t s);
+
 // First layer over binary inputs (layer0_bits.cu).
 struct Layer0Args {
   const uint2* idx;          // packed slots of layer 0 (same layout as LayerDev)

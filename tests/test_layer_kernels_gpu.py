@@ -1,0 +1,85 @@
+"""The two layer kernels -- slot lists kept in tensor memory (the automatic
+choice at N = 1024 .. 4096) and lists streamed per tile (any width; taken when
+a tile shape is asked for) -- at the sizes where their splits have edges:
+fewer rows than CTAs, a part-filled last tile, widths with a part-filled last
+round of groups, and lists deeper than what a warp keeps.
+
+Both add every output's products in the same order, so their rows must agree
+bit for bit; and each output must lie within the rounding bound of a sum of
+its n products in FP32, (n + 2) * 2^-24 * (sum |w y| + |b|), of FP64.
+"""
+import numpy as np
+import pytest
+
+import snicit_gb300 as sg
+
+pytestmark = pytest.mark.gpu
+
+
+def _net(N, nnz, values, seed):
+    """nnz out-edges per input at distinct outputs; in-degrees vary around nnz."""
+    rng = np.random.default_rng([seed, N, nnz])
+    width = N // nnz
+    cols = rng.integers(0, width, (N, nnz)) + np.arange(nnz) * width
+    rows = np.repeat(np.arange(N), nnz)
+    vals = rng.standard_normal(N * nnz) * 0.3 if values else np.full(N * nnz, 0.0625)
+    return rows, cols.reshape(-1), vals.astype(np.float32)
+
+
+@pytest.mark.parametrize("N,nnz,values", [
+    (1024, 32, False), (1024, 24, True), (1056, 32, False), (2048, 32, True), (2304, 36, False),
+    (4096, 32, False), (4096, 20, True),
+    (1024, 80, False),   # lists past the 64 slots kept of a group
+    (1024, 50, True),    # ... past the 40 kept with their values
+    (1024, 200, False),  # too deep to keep: streamed either way
+])
+def test_resident_and_streamed_lists_agree(N, nnz, values):
+    r, c, v = _net(N, nnz, values, 5)
+    bias = -0.3
+    rng = np.random.default_rng(N + nnz)
+    for rows in (1, 7, 153, 1300):
+        Y = np.where(rng.random((rows, N)) < 0.4, rng.random((rows, N)) * 3, 0).astype(np.float32)
+        Y[rows // 2] = 0  # a row that dies
+        got = []
+        for kw in ({}, {"tile_rows": 4 if N == 4096 else 8, "threads": 512},
+                   {"tile_rows": 2 if N == 4096 else 8, "threads": 1024}):
+            with sg.Engine(N, 1, mode="SNIG", batch=rows, bias=bias, **kw) as e:
+                e.set_layer_coo(0, r, c, v)
+                flags, _ = e.infer(Y)
+                got.append((flags, e.activations(rows)))
+        for flags, act in got[1:]:
+            assert np.array_equal(flags, got[0][0])
+            assert np.array_equal(act.view(np.uint32), got[0][1].view(np.uint32))
+        W = np.zeros((N, N))
+        W[r, c] = v
+        Yd, b = Y.astype(np.float64), float(np.float32(bias))
+        want = np.clip(Yd @ W + b, 0, 32)
+        n = np.bincount(c, minlength=N)
+        bound = (n + 2) * 2.0 ** -24 * (Yd @ np.abs(W) + abs(b))
+        assert np.all(np.abs(got[0][1] - want) <= bound)
+        sure = (Yd @ W + b > bound).any(axis=1) | (Yd @ W + b <= -bound).all(axis=1)
+        assert np.array_equal(got[0][0][sure] != 0, (want > 0).any(axis=1)[sure])
+
+
+@pytest.mark.parametrize("N", [256, 8192, 16384, 32768])
+def test_streamed_split_covers_every_row_and_group(N):
+    """Row counts around the number of CTAs and of units per tile."""
+    r, c, v = _net(N, 32, False, 6)
+    bias = -0.3
+    rng = np.random.default_rng(N)
+    order = np.argsort(c, kind="stable")
+    start = np.searchsorted(c[order], np.arange(N + 1))
+    for rows in (1, 2, 151, 310):
+        Y = np.where(rng.random((rows, N)) < 0.4, rng.random((rows, N)) * 3, 0).astype(np.float32)
+        with sg.Engine(N, 1, mode="SNIG", batch=rows, bias=bias) as e:
+            e.set_layer_coo(0, r, c, v)
+            flags, ids = e.infer(Y)
+            act = e.activations(rows)
+        P = Y[:, r[order]].astype(np.float64) * 0.0625
+        S = np.add.reduceat(P, np.minimum(start[:-1], P.shape[1] - 1), axis=1)
+        n = np.diff(start)
+        S[:, n == 0] = 0
+        b = float(np.float32(bias))
+        bound = (n + 2) * 2.0 ** -24 * (S + abs(b))  # inputs and weights >= 0
+        assert np.all(np.abs(act - np.clip(S + b, 0, 32)) <= bound)
+        assert np.array_equal(np.flatnonzero(flags), ids) and len(ids) == rows
