@@ -171,10 +171,10 @@ struct sdnn_engine {
   // merging of identical rows (SNICIT, below the threshold)
   int32_t* d_alias = nullptr;          // [cap] -1 or the row this row was merged into
   unsigned long long* d_mtable = nullptr;  // [mmask + 1]
-  int32_t* d_mrep = nullptr;           // [mmask + 1]
+  unsigned long long* d_mrep = nullptr;    // [mmask + 1]
   int32_t* d_mpos = nullptr;           // [cap]
-  int32_t* d_mtmp = nullptr;           // [cap]
-  int32_t* d_mcount = nullptr;         // [2]
+  int32_t* d_mlist = nullptr;          // [cap] rows of a layer before its merge
+  int32_t* d_mcounts = nullptr;        // [L + 4] ... and their number
   uint32_t mmask = 0;
   int bits_grid = 0;
   bool bits_chunked = false;
@@ -326,8 +326,8 @@ void free_buffers(sdnn_engine* e) {
   dfree(e->d_mtable);
   dfree(e->d_mrep);
   dfree(e->d_mpos);
-  dfree(e->d_mtmp);
-  dfree(e->d_mcount);
+  dfree(e->d_mlist);
+  dfree(e->d_mcounts);
   dfree(e->d_pcounts);
   dfree(e->d_choice);
   dfree(e->d_plist[0]);
@@ -512,12 +512,10 @@ int ensure_buffers(sdnn_engine* e, int64_t rows) {
     e->mmask = (uint32_t)(P - 1);
     T(A(&e->d_alias, (size_t)cap * 4));
     T(A(&e->d_mtable, (size_t)P * 8));
-    T(A(&e->d_mrep, (size_t)P * 4));
+    T(A(&e->d_mrep, (size_t)P * 8));
     T(A(&e->d_mpos, (size_t)cap * 4));
-    T(A(&e->d_mtmp, (size_t)cap * 4));
-    T(A(&e->d_mcount, 16));
-    if (rc == cudaSuccess) rc = cudaMemset(e->d_mtable, 0, (size_t)P * 8);
-    if (rc == cudaSuccess) rc = cudaMemset(e->d_mrep, 0x7F, (size_t)P * 4);
+    T(A(&e->d_mlist, (size_t)cap * 4));
+    T(A(&e->d_mcounts, (size_t)(e->L + 4) * 4));
     if (rc == cudaSuccess) rc = cudaMemset(e->d_alias, 0xFF, (size_t)cap * 4);
   }
   T(A(&e->d_fbcount, 16));
@@ -1002,18 +1000,29 @@ bool merge_after(const sdnn_engine* e, int l, int T) {
 int enqueue_merge(sdnn_engine* e, int l) {
   DedupArgs m{};
   m.y = e->d_y[l & 1];
-  m.list = e->d_list[(l + 1) & 1];
-  m.count = e->d_counts + l + 1;
+  m.list_in = e->d_mlist;
+  m.count_in = e->d_mcounts + l + 1;
+  m.list_out = e->d_list[(l + 1) & 1];
+  m.count_out = e->d_counts + l + 1;
+  m.nrows = e->d_rows;
   m.table = e->d_mtable;
   m.slot_rep = e->d_mrep;
   m.pos_slot = e->d_mpos;
-  m.tmp_list = e->d_mtmp;
-  m.tmp_count = e->d_mcount;
   m.alias = e->d_alias;
   m.N = e->N;
+  m.step = l + 1;
   m.mask = e->mmask;
-  launch_dedup(m, e->num_sms, e->stream);
-  e->launches += 3;
+  CK(launch_dedup(m, e->num_sms, e->stream));
+  e->launches += 2;
+  return SDNN_OK;
+}
+
+// Clears what the merge steps of the last inference left.
+int enqueue_merge_begin(sdnn_engine* e) {
+  if (!merging_on(e)) return SDNN_OK;
+  CK(cudaMemsetAsync(e->d_mcounts, 0, (size_t)(e->L + 4) * 4, e->stream));
+  launch_dedup_clear(e->d_rows, e->d_mtable, e->d_mrep, e->mmask, e->stream);
+  e->launches++;
   CK(cudaGetLastError());
   return SDNN_OK;
 }
@@ -1079,10 +1088,13 @@ int enqueue_plain_layers(sdnn_engine* e, const float* d_in, int T, bool capturin
       if ((rc = record(e, 2, capturing))) return rc;
     }
     const float* in = l == 0 ? d_in : e->d_y[(l - 1) & 1];
-    if ((rc = enqueue_layer(e, l, in, e->d_list[l & 1], e->d_counts + l, e->d_list[(l + 1) & 1],
-                            e->d_counts + l + 1)))
+    // a layer that is merged after lists its rows apart; the merge lists what is left
+    const bool merge = merge_after(e, l, T);
+    if ((rc = enqueue_layer(e, l, in, e->d_list[l & 1], e->d_counts + l,
+                            merge ? e->d_mlist : e->d_list[(l + 1) & 1],
+                            (merge ? e->d_mcounts : e->d_counts) + l + 1)))
       return rc;
-    if (merge_after(e, l, T) && (rc = enqueue_merge(e, l))) return rc;
+    if (merge && (rc = enqueue_merge(e, l))) return rc;
   }
   if (!(split < T && T == L)) {
     if ((rc = record(e, 1, capturing))) return rc;
@@ -1111,8 +1123,10 @@ int enqueue_piece(sdnn_engine* e, int p, int64_t r0, int64_t n, int m, const flo
   for (int l = 0; l < m; ++l) {
     const float* in = l == 0 ? d_in : e->d_y[(l - 1) & 1];
     const bool last = l + 1 == m;
-    int32_t* lout = last ? e->d_list[m & 1] : e->d_plist[(l + 1) & 1] + r0;
-    int32_t* cout = last ? e->d_counts + m : pc + l + 1;
+    // (the rows of layer m; before its merge, where one comes first)
+    const bool merge = last && merge_after(e, l, effective_threshold(e));
+    int32_t* lout = !last ? e->d_plist[(l + 1) & 1] + r0 : merge ? e->d_mlist : e->d_list[m & 1];
+    int32_t* cout = !last ? pc + l + 1 : (merge ? e->d_mcounts : e->d_counts) + m;
     int rc = enqueue_layer(e, l, in, e->d_plist[l & 1] + r0, pc + l, lout, cout);
     if (rc) {
       e->bits_tile0 = 0;
@@ -1145,6 +1159,7 @@ int enqueue(sdnn_engine* e, int phase, int64_t rows, const float* d_in, int32_t*
       launch_begin_rows(e->d_rows, e->d_list[0], e->d_counts, d_flags, e->d_state, e->d_stamp,
                         e->d_alias, s);
       e->launches++;
+      if ((rc = enqueue_merge_begin(e))) return rc;
     }
     if ((rc = enqueue_plain_layers(e, d_in, T, capturing))) return rc;
   }
@@ -1997,6 +2012,7 @@ int run_streamed(sdnn_engine* e, const float* Y0, int64_t n, int m, int P) {
   launch_begin_rows(e->d_rows, e->d_plist[0], e->d_counts, e->d_flags, e->d_state, e->d_stamp,
                     e->d_alias, s);
   e->launches += 2;
+  if ((rc = enqueue_merge_begin(e))) return rc;
   // two lanes: even and odd pieces
   const bool two = true;
   if (two) {

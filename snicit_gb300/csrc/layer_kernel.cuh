@@ -309,7 +309,7 @@ __device__ __forceinline__ uint32_t epilogue_group(const float (&acc)[T], const 
         *dst = clampf(v, hi);
       } else {
         const int k = a.cslot[row];
-        const float pc = __ldg(a.pre_in + (size_t)k * a.N + c);
+        const float pc = a.pre_in[(size_t)k * a.N + c];
         const float y = clampf(pc + acc[t], hi) - clampf(pc, hi);
         *dst = y;
         if (y != 0.f) m |= 1u << t;

@@ -263,18 +263,23 @@ void launch_expand_bits(const uint64_t* bits, int64_t rows, int32_t N, float* ou
 // ---- exact merging of identical rows (dedup.cu) ----
 struct DedupArgs {
   const float* y;               // [rows][N] activations after the layer
-  int32_t* list;                // live rows after the layer; compacted in place
-  int32_t* count;               // its count; rewritten
-  unsigned long long* table;    // [mask + 1] keys, 0 = empty (all empty between calls)
-  int32_t* slot_rep;            // [mask + 1] smallest row per key, 0x7F7F7F7F = empty
+  const int32_t* list_in;       // live rows after the layer
+  const int32_t* count_in;
+  int32_t* list_out;            // ... one per set of equal rows
+  int32_t* count_out;           // must start at 0
+  const int32_t* nrows;         // rows of the inference (sizes the table in use)
+  unsigned long long* table;    // [mask + 1] keys, cleared once per inference
+  unsigned long long* slot_rep; // [mask + 1] smallest row per key, set to ~0 once per inference
   int32_t* pos_slot;            // [rows] table slot of each list position
-  int32_t* tmp_list;            // [rows]
-  int32_t* tmp_count;           // [2]: kept rows, rows listed before
   int32_t* alias;               // [rows] -1, or the row this row was merged into
   int32_t N;
+  int32_t step;                 // number of the merge step (unlike any other of the inference)
   uint32_t mask;                // table entries - 1 (a power of 2 >= 2 x rows, minus 1)
 };
-void launch_dedup(const DedupArgs& a, int num_sms, cudaStream_t s);
+cudaError_t launch_dedup(const DedupArgs& a, int num_sms, cudaStream_t s);
+// table[i] = 0 and slot_rep[i] = ~0 for the entries an inference of *nrows rows uses
+void launch_dedup_clear(const int32_t* nrows, unsigned long long* table,
+                        unsigned long long* slot_rep, uint32_t mask, cudaStream_t s);
 // alias[r] := root of r's chain, flags[r] := flags[root] for merged rows.
 void launch_resolve_alias(const int32_t* nrows, int32_t* alias, int32_t* flags, int32_t max_depth,
                           cudaStream_t s);
