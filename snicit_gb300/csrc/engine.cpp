@@ -118,8 +118,8 @@ struct sdnn_engine {
 
   // kernel configuration
   int Q = 0, nq = 1, G = 0;
-  LayerKernelKey key{};
-  int threads = 512, grid = 0, grid_general = 0, min_split = 1;
+  LayerKernelKey key{}, key_general{};  // one weight value / a value per edge
+  int threads = 512, threads_general = 512, grid = 0, grid_general = 0, min_split = 1;
   size_t smem = 0;
 
   // device weights (owned, or borrowed from weights_owner: a server's slot
@@ -390,7 +390,11 @@ void choose_layout(sdnn_engine* e) {
 int choose_kernel(sdnn_engine* e) {
   const int N = e->N;
   const int req_T = e->cfg.tile_rows;
-  int threads = e->cfg.threads > 0 ? e->cfg.threads : 512;
+  // input chunks: twice the warps with half the groups each hide the chunk
+  // loads better (5000 rows of 65536 neurons 3631 -> 3415 us); with a value per
+  // edge 64 registers a thread do not hold the lists (1000 rows 1028 against
+  // 1986 us), so those layers stay at 512
+  int threads = e->cfg.threads > 0 ? e->cfg.threads : e->nq > 1 ? 1024 : 512;
   if (threads != 256 && threads != 512 && threads != 1024) threads = 512;
   std::vector<LayerKernelKey> cands;
   if (e->nq == 1) {
@@ -423,12 +427,19 @@ int choose_kernel(sdnn_engine* e) {
     LayerKernelKey kc = k, kg = k;
     kc.constw = true;
     kg.constw = false;
+    int threads_general = threads;
+    if (e->cfg.threads == 0 && k.kg == 8) {
+      kg.kg = 16;
+      threads_general = 512;
+    }
     const int b1 = layer_blocks_per_sm(kc, threads, smem);
-    const int b2 = layer_blocks_per_sm(kg, threads, smem);
+    const int b2 = layer_blocks_per_sm(kg, threads_general, smem);
     if (b1 <= 0 || b2 <= 0) continue;
-    e->key = k;
+    e->key = kc;
+    e->key_general = kg;
     e->smem = smem;
     e->threads = threads;
+    e->threads_general = threads_general;
     e->grid = e->num_sms * b1;          // layers with one common weight value
     e->grid_general = e->num_sms * b2;  // layers with per-edge values
     const int nwarps = threads / 32;
@@ -951,9 +962,8 @@ int layer_launch(sdnn_engine* e, int l, int epi, const float* in, float* out, co
   if (resident_on(e, l)) {
     CK(launch_layer_resident(d.res, a, e->num_sms, e->stream));
   } else {
-    LayerKernelKey k = e->key;
-    k.constw = d.constw;
-    CK(launch_layer(k, a, d.constw ? e->grid : e->grid_general, e->threads, e->smem, e->stream));
+    CK(launch_layer(d.constw ? e->key : e->key_general, a, d.constw ? e->grid : e->grid_general,
+                    d.constw ? e->threads : e->threads_general, e->smem, e->stream));
   }
   e->launches++;
   return SDNN_OK;
@@ -1615,8 +1625,8 @@ int prepare(sdnn_engine* e, int64_t rows) {
     rc = choose_kernel(e);
     if (rc) return rc;
   }
-  CK(layer_prepare(LayerKernelKey{e->key.T, e->key.rsw, e->key.kg, true}, e->smem));
-  CK(layer_prepare(LayerKernelKey{e->key.T, e->key.rsw, e->key.kg, false}, e->smem));
+  CK(layer_prepare(e->key, e->smem));
+  CK(layer_prepare(e->key_general, e->smem));
   if (e->nq == 1)
     for (bool constw : {true, false}) {
       const ResidentPlan p = resident_plan(e->N, constw, 0);
@@ -2440,8 +2450,7 @@ int engine_layer_setup(sdnn_engine* e, int layer, LayerArgs* a, LayerKernelKey* 
     if (rc) return rc;
   }
   const DevLayer& d = e->dl[layer];
-  LayerKernelKey k = e->key;
-  k.constw = d.constw;
+  const LayerKernelKey k = d.constw ? e->key : e->key_general;
   *res = resident_on(e, layer) ? d.res : ResidentPlan{};
   *num_sms = e->num_sms;
   if (res->fn) CK(resident_prepare(*res));
@@ -2464,7 +2473,7 @@ int engine_layer_setup(sdnn_engine* e, int layer, LayerArgs* a, LayerKernelKey* 
   a->clampv = e->cfg.clamp;
   *key = k;
   *grid = d.constw ? e->grid : e->grid_general;
-  *threads = e->threads;
+  *threads = d.constw ? e->threads : e->threads_general;
   *smem = e->smem;
   return SDNN_OK;
 }
