@@ -383,7 +383,7 @@ void choose_layout(sdnn_engine* e) {
   // sparse residue rows need the whole row of one warp in shared memory
   // (the transposed layers and the lists exist whenever the layout allows
   // them, so the autotuner may switch between sparse and dense rows)
-  e->sparse_built = e->nq == 1 && sparse_residue_warps(N) > 0;
+  e->sparse_built = e->nq == 1 && sparse_residue_fits(N);
   e->sparse_res = e->sparse_built && !(e->cfg.flags & SDNN_FLAG_DENSE_RESIDUE);
 }
 

@@ -313,8 +313,7 @@ struct SparseResArgs {
   int32_t N;
   float clampv;
 };
-size_t sparse_residue_smem_per_warp(int N);
-int sparse_residue_warps(int N);  // warps per CTA (0: rows too wide for shared memory)
+bool sparse_residue_fits(int N);  // false: rows too wide for shared memory
 cudaError_t sparse_residue_prepare(int N);
 void launch_split_residue(const float* y, const int32_t* list, const int32_t* count,
                           const SparseRows& out, int32_t* dense_list, int32_t* dense_count,
