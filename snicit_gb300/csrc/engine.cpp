@@ -42,6 +42,7 @@ struct DevLayer {
   int2* lists = nullptr;  // per (group, chunk): first block, slots up to the last edge
   float* bias = nullptr;
   float* sums = nullptr;  // layer 0 with one common value: w added k times, k < 128
+  int32_t max_in_degree = 127;
   // transposed layer for the sparse residue update: out-edges of every input
   // position (output positions, values unless the layer has one value)
   int32_t* tr_off = nullptr;
@@ -140,8 +141,6 @@ struct sdnn_engine {
   int32_t* d_rlist[2] = {nullptr, nullptr};
   int32_t* d_counts = nullptr;   // [L + 2]
   int32_t* d_rcounts = nullptr;  // [L + 2]
-  uint32_t* d_tmask = nullptr;   // tile masks and tickets of the chunked binary layer 0
-  int32_t* d_ticket = nullptr;
   int32_t* d_stamp = nullptr;    // [cap] marks of the layer launches that listed a row
   int32_t* d_clist = nullptr;
   int32_t* d_ccount = nullptr;
@@ -176,8 +175,7 @@ struct sdnn_engine {
   int32_t* d_mlist = nullptr;          // [cap] rows of a layer before its merge
   int32_t* d_mcounts = nullptr;        // [L + 4] ... and their number
   uint32_t mmask = 0;
-  int bits_grid = 0;
-  bool bits_chunked = false;
+  bool bits_on = false;            // layer 0 of 0/1 inputs by counting
 
   cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
 
@@ -186,12 +184,10 @@ struct sdnn_engine {
   cudaStream_t copy_stream = nullptr;
   cudaEvent_t piece_ev[kMaxPieces] = {};
   cudaEvent_t ingest_free = nullptr, lane_ev = nullptr;
-  // second lane for odd pieces: its own stream, tile tickets and layer-0
-  // fallback list (swapped in with swap_lane), so one piece's layers fill the
+  // second lane for odd pieces: its own stream and layer-0 fallback list
+  // (swapped in with swap_lane), so one piece's layers fill the
   // last partial wave of the other's
   cudaStream_t stream2 = nullptr;
-  uint32_t* d_tmask2 = nullptr;
-  int32_t* d_ticket2 = nullptr;
   int32_t* d_fallback2 = nullptr;
   int32_t* d_fbcount2 = nullptr;
   int32_t* d_pcounts = nullptr;  // [kMaxPieces][L + 2]
@@ -295,8 +291,6 @@ void free_buffers(sdnn_engine* e) {
   dfree(e->d_rlist[1]);
   dfree(e->d_counts);
   dfree(e->d_rcounts);
-  dfree(e->d_tmask);
-  dfree(e->d_ticket);
   dfree(e->d_stamp);
   dfree(e->d_clist);
   dfree(e->d_ccount);
@@ -332,8 +326,6 @@ void free_buffers(sdnn_engine* e) {
   dfree(e->d_choice);
   dfree(e->d_plist[0]);
   dfree(e->d_plist[1]);
-  dfree(e->d_tmask2);
-  dfree(e->d_ticket2);
   dfree(e->d_fallback2);
   dfree(e->d_fbcount2);
   for (int i = 0; i < 2; ++i) {
@@ -362,12 +354,6 @@ void drop_graph(sdnn_engine* e) {
 }
 
 constexpr size_t kMaxSmem = 227 * 1024;
-// threads per CTA of the binary first-layer kernel: small enough for two or
-// three CTAs per SM, so one CTA's row loads overlap another's counting
-#ifndef SDNN_BITS_THREADS
-#define SDNN_BITS_THREADS 256
-#endif
-constexpr int kBitsThreads = SDNN_BITS_THREADS;
 // first plain layer after which identical rows are merged (SNICIT): rows are
 // still distinct in the first layers, where most of them die
 constexpr int kMergeStart = 4;
@@ -451,6 +437,11 @@ int choose_kernel(sdnn_engine* e) {
                   (req_T > 0 ? " with tile_rows=" + std::to_string(req_T) : std::string()));
 }
 
+// Whether the layout has a counting kernel for 0/1 inputs.
+bool bits_possible(const sdnn_engine* e) {
+  return e->nq > 1 ? layer0_bits_chunked_supported(e->N, e->Q) : layer0_bits_supported(e->N);
+}
+
 int ensure_buffers(sdnn_engine* e, int64_t rows) {
   if (e->cap >= rows && e->cap > 0) return SDNN_OK;
   free_buffers(e);
@@ -477,8 +468,6 @@ int ensure_buffers(sdnn_engine* e, int64_t rows) {
   }
   T(A(&e->d_counts, (size_t)(e->L + 4) * 4));
   T(A(&e->d_rcounts, (size_t)(e->L + 4) * 4));
-  T(A(&e->d_tmask, (size_t)(cap + 1) * 4));
-  T(A(&e->d_ticket, (size_t)(cap + 1) * 4));
   T(A(&e->d_stamp, (size_t)cap * 4));
   T(A(&e->d_clist, (size_t)K * 4));
   T(A(&e->d_ccount, 16));
@@ -512,7 +501,7 @@ int ensure_buffers(sdnn_engine* e, int64_t rows) {
   // grid chain rows: a fresh buffer per layer (wide layouts only, where it runs)
   if (e->N >= 16384) T(A(&e->d_gscratch, grid_chain_scratch_floats(e->L, e->nq, e->Q) * 4));
   T(A(&e->d_gbar, 16));
-  if (e->nq > 1 && layer0_bits_chunked_supported(e->N, e->Q)) {
+  if (bits_possible(e)) {
     const size_t tiles = (size_t)(cap + 31) / 32;
     T(A(&e->d_bits, tiles * (size_t)N * 4));
     T(A(&e->d_tile_state, tiles * 4));
@@ -535,8 +524,6 @@ int ensure_buffers(sdnn_engine* e, int64_t rows) {
   T(A(&e->d_choice, 16));
   T(A(&e->d_plist[0], (size_t)cap * 4));
   T(A(&e->d_plist[1], (size_t)cap * 4));
-  T(A(&e->d_tmask2, (size_t)(cap + 1) * 4));
-  T(A(&e->d_ticket2, (size_t)(cap + 1) * 4));
   T(A(&e->d_fallback2, (size_t)cap * 4));
   T(A(&e->d_fbcount2, 16));
   if (rc == cudaSuccess) T(cudaMallocHost((void**)&e->h_counts, 16));
@@ -546,10 +533,6 @@ int ensure_buffers(sdnn_engine* e, int64_t rows) {
     return fail(e, SDNN_ERR_OOM, std::string("device allocation failed: ") + cudaGetErrorString(rc));
   }
   e->cap = cap;
-  CK(cudaMemsetAsync(e->d_tmask, 0, (size_t)(cap + 1) * 4, e->stream));
-  CK(cudaMemsetAsync(e->d_ticket, 0, (size_t)(cap + 1) * 4, e->stream));
-  CK(cudaMemsetAsync(e->d_tmask2, 0, (size_t)(cap + 1) * 4, e->stream));
-  CK(cudaMemsetAsync(e->d_ticket2, 0, (size_t)(cap + 1) * 4, e->stream));
   CK(cudaMemsetAsync(e->d_err, 0, 16, e->stream));
   return SDNN_OK;
 }
@@ -692,6 +675,15 @@ int upload_layer(sdnn_engine* e, int l, const PackedView& p, std::string& err) {
     T(cudaMemcpy(d.bias, b.data(), (size_t)e->N * 4, cudaMemcpyHostToDevice));
   }
   if (rc == cudaSuccess && l == 0 && p.constw && p.max_depth < 128 && p.max_in_degree < 128) {
+    // the largest in-degree, from the slots themselves
+    d.max_in_degree = 0;
+    for (int32_t g = 0; g < e->G; ++g) {
+      int32_t deg[32] = {};
+      for (int32_t b = p.grp_blk[g * e->nq]; b < p.grp_blk[(g + 1) * e->nq]; ++b)
+        for (int k = 0; k < 128; ++k)
+          deg[k >> 2] += p.idx[(size_t)b * 128 + k] / (slot_index_in_bytes(e->Q) ? 4 : 1) < e->Q;
+      d.max_in_degree = std::max(d.max_in_degree, *std::max_element(deg, deg + 32));
+    }
     // the float kernel adds w once per active edge: reproduce those sums
     float sums[128];
     float acc = 0.f;
@@ -1027,8 +1019,10 @@ int enqueue_merge(sdnn_engine* e, int l) {
   return SDNN_OK;
 }
 
-// Clears what the merge steps of the last inference left.
-int enqueue_merge_begin(sdnn_engine* e) {
+// Clears what the last inference left: tile flags of layer 0, merge steps.
+int enqueue_clear(sdnn_engine* e) {
+  if (e->bits_on)
+    CK(cudaMemsetAsync(e->d_tile_state, 0, (size_t)((e->cap + 31) / 32) * 4, e->stream));
   if (!merging_on(e)) return SDNN_OK;
   CK(cudaMemsetAsync(e->d_mcounts, 0, (size_t)(e->L + 4) * 4, e->stream));
   launch_dedup_clear(e->d_rows, e->d_mtable, e->d_mrep, e->mmask, e->stream);
@@ -1043,7 +1037,7 @@ int enqueue_merge_begin(sdnn_engine* e) {
 int enqueue_layer(sdnn_engine* e, int l, const float* in, const int32_t* lin, const int32_t* cin,
                   int32_t* lout, int32_t* cout) {
   const cudaStream_t s = e->stream;
-  const bool bits = l == 0 && e->dl[0].sums && (e->bits_chunked || e->bits_grid > 0);
+  const bool bits = l == 0 && e->dl[0].sums && e->bits_on;
   if (!bits) return layer_launch(e, l, EPI_PLAIN, in, e->d_y[l & 1], lin, cin, lout, cout);
   CK(cudaMemsetAsync(e->d_fbcount, 0, 16, s));
   Layer0Args b{};
@@ -1053,9 +1047,10 @@ int enqueue_layer(sdnn_engine* e, int l, const float* in, const int32_t* lin, co
   b.bias = e->cfg.bias;
   b.clampv = e->cfg.clamp;
   b.sums = e->dl[0].sums;
+  b.max_count = e->dl[0].max_in_degree;
   b.y_in = in;
   b.y_out = e->d_y[0];
-  b.list_in = lin;
+  b.first_row = (int32_t)(e->bits_tile0 * 32);  // (layer 0 takes the rows in order)
   b.count_in = cin;
   b.list_out = lout;
   b.count_out = cout;
@@ -1063,21 +1058,15 @@ int enqueue_layer(sdnn_engine* e, int l, const float* in, const int32_t* lin, co
   b.fallback_count = e->d_fbcount;
   b.N = e->N;
   b.G = e->G;
-  if (e->bits_chunked) {
-    // input chunks: transpose pass + counting pass
-    b.nq = e->nq;
-    b.Q = e->Q;
-    b.bits = e->d_bits + e->bits_tile0 * e->N;
-    b.tile_state = e->d_tile_state + e->bits_tile0;
-    b.tile_mask = e->d_tmask;
-    b.tile_ticket = e->d_ticket;
-    b.err = e->d_err;
-    CK(launch_layer0_bits_chunked(b, e->num_sms, s));
-    e->launches += 2;
-  } else {
-    CK(launch_layer0_bits(b, e->bits_grid, kBitsThreads, s));
-    e->launches++;
-  }
+  b.nq = e->nq;
+  b.Q = e->Q;
+  b.bits = e->d_bits + e->bits_tile0 * e->N;
+  b.tile_state = e->d_tile_state + e->bits_tile0;
+  b.stamp = e->d_stamp;
+  b.stamp_id = 1;
+  b.err = e->d_err;
+  CK(launch_layer0_bits(b, e->num_sms, s));
+  e->launches += 2;
   return layer_launch(e, 0, EPI_PLAIN, in, e->d_y[0], e->d_fallback, e->d_fbcount, lout, cout);
 }
 
@@ -1127,7 +1116,7 @@ int enqueue_piece(sdnn_engine* e, int p, int64_t r0, int64_t n, int m, const flo
   launch_set_scalar(pc, (int32_t)n, e->stream);
   e->launches++;
   CK(cudaGetLastError());
-  // the piece's bit words (binary layer 0 with input chunks) go to its own
+  // the piece's bit words (binary layer 0) go to its own
   // tiles of the buffer (pieces start on 32-row tiles), so both lanes may run
   e->bits_tile0 = r0 / 32;
   for (int l = 0; l < m; ++l) {
@@ -1169,7 +1158,7 @@ int enqueue(sdnn_engine* e, int phase, int64_t rows, const float* d_in, int32_t*
       launch_begin_rows(e->d_rows, e->d_list[0], e->d_counts, d_flags, e->d_state, e->d_stamp,
                         e->d_alias, s);
       e->launches++;
-      if ((rc = enqueue_merge_begin(e))) return rc;
+      if ((rc = enqueue_clear(e))) return rc;
     }
     if ((rc = enqueue_plain_layers(e, d_in, T, capturing))) return rc;
   }
@@ -1633,12 +1622,7 @@ int prepare(sdnn_engine* e, int64_t rows) {
       if (p.fn) CK(resident_prepare(p));
     }
   if (e->sparse_built) CK(sparse_residue_prepare(e->N));
-  e->bits_chunked = e->nq > 1 && !(e->cfg.flags & SDNN_FLAG_NO_BINARY_FIRST_LAYER) &&
-                    layer0_bits_chunked_supported(e->N, e->Q);
-  e->bits_grid = (e->nq == 1 && !(e->cfg.flags & SDNN_FLAG_NO_BINARY_FIRST_LAYER) &&
-                  layer0_bits_supported(e->N))
-                     ? layer0_bits_grid(e->N, e->num_sms, kBitsThreads)
-                     : 0;
+  e->bits_on = bits_possible(e) && !(e->cfg.flags & SDNN_FLAG_NO_BINARY_FIRST_LAYER);
   return ensure_buffers(e, rows);
 }
 
@@ -1648,8 +1632,6 @@ int check_device_error(sdnn_engine* e) {
   CK(cudaStreamSynchronize(e->stream));
   if (h == DEV_TIMEOUT) {
     cudaMemsetAsync(e->d_err, 0, 4, e->stream);
-    cudaMemsetAsync(e->d_tmask, 0, (size_t)(e->cap + 1) * 4, e->stream);
-    cudaMemsetAsync(e->d_ticket, 0, (size_t)(e->cap + 1) * 4, e->stream);
     return fail(e, SDNN_ERR_TIMEOUT, "a device-side wait timed out");
   }
   if (h != 0) return fail(e, SDNN_ERR_CUDA, "device error word " + std::to_string(h));
@@ -1971,12 +1953,10 @@ int streamed_prefix(const sdnn_engine* e) {
   return m;
 }
 
-// Swaps the engine's stream, tile tickets and layer-0 fallback list with the
+// Swaps the engine's stream and layer-0 fallback list with the
 // second lane's (called in pairs around the work of an odd piece).
 void swap_lane(sdnn_engine* e) {
   std::swap(e->stream, e->stream2);
-  std::swap(e->d_tmask, e->d_tmask2);
-  std::swap(e->d_ticket, e->d_ticket2);
   std::swap(e->d_fallback, e->d_fallback2);
   std::swap(e->d_fbcount, e->d_fbcount2);
 }
@@ -2022,7 +2002,7 @@ int run_streamed(sdnn_engine* e, const float* Y0, int64_t n, int m, int P) {
   launch_begin_rows(e->d_rows, e->d_plist[0], e->d_counts, e->d_flags, e->d_state, e->d_stamp,
                     e->d_alias, s);
   e->launches += 2;
-  if ((rc = enqueue_merge_begin(e))) return rc;
+  if ((rc = enqueue_clear(e))) return rc;
   // two lanes: even and odd pieces
   const bool two = true;
   if (two) {
