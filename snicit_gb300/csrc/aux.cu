@@ -61,34 +61,28 @@ void launch_sum_piece_counts(const int32_t* piece_counts, int pieces, int stride
   sum_piece_counts_kernel<<<1, 256, 0, s>>>(piece_counts, pieces, stride, layers, counts);
 }
 
-__global__ void begin_rows_kernel(const int32_t* nrows, int32_t* list, int32_t* count,
-                                  int32_t* zero_a, int32_t* zero_b, int32_t* zero_c,
-                                  int32_t* neg) {
-  const int n = *nrows;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    list[i] = i;
-    if (zero_a) zero_a[i] = 0;
-    if (zero_b) zero_b[i] = 0;
-    if (zero_c) zero_c[i] = 0;
-    if (neg) neg[i] = -1;
+__global__ void begin_kernel(const BeginArgs a) {
+  const int n = *a.nrows;
+  const int at = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  for (int i = at; i < n; i += stride) {
+    a.list[i] = i;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) a.zero[k][i] = 0;
+    a.alias[i] = -1;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) *count = n;
-}
-void launch_begin_rows(const int32_t* nrows, int32_t* list, int32_t* count, int32_t* zero_a,
-                       int32_t* zero_b, int32_t* zero_c, int32_t* neg, cudaStream_t s) {
-  begin_rows_kernel<<<264, 256, 0, s>>>(nrows, list, count, zero_a, zero_b, zero_c, neg);
-}
-
-__global__ void zero_rows_kernel(const int32_t* nrows, int32_t* a, int32_t* b) {
-  const int n = *nrows;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    a[i] = 0;
-    if (b) b[i] = 0;
+  for (int i = at; i < a.counts_n; i += stride) a.counts[i] = i == 0 ? n : 0;
+  for (int i = at; i < a.extra_n; i += stride) a.extra[i] = 0;
+  if (a.tile_state)
+    for (int i = at; i < (n + 31) / 32; i += stride) a.tile_state[i] = 0;
+  if (a.mask) {
+    const uint32_t mask = dedup_table_mask(n, a.mask);
+    for (uint32_t i = at; i <= mask; i += stride) {
+      a.table[i] = 0ull;
+      a.slot_rep[i] = ~0ull;
+    }
   }
 }
-void launch_zero_rows(const int32_t* nrows, int32_t* a, int32_t* b, cudaStream_t s) {
-  zero_rows_kernel<<<264, 256, 0, s>>>(nrows, a, b);
-}
+void launch_begin(const BeginArgs& a, cudaStream_t s) { begin_kernel<<<264, 256, 0, s>>>(a); }
 
 __global__ void copy_rows_kernel(const int32_t* nrows, const float4* src, float4* dst, int32_t n4) {
   const size_t total = (size_t)(*nrows) * (size_t)n4;
@@ -99,17 +93,6 @@ __global__ void copy_rows_kernel(const int32_t* nrows, const float4* src, float4
 void launch_copy_rows(const int32_t* nrows, const float* src, float* dst, int32_t N, cudaStream_t s) {
   copy_rows_kernel<<<1024, 256, 0, s>>>(nrows, reinterpret_cast<const float4*>(src),
                                         reinterpret_cast<float4*>(dst), N / 4);
-}
-
-__global__ void mark_rows_kernel(const int32_t* list, const int32_t* count, int32_t* flags,
-                                 int32_t value) {
-  const int n = *count;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    flags[list[i]] = value;
-}
-void launch_mark_rows(const int32_t* list, const int32_t* count, int32_t* flags, int32_t value,
-                      cudaStream_t s) {
-  mark_rows_kernel<<<264, 256, 0, s>>>(list, count, flags, value);
 }
 
 // Whether any of at(0) .. at(N - 1) is positive (one warp; 8 loads of a lane in
@@ -131,8 +114,9 @@ __device__ __forceinline__ bool any_positive(int N, int lane, At at) {
 // identify (src/SDGC/utility.hpp:194-212): category = 1 if the row has an
 // activation > 0.  (The reference sums the row with thrust::reduce and an int
 // initial value; see the oracle for that variant.)  One warp per listed row.
-__global__ void identify_kernel(const float* __restrict__ y, const int32_t* list,
-                                const int32_t* count, int32_t N, int32_t* flags) {
+__global__ void identify_kernel(const float* y, const int32_t* list,
+                                const int32_t* count, int32_t N, int32_t* flags, int32_t* state) {
+  pdl_prologue();
   const int n = *count;
   const int lane = threadIdx.x & 31;
   const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -141,12 +125,15 @@ __global__ void identify_kernel(const float* __restrict__ y, const int32_t* list
     const int r = list[i];
     const float* row = y + (size_t)r * N;
     const bool any = any_positive(N, lane, [&](int j) { return row[j]; });
-    if (lane == 0) flags[r] = any ? 1 : 0;
+    if (lane == 0) {
+      flags[r] = any ? 1 : 0;
+      state[r] = 1;
+    }
   }
 }
 void launch_identify(const float* y, const int32_t* list, const int32_t* count, int32_t N,
-                     int32_t* flags, cudaStream_t s) {
-  identify_kernel<<<528, 256, 0, s>>>(y, list, count, N, flags);
+                     int32_t* flags, int32_t* state, int num_sms, cudaStream_t s) {
+  launch_pdl(identify_kernel, num_sms * 4, 256, 0, s, y, list, count, N, flags, state);
 }
 
 // Ordered compaction: ids = sorted indices i with flags[i] != 0.  One CTA.
@@ -214,6 +201,7 @@ constexpr int kHistBins = 4096;
 constexpr int kCandCap = 2048;
 
 __global__ void __launch_bounds__(1024) cand_select_kernel(ClusterArgs a) {
+  pdl_prologue();
   __shared__ int hist[kHistBins];
   __shared__ unsigned long long skey[kCandCap];
   __shared__ int srow[kCandCap];
@@ -305,6 +293,7 @@ __global__ void __launch_bounds__(1024) cand_select_kernel(ClusterArgs a) {
 
 // 16 disjoint bin sums per candidate; one warp per bin, fixed reduction order.
 __global__ void cand_bins_kernel(ClusterArgs a) {
+  pdl_prologue();
   const int k = blockIdx.x;
   if (k >= *a.ncand) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -324,6 +313,7 @@ __global__ void cand_bins_kernel(ClusterArgs a) {
 // bins within 0.03 (the reference drops when fewer than 16*0.03 bins differ by
 // more than 0.03, i.e. when none does).
 __global__ void __launch_bounds__(256) prune_kernel(ClusterArgs a) {
+  pdl_prologue();
   __shared__ int keep[256];
   __shared__ float sb[256 * 16];
   const int tid = threadIdx.x;
@@ -367,6 +357,7 @@ __global__ void __launch_bounds__(256) prune_kernel(ClusterArgs a) {
 // row one after the other; now 30.
 constexpr int kAssignWarps = 8;
 __global__ void __launch_bounds__(kAssignWarps * 32) assign_kernel(ClusterArgs a) {
+  pdl_prologue();
   __shared__ unsigned long long s_best;  // (distance, centroid), the smallest so far
   const int n = *a.live_count;
   const int nc = *a.ccount;
@@ -422,19 +413,21 @@ __global__ void __launch_bounds__(kAssignWarps * 32) assign_kernel(ClusterArgs a
 }
 
 void launch_cluster(const ClusterArgs& a, int num_sms, cudaStream_t s) {
-  cand_select_kernel<<<1, 1024, 0, s>>>(a);
-  cand_bins_kernel<<<a.K, 512, 0, s>>>(a);
-  prune_kernel<<<1, 256, 0, s>>>(a);
-  assign_kernel<<<num_sms * 8, kAssignWarps * 32, 0, s>>>(a);
+  launch_pdl(cand_select_kernel, 1, 1024, 0, s, a);
+  launch_pdl(cand_bins_kernel, a.K, 512, 0, s, a);
+  launch_pdl(prune_kernel, 1, 256, 0, s, a);
+  launch_pdl(assign_kernel, num_sms * 8, kAssignWarps * 32, 0, s, a);
 }
 
 // ------------------------------------------------------------------ recovery
 
 // recover (src/SDGC/SNICIT/kernel.hpp:197-218): flags[r] = any((delta + c) > 0).
-__global__ void recover_kernel(const float* __restrict__ y, const int32_t* live,
+__global__ void recover_kernel(const float* y, const int32_t* live,
                                const int32_t* live_count, const int32_t* cslot,
                                const int32_t* clist, const int32_t* is_centroid,
-                               const int32_t* res_flag, int32_t N, int32_t* flags) {
+                               const int32_t* res_flag, int32_t N, int32_t* flags,
+                               int32_t* state) {
+  pdl_prologue();
   const int n = *live_count;
   const int lane = threadIdx.x & 31;
   const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -450,14 +443,18 @@ __global__ void recover_kernel(const float* __restrict__ y, const int32_t* live,
       if (res_flag[r]) any = any_positive(N, lane, [&](int j) { return yr[j] + yc[j]; });
       else any = any_positive(N, lane, [&](int j) { return yc[j]; });
     }
-    if (lane == 0) flags[r] = any ? 1 : 0;
+    if (lane == 0) {
+      flags[r] = any ? 1 : 0;
+      state[r] = 2;
+    }
   }
 }
 void launch_recover(const float* y, const int32_t* live, const int32_t* live_count,
                     const int32_t* cslot, const int32_t* clist, const int32_t* is_centroid,
-                    const int32_t* res_flag, int32_t N, int32_t* flags, cudaStream_t s) {
-  recover_kernel<<<528, 256, 0, s>>>(y, live, live_count, cslot, clist, is_centroid, res_flag, N,
-                                     flags);
+                    const int32_t* res_flag, int32_t N, int32_t* flags, int32_t* state, int num_sms,
+                    cudaStream_t s) {
+  launch_pdl(recover_kernel, num_sms * 4, 256, 0, s, y, live, live_count, cslot, clist, is_centroid,
+             res_flag, N, flags, state);
 }
 
 // Final activations per row, in neuron order (out[r][c] reads position perm[c]):

@@ -57,13 +57,6 @@ __device__ __forceinline__ void mix_in(uint32_t& h1, uint32_t& h2, uint32_t v) {
 
 constexpr int kDedupWarps = 16;
 
-// Entries in use for an inference of `rows` rows (a power of two >= 2 rows).
-__device__ __forceinline__ uint32_t table_mask(int32_t rows, uint32_t cap_mask) {
-  uint32_t m = 1023u;
-  while (m < 2u * (uint32_t)rows && m < cap_mask) m = 2u * m + 1u;
-  return m < cap_mask ? m : cap_mask;
-}
-
 template <int TEAM>
 __global__ void __launch_bounds__(kDedupWarps * 32) dedup_hash_kernel(const DedupArgs a) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -75,7 +68,7 @@ __global__ void __launch_bounds__(kDedupWarps * 32) dedup_hash_kernel(const Dedu
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const int n = *a.count_in;
   if (n <= 1) return;  // nothing to merge: no slot is looked at
-  const uint32_t mask = table_mask(*a.nrows, a.mask);
+  const uint32_t mask = dedup_table_mask(*a.nrows, a.mask);
   const bool vec = (a.N & 3) == 0;
   for (int base = blockIdx.x * kRows; base < n; base += gridDim.x * kRows) {
     const int i = base + team;
@@ -220,17 +213,9 @@ __global__ void __launch_bounds__(kDedupWarps * 32) dedup_verify_kernel(const De
   }
 }
 
-__global__ void dedup_clear_kernel(const int32_t* nrows, unsigned long long* table,
-                                   unsigned long long* slot_rep, uint32_t cap_mask) {
-  const uint32_t mask = table_mask(*nrows, cap_mask);
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= mask; i += gridDim.x * blockDim.x) {
-    table[i] = 0ull;
-    slot_rep[i] = ~0ull;
-  }
-}
-
 __global__ void resolve_alias_kernel(const int32_t* nrows, int32_t* alias, int32_t* flags,
                                      int32_t max_depth) {
+  pdl_prologue();
   const int n = *nrows;
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
     int x = alias[r];
@@ -250,35 +235,20 @@ __global__ void resolve_alias_kernel(const int32_t* nrows, int32_t* alias, int32
 
 cudaError_t launch_dedup(const DedupArgs& a, int num_sms, cudaStream_t s) {
   // a row's bytes over its team: 4 KB by one warp, 16 KB by 4, more by 16
-  const void* hash = a.N <= 2048   ? (const void*)&dedup_hash_kernel<1>
-                     : a.N <= 8192 ? (const void*)&dedup_hash_kernel<4>
-                                   : (const void*)&dedup_hash_kernel<16>;
-  const void* verify = a.N <= 2048   ? (const void*)&dedup_verify_kernel<1>
-                       : a.N <= 8192 ? (const void*)&dedup_verify_kernel<4>
-                                     : (const void*)&dedup_verify_kernel<16>;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(num_sms * 4);
-  cfg.blockDim = dim3(kDedupWarps * 32);
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  void* args[] = {const_cast<DedupArgs*>(&a)};
-  cudaError_t rc = cudaLaunchKernelExC(&cfg, hash, args);
-  if (rc == cudaSuccess) rc = cudaLaunchKernelExC(&cfg, verify, args);
+  auto hash = a.N <= 2048   ? dedup_hash_kernel<1>
+              : a.N <= 8192 ? dedup_hash_kernel<4>
+                            : dedup_hash_kernel<16>;
+  auto verify = a.N <= 2048   ? dedup_verify_kernel<1>
+                : a.N <= 8192 ? dedup_verify_kernel<4>
+                              : dedup_verify_kernel<16>;
+  cudaError_t rc = launch_pdl(hash, num_sms * 4, kDedupWarps * 32, 0, s, a);
+  if (rc == cudaSuccess) rc = launch_pdl(verify, num_sms * 4, kDedupWarps * 32, 0, s, a);
   return rc;
-}
-
-void launch_dedup_clear(const int32_t* nrows, unsigned long long* table,
-                        unsigned long long* slot_rep, uint32_t mask, cudaStream_t s) {
-  dedup_clear_kernel<<<264, 256, 0, s>>>(nrows, table, slot_rep, mask);
 }
 
 void launch_resolve_alias(const int32_t* nrows, int32_t* alias, int32_t* flags, int32_t max_depth,
                           cudaStream_t s) {
-  resolve_alias_kernel<<<264, 256, 0, s>>>(nrows, alias, flags, max_depth);
+  launch_pdl(resolve_alias_kernel, 264, 256, 0, s, nrows, alias, flags, max_depth);
 }
 
 }  // namespace sdnn

@@ -139,8 +139,13 @@ struct sdnn_engine {
   float* d_y[2] = {nullptr, nullptr};
   int32_t* d_list[2] = {nullptr, nullptr};
   int32_t* d_rlist[2] = {nullptr, nullptr};
-  int32_t* d_counts = nullptr;   // [L + 2]
-  int32_t* d_rcounts = nullptr;  // [L + 2]
+  // counters of an inference, one block: [L + 4] each of the rows per layer, the
+  // dense, sparse and unsplit residue rows and the rows before a merge, then
+  // scalars; an inference begins by clearing all of it up to ctl_clear
+  int32_t* d_ctl = nullptr;
+  int32_t ctl_clear = 0, ctl_size = 0;
+  int32_t* d_counts = nullptr;
+  int32_t* d_rcounts = nullptr;
   int32_t* d_stamp = nullptr;    // [cap] marks of the layer launches that listed a row
   int32_t* d_clist = nullptr;
   int32_t* d_ccount = nullptr;
@@ -289,13 +294,10 @@ void free_buffers(sdnn_engine* e) {
   dfree(e->d_list[1]);
   dfree(e->d_rlist[0]);
   dfree(e->d_rlist[1]);
-  dfree(e->d_counts);
-  dfree(e->d_rcounts);
+  dfree(e->d_ctl);
   dfree(e->d_stamp);
   dfree(e->d_clist);
-  dfree(e->d_ccount);
   dfree(e->d_cand);
-  dfree(e->d_ncand);
   dfree(e->d_bins);
   dfree(e->d_cslot);
   dfree(e->d_iscent);
@@ -303,12 +305,9 @@ void free_buffers(sdnn_engine* e) {
   dfree(e->d_flags);
   dfree(e->d_state);
   dfree(e->d_pre);
-  dfree(e->d_err);
   dfree(e->d_ids);
-  dfree(e->d_idcount);
   dfree(e->d_in);
   dfree(e->d_fallback);
-  dfree(e->d_fbcount);
   dfree(e->d_bits);
   dfree(e->d_tile_state);
   dfree(e->d_gscratch);
@@ -321,22 +320,17 @@ void free_buffers(sdnn_engine* e) {
   dfree(e->d_mrep);
   dfree(e->d_mpos);
   dfree(e->d_mlist);
-  dfree(e->d_mcounts);
   dfree(e->d_pcounts);
-  dfree(e->d_choice);
   dfree(e->d_plist[0]);
   dfree(e->d_plist[1]);
   dfree(e->d_fallback2);
-  dfree(e->d_fbcount2);
   for (int i = 0; i < 2; ++i) {
     dfree(e->d_sp_idx[i]);
     dfree(e->d_sp_val[i]);
     dfree(e->d_sp_cnt[i]);
     dfree(e->d_slist[i]);
   }
-  dfree(e->d_scounts);
   dfree(e->d_rtmp);
-  dfree(e->d_tcounts);
   if (e->h_counts) cudaFreeHost(e->h_counts);
   e->h_counts = nullptr;
   e->cap = 0;
@@ -466,13 +460,38 @@ int ensure_buffers(sdnn_engine* e, int64_t rows) {
     T(A(&e->d_list[i], (size_t)cap * 4));
     T(A(&e->d_rlist[i], (size_t)cap * 4));
   }
-  T(A(&e->d_counts, (size_t)(e->L + 4) * 4));
-  T(A(&e->d_rcounts, (size_t)(e->L + 4) * 4));
   T(A(&e->d_stamp, (size_t)cap * 4));
+  {
+    const int32_t S = e->L + 4;
+    int32_t at = 0;
+    auto part = [&](int32_t n) {
+      at += n;
+      return at - n;
+    };
+    const int32_t o_counts = part(S), o_rcounts = part(S), o_scounts = part(S), o_tcounts = part(S),
+                  o_mcounts = part(S), o_ccount = part(4), o_ncand = part(4), o_fb = part(4),
+                  o_fb2 = part(4);
+    e->ctl_clear = at;
+    const int32_t o_choice = part(4), o_err = part(4), o_id = part(4);
+    e->ctl_size = at;
+    T(A(&e->d_ctl, (size_t)at * 4));
+    if (rc == cudaSuccess) {
+      e->d_counts = e->d_ctl + o_counts;
+      e->d_rcounts = e->d_ctl + o_rcounts;
+      e->d_scounts = e->d_ctl + o_scounts;
+      e->d_tcounts = e->d_ctl + o_tcounts;
+      e->d_mcounts = e->d_ctl + o_mcounts;
+      e->d_ccount = e->d_ctl + o_ccount;
+      e->d_ncand = e->d_ctl + o_ncand;
+      e->d_fbcount = e->d_ctl + o_fb;
+      e->d_fbcount2 = e->d_ctl + o_fb2;
+      e->d_choice = e->d_ctl + o_choice;
+      e->d_err = e->d_ctl + o_err;
+      e->d_idcount = e->d_ctl + o_id;
+    }
+  }
   T(A(&e->d_clist, (size_t)K * 4));
-  T(A(&e->d_ccount, 16));
   T(A(&e->d_cand, (size_t)K * 4));
-  T(A(&e->d_ncand, 16));
   T(A(&e->d_bins, (size_t)K * 16 * 4));
   T(A(&e->d_cslot, (size_t)cap * 4));
   T(A(&e->d_iscent, (size_t)cap * 4));
@@ -480,9 +499,7 @@ int ensure_buffers(sdnn_engine* e, int64_t rows) {
   T(A(&e->d_flags, (size_t)cap * 4));
   T(A(&e->d_state, (size_t)cap * 4));
   T(A(&e->d_pre, (size_t)K * N * 4));
-  T(A(&e->d_err, 16));
   T(A(&e->d_ids, (size_t)cap * 4));
-  T(A(&e->d_idcount, 16));
   T(A(&e->d_fallback, (size_t)cap * 4));
   if (e->sparse_built) {
     // a sparse row's update runs on one warp, entry after entry: rows with
@@ -494,9 +511,7 @@ int ensure_buffers(sdnn_engine* e, int64_t rows) {
       T(A(&e->d_sp_cnt[i], (size_t)cap * 4));
       T(A(&e->d_slist[i], (size_t)cap * 4));
     }
-    T(A(&e->d_scounts, (size_t)(e->L + 4) * 4));
     T(A(&e->d_rtmp, (size_t)cap * 4));
-    T(A(&e->d_tcounts, (size_t)(e->L + 4) * 4));
   }
   // grid chain rows: a fresh buffer per layer (wide layouts only, where it runs)
   if (e->N >= 16384) T(A(&e->d_gscratch, grid_chain_scratch_floats(e->L, e->nq, e->Q) * 4));
@@ -515,17 +530,13 @@ int ensure_buffers(sdnn_engine* e, int64_t rows) {
     T(A(&e->d_mrep, (size_t)P * 8));
     T(A(&e->d_mpos, (size_t)cap * 4));
     T(A(&e->d_mlist, (size_t)cap * 4));
-    T(A(&e->d_mcounts, (size_t)(e->L + 4) * 4));
     if (rc == cudaSuccess) rc = cudaMemset(e->d_alias, 0xFF, (size_t)cap * 4);
   }
-  T(A(&e->d_fbcount, 16));
   T(A(&e->d_rows, 16));
   T(A(&e->d_pcounts, (size_t)kMaxPieces * (e->L + 2) * 4));
-  T(A(&e->d_choice, 16));
   T(A(&e->d_plist[0], (size_t)cap * 4));
   T(A(&e->d_plist[1], (size_t)cap * 4));
   T(A(&e->d_fallback2, (size_t)cap * 4));
-  T(A(&e->d_fbcount2, 16));
   if (rc == cudaSuccess) T(cudaMallocHost((void**)&e->h_counts, 16));
   if (rc != cudaSuccess) {
     free_buffers(e);
@@ -533,7 +544,7 @@ int ensure_buffers(sdnn_engine* e, int64_t rows) {
     return fail(e, SDNN_ERR_OOM, std::string("device allocation failed: ") + cudaGetErrorString(rc));
   }
   e->cap = cap;
-  CK(cudaMemsetAsync(e->d_err, 0, 16, e->stream));
+  CK(cudaMemsetAsync(e->d_ctl, 0, (size_t)e->ctl_size * 4, e->stream));
   return SDNN_OK;
 }
 
@@ -1019,13 +1030,30 @@ int enqueue_merge(sdnn_engine* e, int l) {
   return SDNN_OK;
 }
 
-// Clears what the last inference left: tile flags of layer 0, merge steps.
-int enqueue_clear(sdnn_engine* e) {
-  if (e->bits_on)
-    CK(cudaMemsetAsync(e->d_tile_state, 0, (size_t)((e->cap + 31) / 32) * 4, e->stream));
-  if (!merging_on(e)) return SDNN_OK;
-  CK(cudaMemsetAsync(e->d_mcounts, 0, (size_t)(e->L + 4) * 4, e->stream));
-  launch_dedup_clear(e->d_rows, e->d_mtable, e->d_mrep, e->mmask, e->stream);
+// Starts an inference: the identity row list, the counters and every per-row
+// state cleared, and what the merge steps and layer 0 keep, in one launch.
+int enqueue_begin(sdnn_engine* e, int32_t* list, int32_t* d_flags, int32_t* pcounts,
+                  int32_t pcounts_n) {
+  BeginArgs b{};
+  b.nrows = e->d_rows;
+  b.list = list;
+  b.counts = e->d_ctl;
+  b.counts_n = e->ctl_clear;
+  b.zero[0] = d_flags;
+  b.zero[1] = e->d_state;
+  b.zero[2] = e->d_stamp;
+  b.zero[3] = e->d_iscent;
+  b.zero[4] = e->d_resflag;
+  b.alias = e->d_alias;
+  if (merging_on(e)) {
+    b.table = e->d_mtable;
+    b.slot_rep = e->d_mrep;
+    b.mask = e->mmask;
+  }
+  b.tile_state = e->bits_on ? e->d_tile_state : nullptr;
+  b.extra = pcounts;
+  b.extra_n = pcounts_n;
+  launch_begin(b, e->stream);
   e->launches++;
   CK(cudaGetLastError());
   return SDNN_OK;
@@ -1035,11 +1063,11 @@ int enqueue_clear(sdnn_engine* e) {
 // layer 0 of 0/1 inputs takes the binary counting kernels, with the tiles that
 // hold other values sent to the float kernel.
 int enqueue_layer(sdnn_engine* e, int l, const float* in, const int32_t* lin, const int32_t* cin,
-                  int32_t* lout, int32_t* cout) {
+                  int32_t* lout, int32_t* cout, bool piece = false) {
   const cudaStream_t s = e->stream;
   const bool bits = l == 0 && e->dl[0].sums && e->bits_on;
   if (!bits) return layer_launch(e, l, EPI_PLAIN, in, e->d_y[l & 1], lin, cin, lout, cout);
-  CK(cudaMemsetAsync(e->d_fbcount, 0, 16, s));
+  if (piece) CK(cudaMemsetAsync(e->d_fbcount, 0, 16, s));  // (the lane's last piece used it)
   Layer0Args b{};
   b.idx = e->dl[0].idx;
   b.grp_blk = e->dl[0].grp;
@@ -1126,7 +1154,7 @@ int enqueue_piece(sdnn_engine* e, int p, int64_t r0, int64_t n, int m, const flo
     const bool merge = last && merge_after(e, l, effective_threshold(e));
     int32_t* lout = !last ? e->d_plist[(l + 1) & 1] + r0 : merge ? e->d_mlist : e->d_list[m & 1];
     int32_t* cout = !last ? pc + l + 1 : (merge ? e->d_mcounts : e->d_counts) + m;
-    int rc = enqueue_layer(e, l, in, e->d_plist[l & 1] + r0, pc + l, lout, cout);
+    int rc = enqueue_layer(e, l, in, e->d_plist[l & 1] + r0, pc + l, lout, cout, true);
     if (rc) {
       e->bits_tile0 = 0;
       return rc;
@@ -1154,11 +1182,7 @@ int enqueue(sdnn_engine* e, int phase, int64_t rows, const float* d_in, int32_t*
   if (phase == PH_ALL || phase == PH_PRE) {
     if (e->pipe_start == 0) {
       if ((rc = record(e, 0, capturing))) return rc;
-      CK(cudaMemsetAsync(e->d_counts, 0, (size_t)(L + 4) * 4, s));
-      launch_begin_rows(e->d_rows, e->d_list[0], e->d_counts, d_flags, e->d_state, e->d_stamp,
-                        e->d_alias, s);
-      e->launches++;
-      if ((rc = enqueue_clear(e))) return rc;
+      if ((rc = enqueue_begin(e, e->d_list[0], d_flags, nullptr, 0))) return rc;
     }
     if ((rc = enqueue_plain_layers(e, d_in, T, capturing))) return rc;
   }
@@ -1167,15 +1191,6 @@ int enqueue(sdnn_engine* e, int phase, int64_t rows, const float* d_in, int32_t*
       launch_copy_rows(e->d_rows, d_in, ybuf, e->N, s);
       e->launches++;
     }
-    CK(cudaMemsetAsync(e->d_rcounts, 0, (size_t)(L + 4) * 4, s));
-    if (e->sparse_res) {
-      CK(cudaMemsetAsync(e->d_scounts, 0, (size_t)(L + 4) * 4, s));
-      CK(cudaMemsetAsync(e->d_tcounts, 0, (size_t)(L + 4) * 4, s));
-    }
-    launch_zero_rows(e->d_rows, e->d_iscent, e->d_resflag, s);
-    e->launches++;
-    CK(cudaMemsetAsync(e->d_ccount, 0, 16, s));
-    CK(cudaMemsetAsync(e->d_ncand, 0, 16, s));
     ClusterArgs c{};
     c.y = ybuf;
     c.live = live;
@@ -1293,19 +1308,16 @@ int enqueue(sdnn_engine* e, int phase, int64_t rows, const float* d_in, int32_t*
   }
   if (phase == PH_FINISH) {
     const int pf = L - T;
-    launch_mark_rows(e->d_rlist[pf & 1], e->d_rcounts + pf, e->d_resflag, 1, s);
-    if (e->sparse_res) {
-      // the last sparse rows, written densely into the final buffer: from here
-      // on every residue row reads the same way
-      launch_densify(e->d_slist[pf & 1], e->d_scounts + pf, sparse_rows(e, pf & 1),
-                     e->d_y[(L - 1) & 1], e->N, e->num_sms, s);
-      launch_mark_rows(e->d_slist[pf & 1], e->d_scounts + pf, e->d_resflag, 1, s);
-      e->launches += 2;
-    }
+    // marks the rows that still have a residue; the last sparse rows are written
+    // densely into the final buffer: from here on every residue row reads the
+    // same way
+    const SparseRows none{};
+    launch_finish_rows(e->d_rlist[pf & 1], e->d_rcounts + pf, e->sparse_res ? e->d_slist[pf & 1] : nullptr,
+                       e->d_scounts + pf, e->sparse_res ? sparse_rows(e, pf & 1) : none,
+                       e->d_y[(L - 1) & 1], e->d_resflag, e->N, e->num_sms, s);
     launch_recover(e->d_y[(L - 1) & 1], live, live_count, e->d_cslot, e->d_clist, e->d_iscent,
-                   e->d_resflag, e->N, d_flags, s);
-    launch_mark_rows(live, live_count, e->d_state, 2, s);
-    e->launches += 3;
+                   e->d_resflag, e->N, d_flags, e->d_state, e->num_sms, s);
+    e->launches += 2;
     if (merging_on(e)) {
       launch_resolve_alias(e->d_rows, e->d_alias, d_flags, L, s);
       e->launches++;
@@ -1317,9 +1329,9 @@ int enqueue(sdnn_engine* e, int phase, int64_t rows, const float* d_in, int32_t*
       if ((rc = record(e, 2, capturing))) return rc;
     }
     if ((rc = record(e, 3, capturing))) return rc;
-    launch_identify(e->d_y[(L - 1) & 1], e->d_list[L & 1], e->d_counts + L, e->N, d_flags, s);
-    launch_mark_rows(e->d_list[L & 1], e->d_counts + L, e->d_state, 1, s);
-    e->launches += 2;
+    launch_identify(e->d_y[(L - 1) & 1], e->d_list[L & 1], e->d_counts + L, e->N, d_flags,
+                    e->d_state, e->num_sms, s);
+    e->launches++;
     if (merging_on(e)) {  // SNICIT with the threshold at or past the last layer
       launch_resolve_alias(e->d_rows, e->d_alias, d_flags, L, s);
       e->launches++;
@@ -1996,13 +2008,9 @@ int run_streamed(sdnn_engine* e, const float* Y0, int64_t n, int m, int P) {
   int rc;
   if ((rc = record(e, 0, false))) return rc;
   launch_set_scalar(e->d_rows, (int32_t)n, s);
-  CK(cudaMemsetAsync(e->d_counts, 0, (size_t)(e->L + 4) * 4, s));
-  CK(cudaMemsetAsync(e->d_pcounts, 0, (size_t)P * (e->L + 2) * 4, s));  // the layers append
-  // identity rows into the pieces' layer-0 lists
-  launch_begin_rows(e->d_rows, e->d_plist[0], e->d_counts, e->d_flags, e->d_state, e->d_stamp,
-                    e->d_alias, s);
-  e->launches += 2;
-  if ((rc = enqueue_clear(e))) return rc;
+  // identity rows into the pieces' layer-0 lists (the layers append to the rest)
+  e->launches++;
+  if ((rc = enqueue_begin(e, e->d_plist[0], e->d_flags, e->d_pcounts, P * (e->L + 2)))) return rc;
   // two lanes: even and odd pieces
   const bool two = true;
   if (two) {

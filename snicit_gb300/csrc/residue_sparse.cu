@@ -27,9 +27,9 @@
 //                          row when it grew past SC, or dropped from the lists
 //                          when it is all zero (the row has converged to its
 //                          centroid);
-//   densify_kernel         the final sparse rows written densely into the last
+//   finish_rows_kernel     the final sparse rows written densely into the last
 //                          layer's buffer, so recovery reads every residue row
-//                          the same way.
+//                          the same way, and every residue row marked.
 //
 // A layer has tens of such rows at most, so these wait for memory, row by row.
 // With one warp per row, a bitmap of the outputs reached kept with shared
@@ -44,30 +44,6 @@ namespace {
 constexpr unsigned kFull = 0xffffffffu;
 
 __device__ __forceinline__ float clamp_hi(float v, float hi) { return fminf(hi, fmaxf(0.f, v)); }
-
-// Launched with programmatic stream serialization (like the layer kernel):
-// the next launch may be scheduled now; everything this kernel reads comes
-// from its predecessors, so it waits for them before the first read.
-__device__ __forceinline__ void pdl_prologue() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
-template <typename... Args>
-cudaError_t launch_pdl(void (*fn)(Args...), int grid, int threads, size_t smem, cudaStream_t s,
-                       Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, fn, args...);
-}
 
 constexpr int kRowWarps = 4;  // warps of a CTA that share a residue row
 constexpr int kStage = kRowWarps * 32;   // entries whose edges are staged at a time
@@ -279,15 +255,18 @@ __global__ void __launch_bounds__(kRowWarps * 32) sparse_residue_kernel(const Sp
   }
 }
 
-__global__ void densify_kernel(const int32_t* list, const int32_t* count, SparseRows rows,
-                               float* y, int32_t N) {
+__global__ void finish_rows_kernel(const int32_t* dense_list, const int32_t* dense_count,
+                                   const int32_t* sparse_list, const int32_t* sparse_count,
+                                   SparseRows rows, float* y, int32_t* res_flag, int32_t N) {
   pdl_prologue();
-  const int n = *count;
+  const int nd = *dense_count, n = sparse_list ? *sparse_count : 0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nd; i += gridDim.x * blockDim.x)
+    res_flag[dense_list[i]] = 1;
   const int lane = threadIdx.x & 31;
   const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   for (int i = wid; i < n; i += nw) {
-    const int r = list[i];
+    const int r = sparse_list[i];
     float* dst = y + (size_t)r * N;
     for (int c = lane; c < N; c += 32) dst[c] = 0.f;
     __syncwarp();
@@ -295,6 +274,7 @@ __global__ void densify_kernel(const int32_t* list, const int32_t* count, Sparse
     const int32_t* ei = rows.idx + (size_t)r * rows.cap;
     const float* ev = rows.val + (size_t)r * rows.cap;
     for (int e = lane; e < cnt; e += 32) dst[ei[e]] = ev[e];
+    if (lane == 0) res_flag[r] = 1;
     __syncwarp();
   }
 }
@@ -326,9 +306,12 @@ cudaError_t launch_sparse_residue(const SparseResArgs& a, int num_sms, cudaStrea
   return launch_pdl(sparse_residue_kernel, num_sms * per_sm, kRowWarps * 32, smem, s, a);
 }
 
-void launch_densify(const int32_t* list, const int32_t* count, const SparseRows& rows, float* y,
-                    int32_t N, int num_sms, cudaStream_t s) {
-  launch_pdl(densify_kernel, num_sms * 4, 256, 0, s, list, count, rows, y, N);
+void launch_finish_rows(const int32_t* dense_list, const int32_t* dense_count,
+                        const int32_t* sparse_list, const int32_t* sparse_count,
+                        const SparseRows& rows, float* y, int32_t* res_flag, int32_t N, int num_sms,
+                        cudaStream_t s) {
+  launch_pdl(finish_rows_kernel, num_sms * 2, 256, 0, s, dense_list, dense_count, sparse_list,
+             sparse_count, rows, y, res_flag, N);
 }
 
 }  // namespace sdnn

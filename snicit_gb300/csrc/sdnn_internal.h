@@ -79,6 +79,31 @@ bool layer_instance_exists(const LayerKernelKey& key);
 // Sets the max dynamic shared memory attribute of an instance.
 cudaError_t layer_prepare(const LayerKernelKey& key, size_t smem);
 
+// A launch with programmatic stream serialization: the kernel may be scheduled
+// while its predecessor on the stream finishes, and waits for it with
+// pdl_prologue() (or griddepcontrol.wait) before it reads anything.
+template <typename... Args>
+inline cudaError_t launch_pdl(void (*fn)(Args...), int grid, int threads, size_t smem,
+                              cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, fn, args...);
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void pdl_prologue() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+#endif
+
 // Layer kernel with the slot lists in tensor memory (layer_resident.cu): the
 // plan for a layer, fn == nullptr where it does not apply (N outside 1024 ..
 // 4096, or lists too deep to keep).
@@ -195,19 +220,31 @@ void launch_post_choice(const PostChoiceArgs& a, cudaGraphConditionalHandle h, c
 // (row counts of the layers run piece by piece).
 void launch_sum_piece_counts(const int32_t* piece_counts, int pieces, int stride, int layers,
                              int32_t* counts, cudaStream_t s);
-// list[i] = i, zero_a[i] = zero_b[i] = zero_c[i] = 0 and neg[i] = -1 for i < *nrows;
-// *count = *nrows
-void launch_begin_rows(const int32_t* nrows, int32_t* list, int32_t* count, int32_t* zero_a,
-                       int32_t* zero_b, int32_t* zero_c, int32_t* neg, cudaStream_t s);
-void launch_zero_rows(const int32_t* nrows, int32_t* a, int32_t* b, cudaStream_t s);
+// Start of an inference of n = *nrows rows: list[i] = i, zero[k][i] = 0 and
+// alias[i] = -1 for i < n; counts[0] = n, the rest of counts and extra 0; the
+// merge table's entries in use empty (dedup.cu; mask 0: none); tile_state (one
+// per 32 rows) 0.
+struct BeginArgs {
+  const int32_t* nrows;
+  int32_t* list;
+  int32_t* counts;
+  int32_t counts_n;
+  int32_t* zero[5];
+  int32_t* alias;
+  unsigned long long* table;
+  unsigned long long* slot_rep;
+  uint32_t mask;
+  int32_t* tile_state;
+  int32_t* extra;
+  int32_t extra_n;
+};
+void launch_begin(const BeginArgs& a, cudaStream_t s);
 void launch_copy_rows(const int32_t* nrows, const float* src, float* dst, int32_t N, cudaStream_t s);
+// flags[r] = any entry > 0, state[r] = 1 for the listed rows
 void launch_identify(const float* y, const int32_t* list, const int32_t* count, int32_t N,
-                     int32_t* flags, cudaStream_t s);
+                     int32_t* flags, int32_t* state, int num_sms, cudaStream_t s);
 void launch_flags_to_ids(const int32_t* flags, int32_t n, int32_t* ids, int32_t* count,
                          cudaStream_t s);
-void launch_mark_rows(const int32_t* list, const int32_t* count, int32_t* flags, int32_t value,
-                      cudaStream_t s);
-
 // SNICIT threshold stage.
 struct ClusterArgs {
   float* y;                 // [rows][N] activations at the threshold, rewritten to residues
@@ -231,10 +268,11 @@ void launch_cluster(const ClusterArgs& a, int num_sms, cudaStream_t s);
 
 // Recovery (SNICIT.hpp:644 recover): flags[r] = any(c + delta > 0) for every
 // live row at the threshold; rows absent from the final residue list have
-// delta == 0.
+// delta == 0.  state[r] = 2.
 void launch_recover(const float* y, const int32_t* live, const int32_t* live_count,
                     const int32_t* cslot, const int32_t* clist, const int32_t* is_centroid,
-                    const int32_t* res_flag, int32_t N, int32_t* flags, cudaStream_t s);
+                    const int32_t* res_flag, int32_t N, int32_t* flags, int32_t* state,
+                    int num_sms, cudaStream_t s);
 // Final activations of every row into out[rows][N]: state 0 = dead (zeros),
 // 1 = plain final row, 2 = SNICIT live row (centroid, or centroid + residue).
 // perm[c] = position of neuron c in the final buffer (nullptr = identity).
@@ -275,9 +313,12 @@ struct DedupArgs {
   uint32_t mask;                // table entries - 1 (a power of 2 >= 2 x rows, minus 1)
 };
 cudaError_t launch_dedup(const DedupArgs& a, int num_sms, cudaStream_t s);
-// table[i] = 0 and slot_rep[i] = ~0 for the entries an inference of *nrows rows uses
-void launch_dedup_clear(const int32_t* nrows, unsigned long long* table,
-                        unsigned long long* slot_rep, uint32_t mask, cudaStream_t s);
+// Entries in use for an inference of `rows` rows (a power of two >= 2 rows).
+__host__ __device__ inline uint32_t dedup_table_mask(int32_t rows, uint32_t cap_mask) {
+  uint32_t m = 1023u;
+  while (m < 2u * (uint32_t)rows && m < cap_mask) m = 2u * m + 1u;
+  return m < cap_mask ? m : cap_mask;
+}
 // alias[r] := root of r's chain, flags[r] := flags[root] for merged rows.
 void launch_resolve_alias(const int32_t* nrows, int32_t* alias, int32_t* flags, int32_t max_depth,
                           cudaStream_t s);
@@ -318,7 +359,11 @@ void launch_split_residue(const float* y, const int32_t* list, const int32_t* co
                           int32_t* sparse_list, int32_t* sparse_count, int32_t N, int num_sms,
                           cudaStream_t s);
 cudaError_t launch_sparse_residue(const SparseResArgs& a, int num_sms, cudaStream_t s);
-void launch_densify(const int32_t* list, const int32_t* count, const SparseRows& rows, float* y,
-                    int32_t N, int num_sms, cudaStream_t s);
+// res_flag[r] = 1 for the rows of both lists; the sparse ones (list nullptr:
+// none) written densely into y.
+void launch_finish_rows(const int32_t* dense_list, const int32_t* dense_count,
+                        const int32_t* sparse_list, const int32_t* sparse_count,
+                        const SparseRows& rows, float* y, int32_t* res_flag, int32_t N, int num_sms,
+                        cudaStream_t s);
 
 }  // namespace sdnn
