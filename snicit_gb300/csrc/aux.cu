@@ -136,57 +136,6 @@ void launch_identify(const float* y, const int32_t* list, const int32_t* count, 
   launch_pdl(identify_kernel, num_sms * 4, 256, 0, s, y, list, count, N, flags, state);
 }
 
-// Ordered compaction: ids = sorted indices i with flags[i] != 0.  One CTA.
-__global__ void __launch_bounds__(1024) flags_to_ids_kernel(const int32_t* flags, int32_t n,
-                                                            int32_t* ids, int32_t* count) {
-  __shared__ int wsum[32];
-  __shared__ int s_total;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  int base = 0;
-  for (int start = 0; start < n; start += 4096) {
-    int f[4];
-    int local = 0;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int i = start + tid * 4 + u;
-      f[u] = (i < n && flags[i] != 0) ? 1 : 0;
-      local += f[u];
-    }
-    // inclusive warp scan of local
-    int inc = local;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o) inc += v;
-    }
-    if (lane == 31) wsum[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-      int w = wsum[lane];
-      int winc = w;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, winc, o);
-        if (lane >= o) winc += v;
-      }
-      wsum[lane] = winc - w;
-      if (lane == 31) s_total = winc;
-    }
-    __syncthreads();
-    int pos = base + wsum[warp] + inc - local;
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (f[u]) ids[pos++] = start + tid * 4 + u;
-    base += s_total;
-    __syncthreads();
-  }
-  if (tid == 0) *count = base;
-}
-void launch_flags_to_ids(const int32_t* flags, int32_t n, int32_t* ids, int32_t* count,
-                         cudaStream_t s) {
-  flags_to_ids_kernel<<<1, 1024, 0, s>>>(flags, n, ids, count);
-}
-
 // ------------------------------------------------------- SNICIT threshold stage
 //
 // Reference: reduction + centroid_sel (src/SDGC/SNICIT/kernel.hpp:138-194),

@@ -36,6 +36,7 @@ using namespace sdnn;
 namespace {
 
 struct DevLayer {
+  uint8_t* mem = nullptr;  // holds everything below
   uint2* idx = nullptr;
   float4* val = nullptr;
   int32_t* grp = nullptr;
@@ -122,6 +123,7 @@ struct sdnn_engine {
   LayerKernelKey key{}, key_general{};  // one weight value / a value per edge
   int threads = 512, threads_general = 512, grid = 0, grid_general = 0, min_split = 1;
   size_t smem = 0;
+  bool kernels_ready = false;  // shared memory limits of the chosen kernels raised
 
   // device weights (owned, or borrowed from weights_owner: a server's slot
   // engines read the model engine's copy; share_users counts the borrowers)
@@ -159,8 +161,6 @@ struct sdnn_engine {
   int32_t* d_state = nullptr;
   float* d_pre = nullptr;
   int32_t* d_err = nullptr;
-  int32_t* d_ids = nullptr;
-  int32_t* d_idcount = nullptr;
   float* d_in = nullptr;
   int32_t* d_rows = nullptr;      // row count of the current inference
   int32_t* d_fallback = nullptr;  // layer-0 rows of non-binary tiles
@@ -223,7 +223,10 @@ struct sdnn_engine {
   int last_full = 0;       // 1 + slot of the whole-inference graph that ran last, 0: none
   int32_t* d_choice = nullptr;  // body taken by the last whole-inference graph
   int run_launches = 0;
-  int32_t* h_counts = nullptr;  // pinned: residue rows and centroids after clustering
+  int32_t* h_ctl = nullptr;    // pinned: the control block, read back after an inference
+  int32_t* h_flags = nullptr;  // pinned: [cap] categories of a host call
+  bool report_valid = false;   // h_ctl holds the last inference's counters
+  const int32_t* host(const int32_t* d) const { return h_ctl + (d - d_ctl); }
   int chain_cap = 0;            // centroid rows the cluster chain kernel can carry
   int chain_kc = 1;
   int chain_kind = 0;           // 1 cluster chain kernel, 2 grid chain kernel
@@ -274,15 +277,7 @@ void free_weights(sdnn_engine* e) {
   dfree(e->d_perm_final);
   dfree(e->d_layer_table);
   for (auto& d : e->dl) {
-    dfree(d.idx);
-    dfree(d.val);
-    dfree(d.grp);
-    dfree(d.lists);
-    dfree(d.bias);
-    dfree(d.sums);
-    dfree(d.tr_off);
-    dfree(d.tr_out);
-    dfree(d.tr_val);
+    dfree(d.mem);
   }
   e->dl.clear();
 }
@@ -305,7 +300,6 @@ void free_buffers(sdnn_engine* e) {
   dfree(e->d_flags);
   dfree(e->d_state);
   dfree(e->d_pre);
-  dfree(e->d_ids);
   dfree(e->d_in);
   dfree(e->d_fallback);
   dfree(e->d_bits);
@@ -331,8 +325,10 @@ void free_buffers(sdnn_engine* e) {
     dfree(e->d_slist[i]);
   }
   dfree(e->d_rtmp);
-  if (e->h_counts) cudaFreeHost(e->h_counts);
-  e->h_counts = nullptr;
+  if (e->h_ctl) cudaFreeHost(e->h_ctl);
+  if (e->h_flags) cudaFreeHost(e->h_flags);
+  e->h_ctl = e->h_flags = nullptr;
+  e->report_valid = false;
   e->cap = 0;
 }
 
@@ -472,7 +468,7 @@ int ensure_buffers(sdnn_engine* e, int64_t rows) {
                   o_mcounts = part(S), o_ccount = part(4), o_ncand = part(4), o_fb = part(4),
                   o_fb2 = part(4);
     e->ctl_clear = at;
-    const int32_t o_choice = part(4), o_err = part(4), o_id = part(4);
+    const int32_t o_choice = part(4), o_err = part(4);
     e->ctl_size = at;
     T(A(&e->d_ctl, (size_t)at * 4));
     if (rc == cudaSuccess) {
@@ -487,7 +483,6 @@ int ensure_buffers(sdnn_engine* e, int64_t rows) {
       e->d_fbcount2 = e->d_ctl + o_fb2;
       e->d_choice = e->d_ctl + o_choice;
       e->d_err = e->d_ctl + o_err;
-      e->d_idcount = e->d_ctl + o_id;
     }
   }
   T(A(&e->d_clist, (size_t)K * 4));
@@ -499,7 +494,6 @@ int ensure_buffers(sdnn_engine* e, int64_t rows) {
   T(A(&e->d_flags, (size_t)cap * 4));
   T(A(&e->d_state, (size_t)cap * 4));
   T(A(&e->d_pre, (size_t)K * N * 4));
-  T(A(&e->d_ids, (size_t)cap * 4));
   T(A(&e->d_fallback, (size_t)cap * 4));
   if (e->sparse_built) {
     // a sparse row's update runs on one warp, entry after entry: rows with
@@ -537,7 +531,8 @@ int ensure_buffers(sdnn_engine* e, int64_t rows) {
   T(A(&e->d_plist[0], (size_t)cap * 4));
   T(A(&e->d_plist[1], (size_t)cap * 4));
   T(A(&e->d_fallback2, (size_t)cap * 4));
-  if (rc == cudaSuccess) T(cudaMallocHost((void**)&e->h_counts, 16));
+  if (rc == cudaSuccess) T(cudaMallocHost((void**)&e->h_ctl, (size_t)e->ctl_size * 4));
+  if (rc == cudaSuccess) T(cudaMallocHost((void**)&e->h_flags, (size_t)cap * 4));
   if (rc != cudaSuccess) {
     free_buffers(e);
     cudaGetLastError();
@@ -650,12 +645,21 @@ int upload_layer(sdnn_engine* e, int l, const PackedView& p, std::string& err) {
   }
   const size_t nslot = (size_t)p.nblocks * 128;
   const size_t ngrp = (size_t)e->G * e->nq + 1;
-  cudaError_t rc = cudaSuccess;
-  auto T = [&](cudaError_t r) {
-    if (rc == cudaSuccess) rc = r;
+  // everything of the layer in one host image, then one allocation and one copy
+  std::vector<uint8_t> image;
+  auto put = [&](const void* src, size_t bytes) {  // returns the part's offset
+    const size_t at = (image.size() + 255) / 256 * 256;
+    image.resize(at + bytes);
+    if (bytes) std::memcpy(image.data() + at, src, bytes);
+    return at;
   };
-  T(cudaMalloc((void**)&d.idx, std::max<size_t>(nslot * 2, 16)));
-  T(cudaMalloc((void**)&d.grp, ngrp * 4));
+  const size_t none = ~(size_t)0;
+  size_t o_val = none, o_bias = none, o_sums = none, o_tr_off = none, o_tr_out = none, o_tr_val = none;
+  image.reserve(nslot * (p.constw ? 2 : 6) + ngrp * 12 +
+                (e->sparse_built ? (size_t)p.nnz * (p.constw ? 2 : 6) : 0) + (size_t)e->N * 8 + 4096);
+  const size_t o_idx = put(p.idx, nslot * 2);
+  const size_t o_grp = put(p.grp_blk, ngrp * 4);
+  const int32_t scale = slot_index_in_bytes(e->Q) ? 4 : 1;
   // slots in use of every list: its last block of 4 is rarely full
   std::vector<int2> lists(ngrp - 1);
   for (size_t i = 0; i + 1 < ngrp; ++i) {
@@ -664,35 +668,26 @@ int upload_layer(sdnn_engine* e, int l, const PackedView& p, std::string& err) {
     for (; slots > 0; --slots) {
       const uint16_t* lane0 = p.idx + (size_t)(first + (slots - 1) / 4) * 128 + (slots - 1) % 4;
       bool used = false;
-      for (int lane = 0; lane < 32 && !used; ++lane)
-        used = lane0[lane * 4] / (slot_index_in_bytes(e->Q) ? 4 : 1) < e->Q;
+      for (int lane = 0; lane < 32 && !used; ++lane) used = lane0[lane * 4] < e->Q * scale;
       if (used) break;
     }
     lists[i] = make_int2(first, slots);
   }
-  T(cudaMalloc((void**)&d.lists, lists.size() * sizeof(int2)));
-  if (!p.constw) T(cudaMalloc((void**)&d.val, std::max<size_t>(nslot * 4, 16)));
-  if (p.bias) T(cudaMalloc((void**)&d.bias, (size_t)e->N * 4));
-  if (rc == cudaSuccess && nslot) T(cudaMemcpy(d.idx, p.idx, nslot * 2, cudaMemcpyHostToDevice));
-  if (rc == cudaSuccess) T(cudaMemcpy(d.grp, p.grp_blk, ngrp * 4, cudaMemcpyHostToDevice));
-  if (rc == cudaSuccess)
-    T(cudaMemcpy(d.lists, lists.data(), lists.size() * sizeof(int2), cudaMemcpyHostToDevice));
-  if (rc == cudaSuccess && d.val && nslot)
-    T(cudaMemcpy(d.val, p.val, nslot * 4, cudaMemcpyHostToDevice));
-  if (rc == cudaSuccess && p.bias) {
+  const size_t o_lists = put(lists.data(), lists.size() * sizeof(int2));
+  if (!p.constw) o_val = put(p.val, nslot * 4);
+  if (p.bias) {
     // per-neuron bias follows its neuron to its position
     std::vector<float> b(e->N);
     for (int c = 0; c < e->N; ++c) b[p.pos ? p.pos[c] : c] = p.bias[c];
-    T(cudaMemcpy(d.bias, b.data(), (size_t)e->N * 4, cudaMemcpyHostToDevice));
+    o_bias = put(b.data(), (size_t)e->N * 4);
   }
-  if (rc == cudaSuccess && l == 0 && p.constw && p.max_depth < 128 && p.max_in_degree < 128) {
+  if (l == 0 && p.constw && p.max_depth < 128 && p.max_in_degree < 128) {
     // the largest in-degree, from the slots themselves
     d.max_in_degree = 0;
     for (int32_t g = 0; g < e->G; ++g) {
       int32_t deg[32] = {};
       for (int32_t b = p.grp_blk[g * e->nq]; b < p.grp_blk[(g + 1) * e->nq]; ++b)
-        for (int k = 0; k < 128; ++k)
-          deg[k >> 2] += p.idx[(size_t)b * 128 + k] / (slot_index_in_bytes(e->Q) ? 4 : 1) < e->Q;
+        for (int k = 0; k < 128; ++k) deg[k >> 2] += p.idx[(size_t)b * 128 + k] < e->Q * scale;
       d.max_in_degree = std::max(d.max_in_degree, *std::max_element(deg, deg + 32));
     }
     // the float kernel adds w once per active edge: reproduce those sums
@@ -702,13 +697,11 @@ int upload_layer(sdnn_engine* e, int l, const PackedView& p, std::string& err) {
       sums[k] = acc;
       acc = acc + p.wconst;
     }
-    T(cudaMalloc((void**)&d.sums, sizeof(sums)));
-    if (rc == cudaSuccess) T(cudaMemcpy(d.sums, sums, sizeof(sums), cudaMemcpyHostToDevice));
+    if (d.max_in_degree < 128) o_sums = put(sums, sizeof(sums));
   }
-  if (rc == cudaSuccess && e->sparse_built) {
+  if (e->sparse_built) {
     // out-edges of every input position, from the packed slots (padding slots
     // point past the chunk and are skipped), each input's edges by output
-    const int32_t scale = slot_index_in_bytes(e->Q) ? 4 : 1;
     const int32_t N = e->N, Q = e->Q;
     std::vector<int32_t> off(N + 1, 0);
     for (int32_t g = 0; g < e->G; ++g)
@@ -741,13 +734,24 @@ int upload_layer(sdnn_engine* e, int l, const PackedView& p, std::string& err) {
         if (!p.constw) tval[t] = edges[t].second;
       }
     }
-    T(cudaMalloc((void**)&d.tr_off, (size_t)(N + 1) * 4));
-    T(cudaMalloc((void**)&d.tr_out, std::max<size_t>(ne * 2, 16)));
-    if (!p.constw) T(cudaMalloc((void**)&d.tr_val, std::max<size_t>(ne * 4, 16)));
-    if (rc == cudaSuccess) T(cudaMemcpy(d.tr_off, off.data(), (size_t)(N + 1) * 4, cudaMemcpyHostToDevice));
-    if (rc == cudaSuccess && ne) T(cudaMemcpy(d.tr_out, tout.data(), ne * 2, cudaMemcpyHostToDevice));
-    if (rc == cudaSuccess && d.tr_val && ne)
-      T(cudaMemcpy(d.tr_val, tval.data(), ne * 4, cudaMemcpyHostToDevice));
+    o_tr_off = put(off.data(), (size_t)(N + 1) * 4);
+    o_tr_out = put(tout.data(), ne * 2);
+    if (!p.constw) o_tr_val = put(tval.data(), ne * 4);
+  }
+  cudaError_t rc = cudaMalloc((void**)&d.mem, std::max<size_t>(image.size(), 16));
+  if (rc == cudaSuccess && !image.empty())
+    rc = cudaMemcpy(d.mem, image.data(), image.size(), cudaMemcpyHostToDevice);
+  if (rc == cudaSuccess) {
+    auto at = [&](size_t o) { return o == none ? nullptr : d.mem + o; };
+    d.idx = (uint2*)at(o_idx);
+    d.grp = (int32_t*)at(o_grp);
+    d.lists = (int2*)at(o_lists);
+    d.val = (float4*)at(o_val);
+    d.bias = (float*)at(o_bias);
+    d.sums = (float*)at(o_sums);
+    d.tr_off = (int32_t*)at(o_tr_off);
+    d.tr_out = (uint16_t*)at(o_tr_out);
+    d.tr_val = (float*)at(o_tr_val);
   }
   e->dl[l] = d;
   if (rc != cudaSuccess) {
@@ -1527,6 +1531,14 @@ int run_full(sdnn_engine* e, int64_t rows, const float* d_in, int32_t* d_flags) 
   return SDNN_OK;
 }
 
+// The control block to the host, with everything enqueued before it complete.
+int read_counters(sdnn_engine* e) {
+  CK(cudaMemcpyAsync(e->h_ctl, e->d_ctl, (size_t)e->ctl_size * 4, cudaMemcpyDeviceToHost, e->stream));
+  CK(cudaStreamSynchronize(e->stream));
+  e->report_valid = true;
+  return SDNN_OK;
+}
+
 int run(sdnn_engine* e, int64_t rows, const float* d_in, int32_t* d_flags) {
   if (rows <= 0) return fail(e, SDNN_ERR_INVALID, "rows must be positive");
   if (rows > e->cap) return fail(e, SDNN_ERR_INVALID, "rows exceed the batch capacity");
@@ -1534,6 +1546,7 @@ int run(sdnn_engine* e, int64_t rows, const float* d_in, int32_t* d_flags) {
   e->last_T = T;
   e->last_rows = rows;
   e->run_launches = 0;
+  e->report_valid = false;
   if (e->pipe_start == 0) e->last_pieces = 0;
   // the graphs read the row count from d_rows (one graph for every count)
   launch_set_scalar(e->d_rows, (int32_t)rows, e->stream);
@@ -1560,13 +1573,10 @@ int run(sdnn_engine* e, int64_t rows, const float* d_in, int32_t* d_flags) {
   } else {
     if ((rc = run_phase(e, 1, PH_PRE, rows, d_in, d_flags))) return rc;
     // what did the clustering leave?  (one small read-back per inference)
-    CK(cudaMemcpyAsync(e->h_counts, e->d_rcounts, 4, cudaMemcpyDeviceToHost, e->stream));
-    CK(cudaMemcpyAsync(e->h_counts + 1, e->d_ccount, 4, cudaMemcpyDeviceToHost, e->stream));
-    e->h_counts[2] = 0;
-    if (e->sparse_res)
-      CK(cudaMemcpyAsync(e->h_counts + 2, e->d_scounts, 4, cudaMemcpyDeviceToHost, e->stream));
-    CK(cudaStreamSynchronize(e->stream));
-    const int residues = e->h_counts[0] + e->h_counts[2], centroids = e->h_counts[1];
+    if ((rc = read_counters(e))) return rc;
+    const int residues = e->host(e->d_rcounts)[0] + e->host(e->d_scounts)[0],
+              centroids = e->host(e->d_ccount)[0];
+    e->report_valid = false;  // (the post-threshold layers are still to come)
     // no residue left: one chain launch carries the centroid rows -- the
     // cluster kernel where the rows fit shared memory (measured faster: 1.6
     // and 7.2 us per layer at N = 4096 and 16384 against 13.8 and 11.8 for the
@@ -1626,22 +1636,24 @@ int prepare(sdnn_engine* e, int64_t rows) {
     rc = choose_kernel(e);
     if (rc) return rc;
   }
-  CK(layer_prepare(e->key, e->smem));
-  CK(layer_prepare(e->key_general, e->smem));
-  if (e->nq == 1)
-    for (bool constw : {true, false}) {
-      const ResidentPlan p = resident_plan(e->N, constw, 0);
-      if (p.fn) CK(resident_prepare(p));
-    }
-  if (e->sparse_built) CK(sparse_residue_prepare(e->N));
+  if (!e->kernels_ready) {
+    CK(layer_prepare(e->key));
+    CK(layer_prepare(e->key_general));
+    if (e->nq == 1)
+      for (bool constw : {true, false}) {
+        const ResidentPlan p = resident_plan(e->N, constw, 0);
+        if (p.fn) CK(resident_prepare(p));
+      }
+    if (e->sparse_built) CK(sparse_residue_prepare(e->N));
+    e->kernels_ready = true;
+  }
   e->bits_on = bits_possible(e) && !(e->cfg.flags & SDNN_FLAG_NO_BINARY_FIRST_LAYER);
   return ensure_buffers(e, rows);
 }
 
-int check_device_error(sdnn_engine* e) {
-  int32_t h = 0;
-  CK(cudaMemcpyAsync(&h, e->d_err, 4, cudaMemcpyDeviceToHost, e->stream));
-  CK(cudaStreamSynchronize(e->stream));
+// The error word among the counters read back last.
+int reported_error(sdnn_engine* e) {
+  const int32_t h = *e->host(e->d_err);
   if (h == DEV_TIMEOUT) {
     cudaMemsetAsync(e->d_err, 0, 4, e->stream);
     return fail(e, SDNN_ERR_TIMEOUT, "a device-side wait timed out");
@@ -1650,13 +1662,21 @@ int check_device_error(sdnn_engine* e) {
   return SDNN_OK;
 }
 
+int check_device_error(sdnn_engine* e) {
+  int rc = read_counters(e);
+  return rc ? rc : reported_error(e);
+}
+
 int collect_stats(sdnn_engine* e) {
   if (!e->pending_stats) return SDNN_OK;
-  CK(cudaStreamSynchronize(e->stream));
+  if (!e->report_valid) {
+    int rc = read_counters(e);
+    if (rc) return rc;
+  }
   const int L = e->L, T = e->last_T;
-  std::vector<int32_t> counts(L + 4), rcounts(L + 4);
-  int32_t ccount = 0;
-  CK(cudaMemcpy(counts.data(), e->d_counts, (size_t)(L + 4) * 4, cudaMemcpyDeviceToHost));
+  const int32_t *counts = e->host(e->d_counts), *rcounts = e->host(e->d_rcounts),
+                *scounts = e->host(e->d_scounts);  // (no sparse rows: zeros)
+  const int32_t ccount = *e->host(e->d_ccount);
   sdnn_stats& st = e->stats;
   std::memset(&st, 0, sizeof(st));
   float ms[4] = {0, 0, 0, 0};
@@ -1668,11 +1688,6 @@ int collect_stats(sdnn_engine* e) {
   int64_t pre = 0, post = 0;
   for (int l = 0; l < T; ++l) pre += counts[l];
   if (T < L) {
-    CK(cudaMemcpy(rcounts.data(), e->d_rcounts, (size_t)(L + 4) * 4, cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(&ccount, e->d_ccount, 4, cudaMemcpyDeviceToHost));
-    std::vector<int32_t> scounts(L + 4, 0);
-    if (e->sparse_res)
-      CK(cudaMemcpy(scounts.data(), e->d_scounts, (size_t)(L + 4) * 4, cudaMemcpyDeviceToHost));
     int64_t sparse = 0;
     for (int p = 0; p < L - T; ++p) {
       post += ccount + rcounts[p] + scounts[p];
@@ -1703,8 +1718,7 @@ int collect_stats(sdnn_engine* e) {
   if (e->last_full) {
     // the device chose the post-threshold path: which body ran
     const FullGraph& fg = e->full[e->last_full - 1];
-    int32_t b = 0;
-    CK(cudaMemcpy(&b, e->d_choice, 4, cudaMemcpyDeviceToHost));
+    int32_t b = *e->host(e->d_choice);
     if (b < 0 || b >= kPostBodies) b = 0;
     st.post_kernel = b == 0 ? 1 : (b & 1) ? 1 + fg.variant[(b - 1) / 2] : 4;
     st.launches += fg.body_launches[b];
@@ -2084,22 +2098,19 @@ int infer_host(sdnn_engine* e, const float* Y0, const uint64_t* bits, int64_t ro
       rc = run(e, n, e->d_in, e->d_flags);
     }
     if (rc) return rc;
+    // categories and counters back in one wait; the ids follow on the host
+    const bool want = flags || ids || count;
+    if (want)
+      CK(cudaMemcpyAsync(e->h_flags, e->d_flags, (size_t)n * 4, cudaMemcpyDeviceToHost, e->stream));
+    if ((rc = check_device_error(e))) return rc;
+    if (flags) std::memcpy(flags + off, e->h_flags, (size_t)n * 4);
     if (ids || count) {
-      launch_flags_to_ids(e->d_flags, (int32_t)n, e->d_ids, e->d_idcount, e->stream);
-      int32_t c = 0;
-      CK(cudaMemcpyAsync(&c, e->d_idcount, 4, cudaMemcpyDeviceToHost, e->stream));
-      CK(cudaStreamSynchronize(e->stream));
-      if (ids && c > 0) {
-        CK(cudaMemcpyAsync(ids + total, e->d_ids, (size_t)c * 4, cudaMemcpyDeviceToHost, e->stream));
-        CK(cudaStreamSynchronize(e->stream));
-        for (int32_t i = 0; i < c; ++i) ids[total + i] += (int32_t)off;
+      for (int64_t i = 0; i < n; ++i) {
+        if (!e->h_flags[i]) continue;
+        if (ids) ids[total] = (int32_t)(off + i);
+        ++total;
       }
-      total += c;
     }
-    if (flags)
-      CK(cudaMemcpyAsync(flags + off, e->d_flags, (size_t)n * 4, cudaMemcpyDeviceToHost, e->stream));
-    rc = check_device_error(e);
-    if (rc) return rc;
     rc = collect_stats(e);
     if (rc) return rc;
     if (off == 0) {
@@ -2159,15 +2170,15 @@ int sdnn_infer_batches_host(sdnn_engine* e, const float* const* inputs, const in
   }
   rc = run(e, total, e->d_in, e->d_flags);
   if (rc) return rc;
+  CK(cudaMemcpyAsync(e->h_flags, e->d_flags, (size_t)total * 4, cudaMemcpyDeviceToHost, e->stream));
+  rc = check_device_error(e);
+  if (rc) return rc;
   off = 0;
   for (int32_t b = 0; b < num_batches; ++b) {
     if (flags && flags[b] && rows[b] > 0)
-      CK(cudaMemcpyAsync(flags[b], e->d_flags + off, (size_t)rows[b] * 4, cudaMemcpyDeviceToHost,
-                         e->stream));
+      std::memcpy(flags[b], e->h_flags + off, (size_t)rows[b] * 4);
     off += rows[b];
   }
-  rc = check_device_error(e);
-  if (rc) return rc;
   return collect_stats(e);
 }
 
@@ -2352,20 +2363,14 @@ int sdnn_get_layer_rows(const sdnn_engine* ce, int64_t* out, int32_t num_layers)
   auto* e = const_cast<sdnn_engine*>(ce);
   if (!e->have_run) return fail(e, SDNN_ERR_STATE, "no inference has run");
   CK(cudaSetDevice(e->dev));
-  CK(cudaStreamSynchronize(e->stream));
+  int rc = read_counters(e);
+  if (rc) return rc;
   const int L = e->L, T = e->last_T;
-  std::vector<int32_t> counts(L + 4), rcounts(L + 4);
-  int32_t ccount = 0;
-  CK(cudaMemcpy(counts.data(), e->d_counts, (size_t)(L + 4) * 4, cudaMemcpyDeviceToHost));
+  const int32_t *counts = e->host(e->d_counts), *rcounts = e->host(e->d_rcounts),
+                *scounts = e->host(e->d_scounts);
   for (int l = 0; l < T; ++l) out[l] = counts[l];
-  if (T < L) {
-    CK(cudaMemcpy(rcounts.data(), e->d_rcounts, (size_t)(L + 4) * 4, cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(&ccount, e->d_ccount, 4, cudaMemcpyDeviceToHost));
-    std::vector<int32_t> scounts(L + 4, 0);
-    if (e->sparse_res)
-      CK(cudaMemcpy(scounts.data(), e->d_scounts, (size_t)(L + 4) * 4, cudaMemcpyDeviceToHost));
-    for (int l = T; l < L; ++l) out[l] = (int64_t)ccount + rcounts[l - T] + scounts[l - T];
-  }
+  for (int l = T; l < L; ++l)
+    out[l] = (int64_t)*e->host(e->d_ccount) + rcounts[l - T] + scounts[l - T];
   return SDNN_OK;
 }
 
@@ -2393,6 +2398,7 @@ int engine_set_tile(sdnn_engine* e, int tile_rows, int threads) {
   e->cfg.tile_rows = tile_rows;
   e->cfg.threads = threads;
   e->grid = 0;
+  e->kernels_ready = false;
   drop_graph(e);
   return choose_kernel(e);
 }
@@ -2442,7 +2448,7 @@ int engine_layer_setup(sdnn_engine* e, int layer, LayerArgs* a, LayerKernelKey* 
   *res = resident_on(e, layer) ? d.res : ResidentPlan{};
   *num_sms = e->num_sms;
   if (res->fn) CK(resident_prepare(*res));
-  else CK(layer_prepare(k, e->smem));
+  else CK(layer_prepare(k));
   *a = LayerArgs{};
   a->w.idx = d.idx;
   a->w.val = d.val;

@@ -645,7 +645,7 @@ cudaError_t launch_layer0_bits(const Layer0Args& a, int num_sms, cudaStream_t s)
   if (!fn || (chunked && !layer0_bits_chunked_supported(a.N, a.Q))) return cudaErrorInvalidValue;
   const int threads = chunked ? kChunkWarps * 32 : kCountWarps * 32;
   const size_t smem = (size_t)((chunked ? a.Q : a.N) + 32) * 4 * (chunked ? 1 : count_buffers(a.N));
-  cudaError_t rc = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t rc = allow_smem(fn);
   if (rc != cudaSuccess) return rc;
   int per_sm = 0;
   rc = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem);

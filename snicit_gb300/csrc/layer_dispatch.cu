@@ -35,17 +35,24 @@ static const LayerInstance* find(const LayerKernelKey& k) {
 
 bool layer_instance_exists(const LayerKernelKey& key) { return find(key) != nullptr; }
 
-cudaError_t layer_prepare(const LayerKernelKey& key, size_t smem) {
+cudaError_t allow_smem(const void* fn) {
+  cudaFuncAttributes at;
+  cudaError_t rc = cudaFuncGetAttributes(&at, fn);
+  if (rc != cudaSuccess) return rc;
+  const int most = 227 * 1024 - (int)at.sharedSizeBytes;
+  if (at.maxDynamicSharedSizeBytes >= most) return cudaSuccess;
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
+cudaError_t layer_prepare(const LayerKernelKey& key) {
   const LayerInstance* e = find(key);
-  if (!e) return cudaErrorInvalidValue;
-  return cudaFuncSetAttribute(e->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  return e ? allow_smem(e->fn) : cudaErrorInvalidValue;
 }
 
 int layer_blocks_per_sm(const LayerKernelKey& key, int threads, size_t smem) {
   const LayerInstance* e = find(key);
   if (!e) return 0;
-  if (cudaFuncSetAttribute(e->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess) {
+  if (allow_smem(e->fn) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }

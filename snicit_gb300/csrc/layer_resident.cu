@@ -407,9 +407,7 @@ ResidentPlan resident_plan(int N, bool constw, int max_depth) {
   return p;
 }
 
-cudaError_t resident_prepare(const ResidentPlan& p) {
-  return cudaFuncSetAttribute(p.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
-}
+cudaError_t resident_prepare(const ResidentPlan& p) { return allow_smem(p.fn); }
 
 cudaError_t launch_layer_resident(const ResidentPlan& p, const LayerArgs& a, int num_sms,
                                   cudaStream_t s) {

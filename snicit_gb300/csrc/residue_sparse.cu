@@ -287,8 +287,7 @@ bool sparse_residue_fits(int N) { return N <= 32768; }
 
 cudaError_t sparse_residue_prepare(int N) {
   if (!sparse_residue_fits(N)) return cudaErrorInvalidValue;
-  return cudaFuncSetAttribute(sparse_residue_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)sparse_residue_smem(N));
+  return allow_smem((const void*)sparse_residue_kernel);
 }
 
 void launch_split_residue(const float* y, const int32_t* list, const int32_t* count,

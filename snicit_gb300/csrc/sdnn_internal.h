@@ -76,8 +76,10 @@ cudaError_t launch_layer(const LayerKernelKey& key, const LayerArgs& a, int grid
 int layer_blocks_per_sm(const LayerKernelKey& key, int threads, size_t smem);
 // True if an instance exists.
 bool layer_instance_exists(const LayerKernelKey& key);
-// Sets the max dynamic shared memory attribute of an instance.
-cudaError_t layer_prepare(const LayerKernelKey& key, size_t smem);
+// Raises a kernel's dynamic shared memory limit as far as the SM allows (never
+// lowers it: engines of several widths share the kernels).
+cudaError_t allow_smem(const void* fn);
+cudaError_t layer_prepare(const LayerKernelKey& key);
 
 // A launch with programmatic stream serialization: the kernel may be scheduled
 // while its predecessor on the stream finishes, and waits for it with
@@ -243,8 +245,7 @@ void launch_copy_rows(const int32_t* nrows, const float* src, float* dst, int32_
 // flags[r] = any entry > 0, state[r] = 1 for the listed rows
 void launch_identify(const float* y, const int32_t* list, const int32_t* count, int32_t N,
                      int32_t* flags, int32_t* state, int num_sms, cudaStream_t s);
-void launch_flags_to_ids(const int32_t* flags, int32_t n, int32_t* ids, int32_t* count,
-                         cudaStream_t s);
+
 // SNICIT threshold stage.
 struct ClusterArgs {
   float* y;                 // [rows][N] activations at the threshold, rewritten to residues
