@@ -50,12 +50,13 @@ static __device__ __align__(256) NoAllocScratch g_noalloc_scratch;
 std::mutex g_addr_mutex;
 NoAllocScratch* g_addr[kMaxDevices] = {};
 
-// Resets the parts of the scratch that must start at zero for this call and
-// lists every row.
-__global__ void noalloc_prepare_kernel(NoAllocScratch* s, int32_t rows) {
+// Resets the parts of the scratch that must start at zero for this call, and
+// the caller's flags, and lists every row.
+__global__ void noalloc_prepare_kernel(NoAllocScratch* s, int32_t* alive, int32_t rows) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x) {
     s->list_in[i] = i;
     s->stamp[i] = 0;
+    alive[i] = 0;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     s->counts[0] = rows;
@@ -64,9 +65,10 @@ __global__ void noalloc_prepare_kernel(NoAllocScratch* s, int32_t rows) {
   }
 }
 
-// Writes the survivor flags (d_alive was zeroed before): 1 for every row the
+// Writes the survivor flags (d_alive starts at zero): 1 for every row the
 // layer listed -- or -1 for every row when a device wait of the call gave up.
 __global__ void noalloc_flags_kernel(const NoAllocScratch* s, int32_t* alive, int32_t rows) {
+  sdnn::pdl_prologue();
   const int stride = gridDim.x * blockDim.x;
   if (s->err[0] != 0) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += stride) alive[i] = -1;
@@ -146,7 +148,7 @@ extern "C" int sdnn_layer_noalloc(sdnn_engine* e, int32_t layer, const float* d_
   rc = scratch_address(e, &scratch);
   if (rc) return rc;
   cudaStream_t s = stream ? (cudaStream_t)stream : sdnn::engine_stream(e);
-  noalloc_prepare_kernel<<<64, 256, 0, s>>>(scratch, (int32_t)rows);
+  noalloc_prepare_kernel<<<64, 256, 0, s>>>(scratch, d_alive, (int32_t)rows);
   a.y_in = d_y_in;
   a.y_out = d_y_out;
   a.list_in = scratch->list_in;
@@ -158,11 +160,9 @@ extern "C" int sdnn_layer_noalloc(sdnn_engine* e, int32_t layer, const float* d_
   a.err = &scratch->err[0];
   cudaError_t ce = res.fn ? sdnn::launch_layer_resident(res, a, num_sms, s)
                           : sdnn::launch_layer(key, a, grid, threads, smem, s);
-  if (ce == cudaSuccess) ce = cudaMemsetAsync(d_alive, 0, (size_t)rows * sizeof(int32_t), s);
-  if (ce == cudaSuccess) {
-    noalloc_flags_kernel<<<64, 256, 0, s>>>(scratch, d_alive, (int32_t)rows);
-    ce = cudaGetLastError();
-  }
+  if (ce == cudaSuccess)
+    ce = sdnn::launch_pdl(noalloc_flags_kernel, 64, 256, 0, s, (const NoAllocScratch*)scratch,
+                          d_alive, (int32_t)rows);
   if (ce != cudaSuccess) {
     sdnn::engine_set_error(e, std::string("sdnn_layer_noalloc: ") + cudaGetErrorString(ce));
     return SDNN_ERR_CUDA;
@@ -191,13 +191,11 @@ extern "C" int sdnn_selftest_noalloc_timeout(sdnn_engine* e, int32_t* d_alive, i
   rc = scratch_address(e, &scratch);
   if (rc) return rc;
   cudaStream_t s = stream ? (cudaStream_t)stream : sdnn::engine_stream(e);
-  noalloc_prepare_kernel<<<64, 256, 0, s>>>(scratch, (int32_t)rows);
+  noalloc_prepare_kernel<<<64, 256, 0, s>>>(scratch, d_alive, (int32_t)rows);
   cudaError_t ce = sdnn::launch_wait_selftest(&scratch->err[0], (uint64_t)limit_us * 1000ull, s);
-  if (ce == cudaSuccess) ce = cudaMemsetAsync(d_alive, 0, (size_t)rows * sizeof(int32_t), s);
-  if (ce == cudaSuccess) {
-    noalloc_flags_kernel<<<64, 256, 0, s>>>(scratch, d_alive, (int32_t)rows);
-    ce = cudaGetLastError();
-  }
+  if (ce == cudaSuccess)
+    ce = sdnn::launch_pdl(noalloc_flags_kernel, 64, 256, 0, s, (const NoAllocScratch*)scratch,
+                          d_alive, (int32_t)rows);
   if (ce != cudaSuccess) {
     sdnn::engine_set_error(e, std::string("sdnn_selftest_noalloc_timeout: ") + cudaGetErrorString(ce));
     return SDNN_ERR_CUDA;
