@@ -165,6 +165,7 @@ struct ChainArgs {
   bool stream;               // weights may be streamed into shared memory
   uint32_t wcap8, wcap16;    // largest per-CTA weight slice, clusters of 8 / 16 CTAs
   uint32_t wcap;             // (set by launch_chain) bytes of one streamed weight buffer
+  int32_t nbuf;              // (set by launch_chain) streamed weight buffers
 };
 // Bytes of the largest per-CTA weight slice of a layer when `cluster` CTAs
 // split its groups (grp_blk: G + 1 block offsets; general = per-edge values).
@@ -173,7 +174,7 @@ int chain_capacity(int N);  // largest centroid count the chain kernel takes (0 
 // The chain launch for a centroid count: variant 0 none, 1 weights read from
 // L2, 2 weights streamed into shared memory (cluster size, weight buffers).
 struct ChainPlan {
-  int variant, kc, cluster, nwbuf, threads;
+  int variant, kc, cluster, nbuf, threads;
   uint32_t wcap;
   size_t smem;
 };

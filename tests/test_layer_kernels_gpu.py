@@ -83,3 +83,34 @@ def test_streamed_split_covers_every_row_and_group(N):
         bound = (n + 2) * 2.0 ** -24 * (S + abs(b))  # inputs and weights >= 0
         assert np.all(np.abs(act - np.clip(S + b, 0, 32)) <= bound)
         assert np.array_equal(np.flatnonzero(flags), ids) and len(ids) == rows
+
+
+@pytest.mark.parametrize("N,nnz,values,L,K", [
+    (1024, 32, False, 70, 1), (1024, 3, False, 35, 3),
+    (1024, 80, False, 40, 8),   # lists longer than one batch of 16 blocks
+    (1024, 50, True, 36, 2),    # ... than one of 8 with their values
+    (4096, 32, False, 67, 1), (4096, 32, False, 10, 4), (4096, 20, True, 36, 1),
+    (16384, 20, False, 40, 1),  # one weight buffer
+])
+def test_chain_carries_the_centroids_like_the_layers(N, nnz, values, L, K):
+    """K prototypes, four copies each: after merging, the centroids are all
+    there is, and one chain launch over more layers than it looks up at a time
+    must give the bits of the per-layer launches."""
+    r, c, v = _net(N, nnz, values, 7)
+    v = np.abs(v) * np.float32(0.9 / (nnz * np.abs(v).mean()))  # values settle around 1
+    rng = np.random.default_rng(N + nnz)
+    protos = np.where(rng.random((K, N)) < 0.5, rng.random((K, N)) * 3, 0).astype(np.float32)
+    Y = np.tile(protos, (4, 1))
+    out = []
+    for chain in (True, False):
+        with sg.Engine(N, L, mode="SNICIT", threshold=3, batch=4 * K, bias=0.1, num_centroids=50,
+                       merge_start=1, chain=chain) as e:
+            for l in range(L):
+                e.set_layer_coo(l, r, c, v)
+            flags, ids = e.infer(Y)
+            out.append((flags, e.activations(4 * K), e.stats()))
+    st = out[0][2]
+    if st["residue_rows"] == 0 and st["centroids"] > 0:
+        assert st["post_kernel"] in (2, 3, 4), st
+    assert np.array_equal(out[0][0], out[1][0])
+    assert np.array_equal(out[0][1].view(np.uint32), out[1][1].view(np.uint32))
