@@ -37,6 +37,7 @@ namespace {
 
 struct DevLayer {
   uint8_t* mem = nullptr;  // holds everything below
+  uint32_t list_bytes = 0;  // ... its first part: the lists and their blocks
   uint2* idx = nullptr;
   float4* val = nullptr;
   int32_t* grp = nullptr;
@@ -639,7 +640,7 @@ int upload_layer(sdnn_engine* e, int l, const PackedView& p, std::string& err) {
   d.slots = p.slots;
   d.max_depth = p.max_depth;
   if (e->nq == 1) {
-    d.res = resident_plan(e->N, p.constw, p.max_depth);
+    d.res = resident_plan(e->N, p.constw, p.max_depth, e->num_sms);
     d.chain_slice8 = chain_slice_bytes(p.grp_blk, e->G, !p.constw, 8);
     d.chain_slice16 = chain_slice_bytes(p.grp_blk, e->G, !p.constw, 16);
   }
@@ -675,6 +676,7 @@ int upload_layer(sdnn_engine* e, int l, const PackedView& p, std::string& err) {
   }
   const size_t o_lists = put(lists.data(), lists.size() * sizeof(int2));
   if (!p.constw) o_val = put(p.val, nslot * 4);
+  d.list_bytes = (uint32_t)std::min<size_t>(image.size() & ~(size_t)15, 1u << 30);
   if (p.bias) {
     // per-neuron bias follows its neuron to its position
     std::vector<float> b(e->N);
@@ -936,7 +938,7 @@ bool resident_on(const sdnn_engine* e, int l) {
 }
 
 int layer_launch(sdnn_engine* e, int l, int epi, const float* in, float* out, const int32_t* lin,
-                 const int32_t* cin, int32_t* lout, int32_t* cout) {
+                 const int32_t* cin, const int32_t* hint, int32_t* lout, int32_t* cout) {
   const DevLayer& d = e->dl[l];
   LayerArgs a{};
   a.w.idx = d.idx;
@@ -950,6 +952,7 @@ int layer_launch(sdnn_engine* e, int l, int epi, const float* in, float* out, co
   a.y_out = out;
   a.list_in = lin;
   a.count_in = cin;
+  a.hint = hint;
   a.list_out = lout;
   a.count_out = cout;
   a.stamp = e->d_stamp;
@@ -967,7 +970,11 @@ int layer_launch(sdnn_engine* e, int l, int epi, const float* in, float* out, co
   a.min_split = e->min_split;
   a.clampv = e->cfg.clamp;
   if (resident_on(e, l)) {
-    CK(launch_layer_resident(d.res, a, e->num_sms, e->stream));
+    if (l + 1 < e->L) {
+      a.next = e->dl[l + 1].idx;
+      a.next_bytes = e->dl[l + 1].list_bytes;
+    }
+    CK(launch_layer_resident(d.res, a, e->stream));
   } else {
     CK(launch_layer(d.constw ? e->key : e->key_general, a, d.constw ? e->grid : e->grid_general,
                     d.constw ? e->threads : e->threads_general, e->smem, e->stream));
@@ -1070,7 +1077,10 @@ int enqueue_layer(sdnn_engine* e, int l, const float* in, const int32_t* lin, co
                   int32_t* lout, int32_t* cout, bool piece = false) {
   const cudaStream_t s = e->stream;
   const bool bits = l == 0 && e->dl[0].sums && e->bits_on;
-  if (!bits) return layer_launch(e, l, EPI_PLAIN, in, e->d_y[l & 1], lin, cin, lout, cout);
+  // rows only get fewer: the count of the layer before is known earlier
+  if (!bits)
+    return layer_launch(e, l, EPI_PLAIN, in, e->d_y[l & 1], lin, cin, l > 0 ? cin - 1 : e->d_rows,
+                        lout, cout);
   if (piece) CK(cudaMemsetAsync(e->d_fbcount, 0, 16, s));  // (the lane's last piece used it)
   Layer0Args b{};
   b.idx = e->dl[0].idx;
@@ -1099,7 +1109,8 @@ int enqueue_layer(sdnn_engine* e, int l, const float* in, const int32_t* lin, co
   b.err = e->d_err;
   CK(launch_layer0_bits(b, e->num_sms, s));
   e->launches += 2;
-  return layer_launch(e, 0, EPI_PLAIN, in, e->d_y[0], e->d_fallback, e->d_fbcount, lout, cout);
+  return layer_launch(e, 0, EPI_PLAIN, in, e->d_y[0], e->d_fallback, e->d_fbcount, e->d_fbcount,
+                      lout, cout);
 }
 
 // Enqueues plain layers e->pipe_start .. T - 1 over the global row lists (the
@@ -1228,17 +1239,19 @@ int enqueue(sdnn_engine* e, int phase, int64_t rows, const float* d_in, int32_t*
       const int p = l - T;
       const float* in = e->d_y[(l - 1 + 2) & 1];
       float* out = e->d_y[l & 1];
-      if ((rc = layer_launch(e, l, EPI_CENTROID, in, out, e->d_clist, e->d_ccount, nullptr,
-                             nullptr)))
+      if ((rc = layer_launch(e, l, EPI_CENTROID, in, out, e->d_clist, e->d_ccount,
+                             e->d_ccount, nullptr, nullptr)))
         return rc;
       if (!e->sparse_res) {
         if ((rc = layer_launch(e, l, EPI_RESIDUE, in, out, e->d_rlist[p & 1], e->d_rcounts + p,
+                               e->d_rcounts + p,
                                e->d_rlist[(p + 1) & 1], e->d_rcounts + p + 1)))
           return rc;
         continue;
       }
       // dense residue rows: the layer kernel, then their split by nonzeros
       if ((rc = layer_launch(e, l, EPI_RESIDUE, in, out, e->d_rlist[p & 1], e->d_rcounts + p,
+                               e->d_rcounts + p,
                              e->d_rtmp, e->d_tcounts + p + 1)))
         return rc;
       const SparseRows next = sparse_rows(e, (p + 1) & 1);
@@ -1641,7 +1654,7 @@ int prepare(sdnn_engine* e, int64_t rows) {
     CK(layer_prepare(e->key_general));
     if (e->nq == 1)
       for (bool constw : {true, false}) {
-        const ResidentPlan p = resident_plan(e->N, constw, 0);
+        const ResidentPlan p = resident_plan(e->N, constw, 0, e->num_sms);
         if (p.fn) CK(resident_prepare(p));
       }
     if (e->sparse_built) CK(sparse_residue_prepare(e->N));
@@ -2434,7 +2447,7 @@ sdnn_config engine_config(const sdnn_engine* e) { return e->cfg; }
 // launch shape, without allocating anything: the weights must already be on
 // the device (sdnn_finalize_weights or an earlier inference).
 int engine_layer_setup(sdnn_engine* e, int layer, LayerArgs* a, LayerKernelKey* key, int* grid,
-                       int* threads, size_t* smem, ResidentPlan* res, int* num_sms) {
+                       int* threads, size_t* smem, ResidentPlan* res) {
   if (layer < 0 || layer >= e->L) return fail(e, SDNN_ERR_INVALID, "bad layer");
   if (!e->stream || e->weights_dirty || (int)e->dl.size() != e->L)
     return fail(e, SDNN_ERR_STATE, "weights are not on the device: call sdnn_finalize_weights first");
@@ -2446,7 +2459,6 @@ int engine_layer_setup(sdnn_engine* e, int layer, LayerArgs* a, LayerKernelKey* 
   const DevLayer& d = e->dl[layer];
   const LayerKernelKey k = d.constw ? e->key : e->key_general;
   *res = resident_on(e, layer) ? d.res : ResidentPlan{};
-  *num_sms = e->num_sms;
   if (res->fn) CK(resident_prepare(*res));
   else CK(layer_prepare(k));
   *a = LayerArgs{};

@@ -25,7 +25,7 @@
 
 namespace sdnn {
 int engine_layer_setup(sdnn_engine* e, int layer, LayerArgs* a, LayerKernelKey* key, int* grid,
-                       int* threads, size_t* smem, ResidentPlan* res, int* num_sms);
+                       int* threads, size_t* smem, ResidentPlan* res);
 cudaStream_t engine_stream(const sdnn_engine* e);
 void engine_set_error(sdnn_engine* e, const std::string& msg);
 }  // namespace sdnn
@@ -131,10 +131,9 @@ extern "C" int sdnn_layer_noalloc(sdnn_engine* e, int32_t layer, const float* d_
   sdnn::LayerArgs a;
   sdnn::LayerKernelKey key;
   sdnn::ResidentPlan res;
-  int grid = 0, threads = 0, num_sms = 0;
+  int grid = 0, threads = 0;
   size_t smem = 0;
-  int rc = sdnn::engine_layer_setup(e, layer, &a, &key, &grid, &threads, &smem, &res,
-                                    &num_sms);
+  int rc = sdnn::engine_layer_setup(e, layer, &a, &key, &grid, &threads, &smem, &res);
   if (rc) return rc;
   // CTAs that share a tile write one row's outputs while others may still be
   // loading that row: input and output must not overlap
@@ -153,12 +152,13 @@ extern "C" int sdnn_layer_noalloc(sdnn_engine* e, int32_t layer, const float* d_
   a.y_out = d_y_out;
   a.list_in = scratch->list_in;
   a.count_in = &scratch->counts[0];
+  a.rows = (int32_t)rows;
   a.list_out = scratch->list_out;
   a.count_out = &scratch->counts[1];
   a.stamp = scratch->stamp;
   a.stamp_id = 1;
   a.err = &scratch->err[0];
-  cudaError_t ce = res.fn ? sdnn::launch_layer_resident(res, a, num_sms, s)
+  cudaError_t ce = res.fn ? sdnn::launch_layer_resident(res, a, s)
                           : sdnn::launch_layer(key, a, grid, threads, smem, s);
   if (ce == cudaSuccess)
     ce = sdnn::launch_pdl(noalloc_flags_kernel, 64, 256, 0, s, (const NoAllocScratch*)scratch,
@@ -182,10 +182,9 @@ extern "C" int sdnn_selftest_noalloc_timeout(sdnn_engine* e, int32_t* d_alive, i
   sdnn::LayerArgs a;
   sdnn::LayerKernelKey key;
   sdnn::ResidentPlan res;
-  int grid = 0, threads = 0, num_sms = 0;
+  int grid = 0, threads = 0;
   size_t smem = 0;
-  int rc = sdnn::engine_layer_setup(e, 0, &a, &key, &grid, &threads, &smem, &res,
-                                    &num_sms);  // engine's device
+  int rc = sdnn::engine_layer_setup(e, 0, &a, &key, &grid, &threads, &smem, &res);  // engine's device
   if (rc) return rc;
   NoAllocScratch* scratch = nullptr;
   rc = scratch_address(e, &scratch);

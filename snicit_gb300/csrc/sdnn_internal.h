@@ -39,6 +39,10 @@ struct LayerArgs {
   float* y_out;             // [rows][N]
   const int32_t* list_in;   // row ids to process
   const int32_t* count_in;  // number of ids (device scalar)
+  const int32_t* hint;      // about the number of ids, known earlier (null: `rows`)
+  int32_t rows;             // the number of ids where the host knows it
+  const void* next;         // lists and blocks that the next launch reads, or null
+  uint32_t next_bytes;
   int32_t* list_out;        // surviving ids (PLAIN) / non-empty residues (RESIDUE)
   int32_t* count_out;       // device scalar, must start at 0
   int32_t* stamp;           // [rows] mark of the launch that last listed the row
@@ -109,15 +113,21 @@ __device__ __forceinline__ void pdl_prologue() {
 // Layer kernel with the slot lists in tensor memory (layer_resident.cu): the
 // plan for a layer, fn == nullptr where it does not apply (N outside 1024 ..
 // 4096, or lists too deep to keep).
+struct FewRows {
+  int32_t teams;   // CTAs with a tile each at the least split
+  int32_t few;     // up to this many rows, tiles are shared by more CTAs
+  int32_t cap[3];  // ... in tiles of 1, 2, 4 rows up to these many
+  int32_t most;    // CTAs that share a tile at most
+};
 struct ResidentPlan {
   const void* fn;
   int T, rsw, split, stages;
   size_t smem;
+  FewRows few;
 };
-ResidentPlan resident_plan(int N, bool constw, int max_depth);
+ResidentPlan resident_plan(int N, bool constw, int max_depth, int num_sms);
 cudaError_t resident_prepare(const ResidentPlan& p);
-cudaError_t launch_layer_resident(const ResidentPlan& p, const LayerArgs& a, int num_sms,
-                                  cudaStream_t s);
+cudaError_t launch_layer_resident(const ResidentPlan& p, const LayerArgs& a, cudaStream_t s);
 
 // First layer over binary inputs (layer0_bits.cu).
 struct Layer0Args {

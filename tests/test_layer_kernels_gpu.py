@@ -114,3 +114,27 @@ def test_chain_carries_the_centroids_like_the_layers(N, nnz, values, L, K):
         assert st["post_kernel"] in (2, 3, 4), st
     assert np.array_equal(out[0][0], out[1][0])
     assert np.array_equal(out[0][1].view(np.uint32), out[1][1].view(np.uint32))
+
+
+@pytest.mark.parametrize("N,nnz,values", [(1024, 32, False), (1056, 32, False), (2048, 32, True),
+                                          (4096, 32, False), (4096, 20, True)])
+def test_few_rows_share_their_tiles(N, nnz, values):
+    """Row counts on both sides of each step of the few-rows split (tiles of 1,
+    2, 4 and all rows, then a tile per team): every row must keep the bits that
+    it has among many others, whose lists are kept whole."""
+    r, c, v = _net(N, nnz, values, 8)
+    rng = np.random.default_rng(N)
+    all_rows = 2500 if N <= 2048 else 900
+    Y = np.where(rng.random((all_rows, N)) < 0.4, rng.random((all_rows, N)) * 3, 0).astype(np.float32)
+    Y[3] = 0
+    with sg.Engine(N, 2, mode="SNIG", batch=all_rows, bias=-0.3) as e:
+        for l in range(2):
+            e.set_layer_coo(l, r, c, v)
+        flags, _ = e.infer(Y)
+        act = e.activations(all_rows)
+        for rows in (1, 2, 5, 18, 19, 37, 38, 74, 77, 151, 153, 227, 229, 305, 607, 609):
+            if rows > all_rows:
+                continue
+            f, ids = e.infer(Y[:rows])
+            assert np.array_equal(f, flags[:rows]) and np.array_equal(ids, np.flatnonzero(f))
+            assert np.array_equal(e.activations(rows).view(np.uint32), act[:rows].view(np.uint32)), rows
