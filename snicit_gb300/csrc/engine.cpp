@@ -182,6 +182,7 @@ struct sdnn_engine {
   int32_t* d_mcounts = nullptr;        // [L + 4] ... and their number
   uint32_t mmask = 0;
   bool bits_on = false;            // layer 0 of 0/1 inputs by counting
+  bool bit_rows = false;           // ... from d_inbits (the call's rows came as bits)
 
   cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
 
@@ -216,9 +217,10 @@ struct sdnn_engine {
   int last_pieces = 0;
 
   // graph cache: one captured graph per phase of an inference (slots 5 and 6:
-  // PH_ALL and PH_PRE starting after the layers run piece by piece)
-  GraphSlot graphs[7];
-  FullGraph full[2];       // SNICIT whole-inference graphs (pipe_start 0 / > 0)
+  // PH_ALL and PH_PRE starting after the layers run piece by piece, 7 and 8: from
+  // rows that came as bits)
+  GraphSlot graphs[9];
+  FullGraph full[3];       // SNICIT whole-inference graphs (pipe_start 0 / > 0, bit rows)
   bool full_off = false;   // building one failed: the host picks the post path
   bool in_body = false;    // capturing a conditional body (no event records)
   int last_full = 0;       // 1 + slot of the whole-inference graph that ran last, 0: none
@@ -1070,13 +1072,16 @@ int enqueue_begin(sdnn_engine* e, int32_t* list, int32_t* d_flags, int32_t* pcou
   return SDNN_OK;
 }
 
+// Layer 0 of 0/1 inputs takes the binary counting kernels.
+bool layer0_counts(const sdnn_engine* e, int l) { return l == 0 && e->dl[0].sums && e->bits_on; }
+
 // Enqueues plain layer l over the row list (lin, cin) into (lout, cout);
 // layer 0 of 0/1 inputs takes the binary counting kernels, with the tiles that
 // hold other values sent to the float kernel.
 int enqueue_layer(sdnn_engine* e, int l, const float* in, const int32_t* lin, const int32_t* cin,
                   int32_t* lout, int32_t* cout, bool piece = false) {
   const cudaStream_t s = e->stream;
-  const bool bits = l == 0 && e->dl[0].sums && e->bits_on;
+  const bool bits = layer0_counts(e, l);
   // rows only get fewer: the count of the layer before is known earlier
   if (!bits)
     return layer_launch(e, l, EPI_PLAIN, in, e->d_y[l & 1], lin, cin, l > 0 ? cin - 1 : e->d_rows,
@@ -1091,6 +1096,7 @@ int enqueue_layer(sdnn_engine* e, int l, const float* in, const int32_t* lin, co
   b.sums = e->dl[0].sums;
   b.max_count = e->dl[0].max_in_degree;
   b.y_in = in;
+  b.bit_rows = e->bit_rows ? e->d_inbits : nullptr;
   b.y_out = e->d_y[0];
   b.first_row = (int32_t)(e->bits_tile0 * 32);  // (layer 0 takes the rows in order)
   b.count_in = cin;
@@ -1109,6 +1115,7 @@ int enqueue_layer(sdnn_engine* e, int l, const float* in, const int32_t* lin, co
   b.err = e->d_err;
   CK(launch_layer0_bits(b, e->num_sms, s));
   e->launches += 2;
+  if (b.bit_rows) return SDNN_OK;  // (nothing but 0 and 1)
   return layer_launch(e, 0, EPI_PLAIN, in, e->d_y[0], e->d_fallback, e->d_fbcount, e->d_fbcount,
                       lout, cout);
 }
@@ -1371,10 +1378,11 @@ int run_phase(sdnn_engine* e, int slot, int phase, int64_t rows, const float* d_
     e->launches = before;
     return rc;
   }
-  const bool streamed = e->pipe_start > 0 && (phase == PH_ALL || phase == PH_PRE);
-  GraphSlot& g = e->graphs[streamed ? 5 + slot : slot];
-  const GraphKey key{0, d_in, d_flags, effective_threshold(e), std::max(1, e->cfg.num_centroids), e->cfg.mode,
-                     e->key.T, e->threads,
+  const bool reads_in = phase == PH_ALL || phase == PH_PRE;
+  const bool streamed = e->pipe_start > 0 && reads_in, bit_rows = e->bit_rows && reads_in;
+  GraphSlot& g = e->graphs[streamed ? 5 + slot : bit_rows ? 7 + slot : slot];
+  const GraphKey key{0, reads_in ? d_in : nullptr, d_flags, effective_threshold(e),
+                     std::max(1, e->cfg.num_centroids), e->cfg.mode, e->key.T, e->threads,
                      phase == PH_POST_CHAIN ? e->chain_kc * 4 + e->chain_kind : 0,
                      streamed ? e->pipe_start : 0};
   if (!g.exec || !(g.key == key)) {
@@ -1528,7 +1536,7 @@ int build_full_graph(sdnn_engine* e, FullGraph& fg, int64_t rows, const float* d
 // SDNN_ERR_UNSUPPORTED when the graph cannot be built (the caller then lets
 // the host choose the post-threshold path, for this and every later call).
 int run_full(sdnn_engine* e, int64_t rows, const float* d_in, int32_t* d_flags) {
-  const int slot = e->pipe_start > 0 ? 1 : 0;
+  const int slot = e->pipe_start > 0 ? 1 : e->bit_rows ? 2 : 0;
   FullGraph& fg = e->full[slot];
   const GraphKey key{0, d_in, d_flags, effective_threshold(e), std::max(1, e->cfg.num_centroids), e->cfg.mode,
                      e->key.T, e->threads, 0, e->pipe_start};
@@ -2100,9 +2108,15 @@ int infer_host(sdnn_engine* e, const float* Y0, const uint64_t* bits, int64_t ro
     if (bits) {
       CK(cudaMemcpyAsync(e->d_inbits, bits + off * W, (size_t)(n * W) * 8, cudaMemcpyHostToDevice,
                          e->stream));
-      launch_expand_bits(e->d_inbits, n, e->N, e->d_in, e->stream);
-      CK(cudaGetLastError());
-      rc = run(e, n, e->d_in, e->d_flags);
+      if (effective_threshold(e) > 0 && layer0_counts(e, 0)) {
+        e->bit_rows = true;
+        rc = run(e, n, reinterpret_cast<const float*>(e->d_inbits), e->d_flags);
+        e->bit_rows = false;
+      } else {
+        launch_expand_bits(e->d_inbits, n, e->N, e->d_in, e->stream);
+        CK(cudaGetLastError());
+        rc = run(e, n, e->d_in, e->d_flags);
+      }
     } else if (P > 1) {
       rc = run_streamed(e, Y0 + off * N, n, m, P);
     } else {

@@ -138,6 +138,7 @@ struct Layer0Args {
   const float* sums;         // [128]: w added k times in FP32, k = 0..127
   int32_t max_count;         // largest in-degree of the layer (< 128)
   const float* y_in;
+  const uint64_t* bit_rows;  // the rows as bits, (N + 63) / 64 words each, instead of y_in
   float* y_out;
   int32_t first_row;         // the rows are first_row .. first_row + *count_in - 1
   const int32_t* count_in;

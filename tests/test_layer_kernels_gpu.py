@@ -138,3 +138,22 @@ def test_few_rows_share_their_tiles(N, nnz, values):
             f, ids = e.infer(Y[:rows])
             assert np.array_equal(f, flags[:rows]) and np.array_equal(ids, np.flatnonzero(f))
             assert np.array_equal(e.activations(rows).view(np.uint32), act[:rows].view(np.uint32)), rows
+
+
+@pytest.mark.parametrize("N,rows", [(256, 1), (1024, 31), (1024, 97), (4096, 33), (16384, 40),
+                                    (65536, 35)])
+@pytest.mark.parametrize("mode", ["SNIG", "SNICIT"])
+def test_rows_that_come_as_bits(N, rows, mode):
+    """One-bit rows go straight to the counting kernels: same categories and
+    activations, bit for bit, as the same rows in floats, in either order of
+    calls; ragged last tiles of 32 rows, and fewer rows after more."""
+    Y = sg.generate_inputs(N, 11, 0, rows)
+    with sg.Engine(N, 3, mode=mode, threshold=2, batch=rows, bias=-0.3) as e:
+        e.generate_weights(4)
+        for n in (rows, max(1, rows - 7), rows):
+            f1, i1 = e.infer(Y[:n])
+            a1 = e.activations(n)
+            f2, i2 = e.infer_bits(sg.pack_bits(Y[:n]))
+            a2 = e.activations(n)
+            assert np.array_equal(f1, f2) and np.array_equal(i1, i2)
+            assert np.array_equal(a1.view(np.uint32), a2.view(np.uint32))
