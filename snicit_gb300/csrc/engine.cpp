@@ -2082,6 +2082,38 @@ int run_streamed(sdnn_engine* e, const float* Y0, int64_t n, int m, int P) {
   return SDNN_OK;
 }
 
+// The batches as tables for the gather and scatter kernels; false where a copy
+// takes more than they do: memory that is not this device's, inputs that are
+// not aligned to 16 bytes, or flags that overlap (the last batch then wins).
+bool batch_tables(const sdnn_engine* e, const float* const* in, const int64_t* rows, int32_t n,
+                  int32_t* const* flags, int64_t total, std::vector<BatchTable>& tables) {
+  if (total > INT32_MAX || e->N % 4) return false;
+  auto here = [&](const void* p) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    return at.type == cudaMemoryTypeDevice && at.device == e->dev;
+  };
+  int64_t off = 0;
+  for (int32_t b = 0; b < n; ++b) {
+    if (rows[b] == 0) continue;
+    if ((uintptr_t)in[b] % 16 || (uintptr_t)flags[b] % 4 || !here(in[b]) || !here(flags[b])) return false;
+    if (tables.empty() || tables.back().n == kBatchTable) tables.push_back(BatchTable{});
+    BatchTable& t = tables.back();
+    for (int i = 0; i < t.n; ++i)
+      if (flags[b] < t.flags[i] + (t.first[i + 1] - t.first[i]) && t.flags[i] < flags[b] + rows[b])
+        return false;
+    t.in[t.n] = in[b];
+    t.flags[t.n] = flags[b];
+    t.first[t.n] = (int32_t)off;
+    off += rows[b];
+    t.first[++t.n] = (int32_t)off;
+  }
+  return true;
+}
+
 // Host inference over batches of cfg.batch rows; inputs as FP32 rows, or as
 // one-bit rows (bits != nullptr) expanded on the device.
 int infer_host(sdnn_engine* e, const float* Y0, const uint64_t* bits, int64_t rows, int32_t* flags,
@@ -2230,14 +2262,24 @@ int sdnn_infer_batches_device(sdnn_engine* e, const float* const* d_inputs, cons
   }
   const int64_t N = e->N;
   int64_t off = 0;
-  for (int32_t b = 0; b < num_batches; ++b) {
+  std::vector<BatchTable> tables;
+  const bool tabled = batch_tables(e, d_inputs, rows, num_batches, d_flags, total, tables);
+  if (tabled) {
+    for (const BatchTable& t : tables) launch_gather_batches(t, e->d_in, e->N, e->num_sms, e->stream);
+    CK(cudaGetLastError());
+  }
+  for (int32_t b = 0; b < num_batches && !tabled; ++b) {
     if (rows[b] > 0)
       CK(cudaMemcpyAsync(e->d_in + off * N, d_inputs[b], (size_t)(rows[b] * N) * 4,
                          cudaMemcpyDeviceToDevice, e->stream));
     off += rows[b];
   }
   rc = run(e, total, e->d_in, e->d_flags);
-  if (rc == SDNN_OK) {
+  if (rc == SDNN_OK && tabled) {
+    for (const BatchTable& t : tables) launch_scatter_flags(t, e->d_flags, e->stream);
+    if (cudaError_t ce = cudaGetLastError(); ce != cudaSuccess) rc = cuda_fail(e, ce, "scatter_flags");
+    e->launches += 2 * (int)tables.size();
+  } else if (rc == SDNN_OK) {
     off = 0;
     for (int32_t b = 0; b < num_batches; ++b) {
       if (rows[b] > 0) {

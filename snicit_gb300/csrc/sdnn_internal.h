@@ -254,6 +254,17 @@ struct BeginArgs {
 };
 void launch_begin(const BeginArgs& a, cudaStream_t s);
 void launch_copy_rows(const int32_t* nrows, const float* src, float* dst, int32_t N, cudaStream_t s);
+// Batches of a schedule: their rows gathered into one buffer, and the flags of
+// all rows handed back to each batch's own.
+constexpr int kBatchTable = 64;
+struct BatchTable {
+  int32_t n;
+  const float* in[kBatchTable];  // 16-byte aligned
+  int32_t* flags[kBatchTable];
+  int32_t first[kBatchTable + 1];  // first row of each batch, then the end
+};
+void launch_gather_batches(const BatchTable& t, float* rows, int32_t N, int num_sms, cudaStream_t s);
+void launch_scatter_flags(const BatchTable& t, const int32_t* flags, cudaStream_t s);
 // flags[r] = any entry > 0, state[r] = 1 for the listed rows
 void launch_identify(const float* y, const int32_t* list, const int32_t* count, int32_t N,
                      int32_t* flags, int32_t* state, int num_sms, cudaStream_t s);

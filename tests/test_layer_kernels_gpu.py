@@ -157,3 +157,40 @@ def test_rows_that_come_as_bits(N, rows, mode):
             a2 = e.activations(n)
             assert np.array_equal(f1, f2) and np.array_equal(i1, i2)
             assert np.array_equal(a1.view(np.uint32), a2.view(np.uint32))
+
+
+@pytest.mark.parametrize("N,count,shift", [(256, 1, 0), (1024, 7, 0), (1024, 65, 0), (4096, 5, 0),
+                                           (1024, 4, 1)])
+def test_device_batches_are_gathered_and_handed_back(N, count, shift):
+    """Batches of uneven size, some empty, more than one table of them, and
+    inputs that are not aligned to 16 bytes (copied instead): the flags of each
+    batch are those of its rows in one batch of all."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(count)
+    sizes = [int(s) for s in rng.integers(0, 40, count)]
+    sizes[0] = 33
+    total = sum(sizes)
+    Y = sg.generate_inputs(N, 21, 0, total)
+    Y[1::3] = 0
+    with sg.Engine(N, 4, mode="SNIG", batch=total, bias=-0.3) as e:
+        e.generate_weights(6)
+        want, _ = e.infer(Y)
+        assert 0 < want.sum() < total
+        y, flags, at = [], [], 0
+        for s in sizes:
+            buf = torch.zeros(max(s, 1) * N + 4, device="cuda")
+            part = buf[shift:shift + s * N]
+            part.copy_(torch.from_numpy(Y[at:at + s]).reshape(-1))
+            y.append((buf, part))
+            flags.append(torch.full((max(s, 1),), -7, dtype=torch.int32, device="cuda"))
+            at += s
+        torch.cuda.synchronize()
+        e.infer_batches_device([p.data_ptr() for _, p in y], sizes, [f.data_ptr() for f in flags],
+                               torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        at = 0
+        for s, f in zip(sizes, flags):
+            assert np.array_equal(f.cpu().numpy()[:s], want[at:at + s])
+            if s == 0:
+                assert int(f[0]) == -7
+            at += s
