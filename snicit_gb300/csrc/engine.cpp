@@ -971,11 +971,11 @@ int layer_launch(sdnn_engine* e, int l, int epi, const float* in, float* out, co
   a.max_split = e->G;
   a.min_split = e->min_split;
   a.clampv = e->cfg.clamp;
+  if (l + 1 < e->L) {
+    a.next = e->dl[l + 1].idx;
+    a.next_bytes = e->dl[l + 1].list_bytes;
+  }
   if (resident_on(e, l)) {
-    if (l + 1 < e->L) {
-      a.next = e->dl[l + 1].idx;
-      a.next_bytes = e->dl[l + 1].list_bytes;
-    }
     CK(launch_layer_resident(d.res, a, e->stream));
   } else {
     CK(launch_layer(d.constw ? e->key : e->key_general, a, d.constw ? e->grid : e->grid_general,

@@ -76,6 +76,16 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
       "l"(src), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
 }
+// This CTA's share of the lists that the next launch reads, into L2 (one
+// thread): a layer's weights are read once per inference, far apart.
+__device__ __forceinline__ void fetch_next_lists(const LayerArgs& a) {
+  if (!a.next) return;
+  const uint32_t share = (a.next_bytes / gridDim.x + 16) & ~15u, from = blockIdx.x * share;
+  if (from < a.next_bytes)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"((const char*)a.next + from),
+                 "r"(min(share, a.next_bytes - from))
+                 : "memory");
+}
 __device__ __forceinline__ float clampf(float v, float hi) { return fminf(hi, fmaxf(0.f, v)); }
 
 
@@ -365,9 +375,13 @@ __device__ __forceinline__ void publish_rows(const LayerArgs& a, uint32_t m, boo
 // With fewer units than CTAs the tiles are cut finer, at most one piece per
 // CTA.  Small row counts use smaller tiles (TE < T): what bounds them is the
 // time to fetch rows and lists, which the CTAs then share.
+//
+// A CTA's run is worked out by one warp, in 32 bits (rows in memory times
+// groups stay far below 2^32 units): done by every warp in 64 bits it took
+// longer than the copy of a row.
 struct Cut {
   int count, TE, unit, per_tile;  // rows, rows per tile, groups per unit, units per tile
-  long long units;
+  int tile, first, left;          // the CTA's run: first tile and unit in it, units
 };
 // Largest tile size <= T, then halved from the power of 2 below it, that
 // still gives every CTA a unit.
@@ -380,17 +394,22 @@ __device__ __forceinline__ Cut make_cut(int count, int G, int nwarps) {
   c.TE = T;
   int p2 = 1;
   while (2 * p2 < T) p2 *= 2;
-  const long long grid = gridDim.x;
-  while (c.TE > 1 && (long long)((count + c.TE - 1) / c.TE) * c.per_tile < grid) {
+  const unsigned grid = gridDim.x, rows = (unsigned)count;
+  unsigned tiles = (rows + T - 1) / T;
+  while (c.TE > 1 && tiles * c.per_tile < grid) {
     c.TE = c.TE == T ? p2 : c.TE / 2;
+    tiles = (rows + c.TE - 1) / (unsigned)c.TE;
   }
-  const long long tiles = (count + c.TE - 1) / c.TE;
   if (tiles * c.per_tile < grid && tiles > 0) {
-    const int parts = (int)(grid / tiles);
-    c.unit = (G + parts - 1) / parts;
-    c.per_tile = (G + c.unit - 1) / c.unit;
+    const unsigned parts = grid / tiles;
+    c.unit = (int)(((unsigned)G + parts - 1) / parts);
+    c.per_tile = (int)(((unsigned)G + c.unit - 1) / (unsigned)c.unit);
   }
-  c.units = tiles * c.per_tile;
+  const unsigned units = tiles * c.per_tile, share = units / grid, more = units % grid;
+  const unsigned lo = share * blockIdx.x + min(blockIdx.x, more);
+  c.left = (int)(share + (blockIdx.x < more ? 1 : 0));
+  c.tile = (int)(lo / (unsigned)c.per_tile);
+  c.first = (int)(lo % (unsigned)c.per_tile);
   return c;
 }
 
@@ -431,6 +450,7 @@ __global__ void __launch_bounds__(1024, 1) layer_rows_kernel(const LayerArgs a) 
   __shared__ int32_t s_rows[2][32];
   __shared__ uint32_t s_mask[2];
   __shared__ int32_t s_fail;
+  __shared__ Cut s_cut;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
   const int RS = RSW > 0 ? RSW : a.Q + 32;
@@ -439,6 +459,7 @@ __global__ void __launch_bounds__(1024, 1) layer_rows_kernel(const LayerArgs a) 
   // ended -- so only CTA-local setup comes before griddepcontrol.wait, which
   // returns once the predecessor has completed and its writes are visible.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (tid == (int)blockDim.x - 32) fetch_next_lists(a);
   // One tile buffer, reloaded per tile: the load of one CTA overlaps the
   // compute of the other CTAs on the SM (up to four).
   for (int i = tid; i < T * 32; i += blockDim.x) ys[(i >> 5) * RS + a.Q + (i & 31)] = 0.f;
@@ -450,15 +471,14 @@ __global__ void __launch_bounds__(1024, 1) layer_rows_kernel(const LayerArgs a) 
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const Cut cut = make_cut<T>(*a.count_in, a.G, nwarps);
-  const long long grid = gridDim.x;
-  const long long lo = cut.units >= grid ? cut.units * blockIdx.x / grid : (long long)blockIdx.x;
-  const long long hi = cut.units >= grid ? cut.units * (blockIdx.x + 1) / grid
-                                         : min(cut.units, (long long)blockIdx.x + 1);
-  if (lo >= hi) return;
-
-  int tile = (int)(lo / cut.per_tile), first = (int)(lo % cut.per_tile);
-  int left = (int)min(hi - lo, (long long)0x7fffffff);
+  if (warp == 0) {
+    const Cut c = make_cut<T>(__ldcg(a.count_in), a.G, nwarps);
+    if (lane == 0) s_cut = c;
+  }
+  __syncthreads();
+  const Cut cut = s_cut;
+  int tile = cut.tile, first = cut.first, left = cut.left;
+  if (left == 0) return;
   // the row ids of the tile after the current one are fetched while it runs
   int next_row = -1;
   if (warp == 0 && lane < cut.TE && tile * cut.TE + lane < cut.count)
@@ -520,7 +540,7 @@ __global__ void __launch_bounds__(1024, 1) layer_rows_kernel(const LayerArgs a) 
 // the groups), parts sized to the registers that hold the accumulators.
 struct Split {
   int count, n_tiles, spl;
-  long items;
+  int items;
 };
 template <int T>
 __device__ __forceinline__ Split make_split(const LayerArgs& a) {
@@ -531,7 +551,7 @@ __device__ __forceinline__ Split make_split(const LayerArgs& a) {
   spl = max(spl, a.min_split);
   spl = min(spl, a.max_split);
   sp.spl = max(spl, 1);
-  sp.items = (long)sp.n_tiles * sp.spl;
+  sp.items = sp.n_tiles * sp.spl;
   return sp;
 }
 
@@ -551,6 +571,7 @@ __global__ void __launch_bounds__(KG <= 8 ? 1024 : 512, 1) layer_chunk_kernel(co
   const int RS = RSW > 0 ? RSW : a.Q + 32;
   // (programmatic stream serialization, see layer_rows_kernel)
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (tid == (int)blockDim.x - 32) fetch_next_lists(a);
   for (int i = tid; i < T * 32; i += blockDim.x) ys[(i >> 5) * RS + a.Q + (i & 31)] = 0.f;
   if (tid == 0) {
     mbar_init(&bar[0], 1);
@@ -561,7 +582,7 @@ __global__ void __launch_bounds__(KG <= 8 ? 1024 : 512, 1) layer_chunk_kernel(co
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const Split sp = make_split<T>(a);
-  if (sp.count <= 0 || (long)blockIdx.x >= sp.items) return;
+  if (sp.count <= 0 || (int)blockIdx.x >= sp.items) return;
   __syncthreads();
 
   // Per item: row ids of the item after it are fetched while it runs, and the
@@ -570,7 +591,7 @@ __global__ void __launch_bounds__(KG <= 8 ? 1024 : 512, 1) layer_chunk_kernel(co
   // warp; s_rows is double-buffered, and the pending state lives in shared
   // memory so that it costs the compute warps no registers.
   const bool last_warp = warp == nwarps - 1;
-  auto item_row = [&](long it, int t) -> int {
+  auto item_row = [&](int it, int t) -> int {
     const int r0 = (int)(it / sp.spl) * T;
     return t < min(T, sp.count - r0) ? a.list_in[r0 + t] : -1;
   };
@@ -578,7 +599,7 @@ __global__ void __launch_bounds__(KG <= 8 ? 1024 : 512, 1) layer_chunk_kernel(co
   if (last_warp && lane == 31) s_ppending = 0;
   uint32_t phase = 0;
   int b = 0;
-  for (long item = blockIdx.x; item < sp.items; item += gridDim.x, b ^= 1) {
+  for (int item = blockIdx.x; item < sp.items; item += gridDim.x, b ^= 1) {
     const int tile = (int)(item / sp.spl), part = (int)(item % sp.spl);
     const int row0 = tile * T;
     const int nrows = min(T, sp.count - row0);

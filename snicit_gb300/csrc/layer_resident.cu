@@ -272,14 +272,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
-  // (this CTA's share of the next layer's lists, into L2)
-  if (tid == kWarps * 32 - 32 && a.next) {
-    const uint32_t share = (a.next_bytes / gridDim.x + 16) & ~15u, from = blockIdx.x * share;
-    if (from < a.next_bytes)
-      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"((const char*)a.next + from),
-                   "r"(min(share, a.next_bytes - from))
-                   : "memory");
-  }
+  if (tid == kWarps * 32 - 32) fetch_next_lists(a);
   for (int i = warp; i < T * stages; i += kWarps) ring[(size_t)i * RS + a.Q + lane] = 0.f;
   if (tid < kMaxStages) {
     mbar_init(&full[tid], 1);
