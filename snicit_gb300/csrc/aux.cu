@@ -24,6 +24,13 @@ static int grid_for(long work, int per_block, int cap = 4096) {
 // Rows of the current inference come from a device scalar (set just before a
 // captured graph is launched), so one graph serves every row count.
 __global__ void set_scalar_kernel(int32_t* p, int32_t v) { *p = v; }
+__global__ void set_rows_kernel(int32_t* p, int32_t rows, int32_t share) {
+  p[0] = rows;
+  p[1] = share;
+}
+void launch_set_rows(int32_t* p, int32_t rows, int32_t share, cudaStream_t s) {
+  set_rows_kernel<<<1, 1, 0, s>>>(p, rows, share);
+}
 void launch_set_scalar(int32_t* p, int32_t v, cudaStream_t s) { set_scalar_kernel<<<1, 1, 0, s>>>(p, v); }
 
 __global__ void post_choice_kernel(const PostChoiceArgs a, cudaGraphConditionalHandle h) {

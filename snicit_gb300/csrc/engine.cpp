@@ -182,6 +182,8 @@ struct sdnn_engine {
   int32_t* d_mcounts = nullptr;        // [L + 4] ... and their number
   uint32_t mmask = 0;
   bool bits_on = false;            // layer 0 of 0/1 inputs by counting
+  bool slot = false;               // one of several of a server
+  int share = 1;                   // engines that work side by side now (servers)
   bool bit_rows = false;           // ... from d_inbits (the call's rows came as bits)
 
   cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -955,6 +957,7 @@ int layer_launch(sdnn_engine* e, int l, int epi, const float* in, float* out, co
   a.list_in = lin;
   a.count_in = cin;
   a.hint = hint;
+  a.share = e->slot ? e->d_rows + 1 : nullptr;
   a.list_out = lout;
   a.count_out = cout;
   a.stamp = e->d_stamp;
@@ -1570,7 +1573,7 @@ int run(sdnn_engine* e, int64_t rows, const float* d_in, int32_t* d_flags) {
   e->report_valid = false;
   if (e->pipe_start == 0) e->last_pieces = 0;
   // the graphs read the row count from d_rows (one graph for every count)
-  launch_set_scalar(e->d_rows, (int32_t)rows, e->stream);
+  launch_set_rows(e->d_rows, (int32_t)rows, e->share, e->stream);
   e->run_launches++;
   int rc;
   e->last_full = 0;
@@ -2042,7 +2045,7 @@ int run_streamed(sdnn_engine* e, const float* Y0, int64_t n, int m, int P) {
   e->launches = 0;
   int rc;
   if ((rc = record(e, 0, false))) return rc;
-  launch_set_scalar(e->d_rows, (int32_t)n, s);
+  launch_set_rows(e->d_rows, (int32_t)n, e->share, s);
   // identity rows into the pieces' layer-0 lists (the layers append to the rest)
   e->launches++;
   if ((rc = enqueue_begin(e, e->d_plist[0], e->d_flags, e->d_pcounts, P * (e->L + 2)))) return rc;
@@ -2570,7 +2573,15 @@ int engine_share_weights(sdnn_engine* dst, sdnn_engine* src) {
 int engine_prepare(sdnn_engine* e, int64_t rows) { return prepare(e, rows); }
 float* engine_input(sdnn_engine* e) { return e->d_in; }
 int32_t* engine_flags(sdnn_engine* e) { return e->d_flags; }
-int engine_run(sdnn_engine* e, int64_t rows) { return run(e, rows, e->d_in, e->d_flags); }
+// One of several slots: `at_work` of them run now.  Passes of few tiles per CTA
+// share the SMs, as one alone would wait for round trips most of the time; from
+// 8 rounds of tiles on a pass takes them all.
+int engine_run(sdnn_engine* e, int64_t rows, int slots, int at_work) {
+  e->slot = slots > 1;
+  const int64_t all = std::max<int64_t>(1, 8ll * 8 * e->num_sms / std::max<int64_t>(1, rows));
+  e->share = (int)std::clamp<int64_t>(all, 1, std::max(1, at_work));
+  return run(e, rows, e->d_in, e->d_flags);
+}
 int engine_check(sdnn_engine* e) { return check_device_error(e); }
 // Positions of the neurons after the last layer (empty = identity).
 std::vector<int32_t> engine_final_positions(const sdnn_engine* e) {

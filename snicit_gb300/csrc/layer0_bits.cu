@@ -3,7 +3,7 @@
 // When every input of a row is 0 or 1 and the layer has one common weight
 // value w, the pre-activation of output c is S(k) + b, where k is the number
 // of active in-edges of c and S(k) is w added k times in FP32 -- exactly what
-// the float gather (layer_kernel, which adds w * 1 or w * 0 slot by slot)
+// the float gather (the layer kernels, which add w * 1 or w * 0 slot by slot)
 // computes.  This kernel therefore counts instead of multiplying:
 //
 //  * bits_transpose_kernel turns tiles of 32 rows into one 32-bit word per input
@@ -14,7 +14,7 @@
 //    take (tile, part of the groups) items: the tile's words come into shared
 //    memory by TMA (N + 32 words, the last 32 zero for the padding slots), and
 //    lane i of a warp owns output 32g + i and walks the same bank-scheduled
-//    slots as layer_kernel, loading one word per slot (one wavefront per slot
+//    slots as the layer kernels, loading one word per slot (one wavefront per slot
 //    for all 32 rows) and adding it into bit-sliced counters with a Harley-Seal
 //    carry-save tree (15 full adders per 16 slots);
 //  * the epilogue extracts each row's count, looks up S(k) (a 128-entry table

@@ -11,7 +11,7 @@
 //  * every CTA of the cluster keeps all K rows in shared memory (two buffers,
 //    this layer's input and the next layer's);
 //  * CTA r computes the outputs of its share of the 32-neuron groups for all K
-//    rows, with the same bank-scheduled slots and FP32 order as layer_kernel
+//    rows, with the same bank-scheduled slots and FP32 order as the layer kernels
 //    (so the rows are bitwise equal to the per-layer path), applies bias and
 //    clamp, and stores each output into the next-layer buffer of every CTA of
 //    the cluster (distributed shared memory);

@@ -11,7 +11,7 @@
 //    so the gathers may be cached in L1 (no stale copy can exist);
 //  * warp w of the grid takes output groups w, w + W, ...; lane i owns output
 //    32g + i and walks the same bank-scheduled slots in the same FP32 order
-//    as layer_kernel (chunk by chunk);
+//    as the layer kernels (chunk by chunk);
 //  * a grid barrier (one counter, bounded wait) separates layers; the last
 //    layer writes the rows to the final activation buffer.
 // Bitwise equal to the per-layer launches.

@@ -41,6 +41,7 @@ struct LayerArgs {
   const int32_t* count_in;  // number of ids (device scalar)
   const int32_t* hint;      // about the number of ids, known earlier (null: `rows`)
   int32_t rows;             // the number of ids where the host knows it
+  const int32_t* share;     // resident kernel: engines that share the SMs, or null: this alone
   const void* next;         // lists and blocks that the next launch reads, or null
   uint32_t next_bytes;
   int32_t* list_out;        // surviving ids (PLAIN) / non-empty residues (RESIDUE)
@@ -213,6 +214,7 @@ cudaError_t launch_grid_chain(const GridChainArgs& a, int kc_needed, int num_sms
 
 // ---- auxiliary kernels (aux.cu) ----
 void launch_set_scalar(int32_t* p, int32_t v, cudaStream_t s);
+void launch_set_rows(int32_t* p, int32_t rows, int32_t share, cudaStream_t s);  // p[0], p[1]
 
 // Post-threshold path chosen on the device, inside the inference's graph: a
 // one-thread kernel reads what the clustering left and sets the value of the
