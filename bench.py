@@ -293,7 +293,7 @@ def layer_kernel_roofline(torch, sg, eng, d_in, B, N, stream, peak, peak_kind, s
     smem_gbs = 128.0 * sms * (sm_mhz or 0) * 1e6 / 1e9 if sm_mhz else None
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
-            "kernel": f"sdnn::layer_kernel (layer 1 of the workload, {rows} rows)",
+            "kernel": f"sdnn layer kernel (layer 1 of the workload, {rows} rows)",
             "per": "one launch", "algorithmic_bytes_per_launch": algo, "avg_launch_ms": ms,
             "frac_of_8tbs": achieved / 8000.0,
             "smem_gather_bytes_per_launch": 4.0 * 32 * N * rows,

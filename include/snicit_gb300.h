@@ -225,7 +225,7 @@ int sdnn_infer_host(sdnn_engine* e, const float* Y0, int64_t rows,
 /* The same with one-bit input rows (entry j of a row in bit j % 64 of word
  * j / 64, ceil(N / 64) words per row -- the layout of the bit-encoded input
  * files): 32x fewer bytes over the host link for 0/1 inputs such as the SDGC
- * images; the rows are expanded on the device.  N must be a multiple of 4. */
+ * images; the rows are packed or expanded on the device.  N must be a multiple of 4. */
 int sdnn_infer_host_bits(sdnn_engine* e, const uint64_t* bits, int64_t rows, int32_t* flags,
                          int32_t* ids, int64_t* count);
 
