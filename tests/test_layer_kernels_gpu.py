@@ -194,3 +194,26 @@ def test_device_batches_are_gathered_and_handed_back(N, count, shift):
             if s == 0:
                 assert int(f[0]) == -7
             at += s
+
+
+@pytest.mark.parametrize("N,values", [(1024, True), (2048, False), (4096, False), (4096, True)])
+def test_passes_that_share_the_sms(N, values):
+    """Passes of several slots at once take a share of the SMs each (few rows,
+    and a few rounds of tiles): logits and flags of a request are those it gets
+    alone, bit for bit."""
+    r, c, v = _net(N, 24, values, 9)
+    rng = np.random.default_rng(N)
+    sizes = [1, 700, 33, 300, 5, 640, 90, 2, 512, 260]
+    reqs = [np.where(rng.random((s, N)) < 0.4, rng.random((s, N)) * 3, 0).astype(np.float32)
+            for s in sizes]
+    hw, hb = rng.standard_normal((N, 4)).astype(np.float32), np.zeros(4, np.float32)
+    with sg.Engine(N, 6, mode="SNIG", batch=1024, bias=-0.1) as e:
+        for l in range(6):
+            e.set_layer_coo(l, r, c, v)
+        with sg.Server(e, hw, hb, slots=4, max_rows=1024, max_requests_per_pass=1) as sv:
+            alone = [sv.wait(sv.submit(x)) for x in reqs]
+            for _ in range(3):
+                mix = [sv.wait(i) for i in [sv.submit(x) for x in reqs]]
+                for a, m in zip(alone, mix):
+                    assert np.array_equal(a.flags, m.flags)
+                    assert np.array_equal(a.logits.view(np.uint32), m.logits.view(np.uint32))
