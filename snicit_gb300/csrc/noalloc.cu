@@ -51,12 +51,12 @@ std::mutex g_addr_mutex;
 NoAllocScratch* g_addr[kMaxDevices] = {};
 
 // Resets the parts of the scratch that must start at zero for this call, and
-// the caller's flags, and lists every row.
+// the caller's flags (unless null), and lists every row.
 __global__ void noalloc_prepare_kernel(NoAllocScratch* s, int32_t* alive, int32_t rows) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x) {
     s->list_in[i] = i;
     s->stamp[i] = 0;
-    alive[i] = 0;
+    if (alive) alive[i] = 0;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     s->counts[0] = rows;
@@ -143,11 +143,15 @@ extern "C" int sdnn_layer_noalloc(sdnn_engine* e, int32_t layer, const float* d_
     sdnn::engine_set_error(e, "sdnn_layer_noalloc: d_y_in and d_y_out overlap");
     return SDNN_ERR_INVALID;
   }
+  // d_alive may lie in either of them (a caller short of memory has its flags
+  // where the inputs were): it is then cleared only after the layer, by a memset
+  const uintptr_t al0 = (uintptr_t)d_alive, al1 = al0 + (uintptr_t)rows * sizeof(int32_t);
+  const bool late = (al0 < in0 + bytes && in0 < al1) || (al0 < out0 + bytes && out0 < al1);
   NoAllocScratch* scratch = nullptr;
   rc = scratch_address(e, &scratch);
   if (rc) return rc;
   cudaStream_t s = stream ? (cudaStream_t)stream : sdnn::engine_stream(e);
-  noalloc_prepare_kernel<<<64, 256, 0, s>>>(scratch, d_alive, (int32_t)rows);
+  noalloc_prepare_kernel<<<64, 256, 0, s>>>(scratch, late ? nullptr : d_alive, (int32_t)rows);
   a.y_in = d_y_in;
   a.y_out = d_y_out;
   a.list_in = scratch->list_in;
@@ -160,7 +164,13 @@ extern "C" int sdnn_layer_noalloc(sdnn_engine* e, int32_t layer, const float* d_
   a.err = &scratch->err[0];
   cudaError_t ce = res.fn ? sdnn::launch_layer_resident(res, a, s)
                           : sdnn::launch_layer(key, a, grid, threads, smem, s);
-  if (ce == cudaSuccess)
+  if (ce == cudaSuccess && late) {
+    ce = cudaMemsetAsync(d_alive, 0, (size_t)rows * sizeof(int32_t), s);
+    if (ce == cudaSuccess) {
+      noalloc_flags_kernel<<<64, 256, 0, s>>>(scratch, d_alive, (int32_t)rows);
+      ce = cudaGetLastError();
+    }
+  } else if (ce == cudaSuccess)
     ce = sdnn::launch_pdl(noalloc_flags_kernel, 64, 256, 0, s, (const NoAllocScratch*)scratch,
                           d_alive, (int32_t)rows);
   if (ce != cudaSuccess) {

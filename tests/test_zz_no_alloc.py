@@ -215,3 +215,37 @@ def test_noalloc_reports_a_device_wait_that_gave_up():
         d_in = torch.from_numpy(Y0).cuda()
         _run_twice(eng, 0, d_in, B, lambda y, a: np.testing.assert_array_equal(a, flags_ref))
         assert torch.cuda.current_device() == 0
+
+
+@pytest.mark.parametrize("N,rows", [(1024, 9), (4096, 150), (16384, 33)])
+@pytest.mark.parametrize("where", ["inputs", "outputs", "before the inputs"])
+def test_noalloc_flags_may_lie_in_the_rows(N, rows, where):
+    """d_alive inside the input rows (no longer needed after the call), inside
+    the output rows, or ending right before the inputs: the flags are those of
+    a buffer of their own, and so is every output that they do not cover."""
+    torch = pytest.importorskip("torch")
+    Y0 = sg.generate_inputs(N, 3, 0, rows)
+    Y0[rows // 2] = 0
+    with sg.Engine(N, 1, mode="SNIG", batch=rows, bias=-0.3, placement=False) as eng:
+        eng.generate_weights(2)
+        eng.finalize()
+        want = []
+        _run_twice(eng, 0, torch.from_numpy(Y0).cuda(), rows, lambda y, a: want.append((y, a)))
+        y_want, a_want = want[0]
+        assert 0 < a_want.sum() < rows
+        pad = (rows + 3) // 4 * 4
+        mem = torch.zeros(pad + rows * N, dtype=torch.float32, device="cuda")
+        x = mem[pad:].view(rows, N)
+        x.copy_(torch.from_numpy(Y0))
+        y = torch.full_like(x, -1.0)
+        flat = {"inputs": x, "outputs": y}[where].view(-1) if where != "before the inputs" else mem
+        at = pad - rows if where == "before the inputs" else N  # the second row on
+        alive = flat[at:at + rows].view(torch.int32)
+        assert _noalloc(eng, 0, x, y, rows, alive) == 0, sg.load().sdnn_last_error(eng._h)
+        torch.cuda.synchronize()
+        got = y.cpu().numpy().reshape(-1)
+        assert np.array_equal(alive.cpu().numpy(), a_want)
+        keep = np.ones(rows * N, bool)
+        if where == "outputs":
+            keep[at:at + rows] = False
+        assert _bits_equal(got[keep], y_want.reshape(-1)[keep])
