@@ -212,8 +212,10 @@ __global__ void __launch_bounds__(kRowWarps * 32) sparse_residue_kernel(const Sp
 #pragma unroll
       for (int h = 0; h < 8; ++h) {
         if (w0 + h < w_end) {
+          // (not computed where W Delta = 0: with no clamp, pre_c may be infinite)
           float* at = acc + (w0 + h) * 32 + lane;
-          const float y = clamp_hi(pc[h] + *at, hi) - clamp_hi(pc[h], hi);
+          const float d = *at;
+          const float y = d != 0.f ? clamp_hi(pc[h] + d, hi) - clamp_hi(pc[h], hi) : 0.f;
           *at = y;
           nz += y != 0.f;
         }

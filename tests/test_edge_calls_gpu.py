@@ -1,0 +1,45 @@
+"""Calls at the edges of what the engine takes: infinite clamps, weights that are
+loaded anew after a run, buffers that do not fit, in-degrees at the limits of
+the counting kernels.
+"""
+import numpy as np
+import pytest
+
+import snicit_gb300 as sg
+
+pytestmark = pytest.mark.gpu
+
+
+def _identity(N, vals):
+    j = np.arange(N)
+    return j, j, np.broadcast_to(np.float32(vals), (N,)).copy()
+
+
+def test_sparse_residues_beside_an_infinite_centroid():
+    """With no clamp, a centroid's pre-activation overflows at one neuron.  The
+    residue rows equal it there, so their residue stays 0 and they end infinite
+    as well (not NaN), as the same rows do without clustering."""
+    N, L, rows, hot = 1024, 4, 8, 100
+    rng = np.random.default_rng(2)
+    Y = np.tile(rng.integers(1, 256, N).astype(np.float32) / 256, (rows, 1))
+    Y[:, hot] = 1e30
+    for r in range(1, rows):
+        Y[r, 7 * r] += 1 / 256  # within the pruning limit of row 0
+    up = np.ones(N, np.float32)
+    up[hot] = 1e10
+    out = []
+    for mode in ("SNICIT", "SNIG"):
+        with sg.Engine(N, L, mode=mode, threshold=1, batch=rows, bias=0.0, clamp=np.inf,
+                       merge=False) as e:
+            for l in range(L):
+                e.set_layer_coo(l, *_identity(N, up if l == 1 else 1.0))
+            flags, _ = e.infer(Y)
+            out.append((flags, e.activations(rows)))
+            if mode == "SNICIT":
+                st = e.stats()
+                assert st["centroids"] == 1 and st["sparse_residue_rows"] == rows - 1, st
+    want = Y.copy()
+    want[:, hot] = np.inf
+    for flags, act in out:
+        assert flags.all()
+        assert np.array_equal(act, want)
