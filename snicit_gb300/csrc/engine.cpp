@@ -246,6 +246,7 @@ struct sdnn_engine {
   int launches = 0;
   bool have_run = false;
   int pending_stats = 0;
+  int last_tile = 0, last_threads = 0;  // of the last run's last layer (stats)
   sdnn_stats stats{};
 };
 
@@ -1634,6 +1635,10 @@ int run(sdnn_engine* e, int64_t rows, const float* d_in, int32_t* d_flags) {
     if ((rc = run_phase(e, 4, PH_FINISH, rows, d_in, d_flags))) return rc;
   }
   e->launches = e->run_launches;
+  // (the weights may be gone or others by the time the stats are asked for)
+  const bool resident = resident_on(e, e->L - 1);
+  e->last_tile = resident ? e->dl[e->L - 1].res.T : e->key.T;
+  e->last_threads = resident ? 512 : e->threads;
   e->have_run = true;
   e->pending_stats = 1;
   return SDNN_OK;
@@ -1731,9 +1736,8 @@ int collect_stats(sdnn_engine* e) {
   st.weight_nnz = e->total_nnz;
   st.launches = e->launches;
   st.threshold = T;
-  const bool resident = resident_on(e, L - 1);
-  st.tile_rows = resident ? e->dl[L - 1].res.T : e->key.T;
-  st.threads = resident ? 512 : e->threads;
+  st.tile_rows = e->last_tile;
+  st.threads = e->last_threads;
   st.input_pieces = e->last_pieces;
   st.centroid_candidates = e->cfg.num_centroids;
   st.merge_start = merging_on(e) ? (e->cfg.merge_start > 0 ? e->cfg.merge_start : kMergeStart) : 0;

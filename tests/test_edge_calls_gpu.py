@@ -43,3 +43,39 @@ def test_sparse_residues_beside_an_infinite_centroid():
     for flags, act in out:
         assert flags.all()
         assert np.array_equal(act, want)
+
+
+def test_stats_of_a_run_whose_weights_were_replaced(tmp_path):
+    """Statistics are those of the run, whatever became of its weights: a file
+    that loads but is refused when its layers are checked, then good weights
+    that take another kernel."""
+    torch = pytest.importorskip("torch")
+    N, L, rows = 1024, 3, 40
+    path = tmp_path / "w.sdnnw"
+    with sg.Engine(N, L, mode="SNIG", batch=rows, bias=-0.3) as e:
+        e.generate_weights(1)
+        e.save_packed(path)
+    image = bytearray(path.read_bytes())
+    at = 64 + 64 + ((N // 32 + 1) * 4 + 63) // 64 * 64  # the first layer's first slot
+    image[at:at + 2] = b"\xff\xff"
+    bad = tmp_path / "bad.sdnnw"
+    bad.write_bytes(image)
+    y = torch.from_numpy(sg.generate_inputs(N, 1, 0, rows)).cuda()
+    f = torch.zeros(rows, dtype=torch.int32, device="cuda")
+    shape = lambda st: (st["tile_rows"], st["threads"], st["rows_in"])
+    with sg.Engine(N, L, mode="SNIG", batch=rows, bias=-0.3) as e:
+        e.generate_weights(1)
+        e.infer_device(y.data_ptr(), rows, f.data_ptr())
+        want = shape(e.stats())
+        e.infer_device(y.data_ptr(), rows, f.data_ptr())
+        e.load_packed(bad)
+        with pytest.raises(sg.SdnnError):
+            e.finalize()
+        assert shape(e.stats()) == want
+        e.generate_weights(1)
+        e.infer_device(y.data_ptr(), rows, f.data_ptr())
+        e.generate_weights(1, nnz_per_row=200)  # too deep for the kernel of the run
+        e.finalize()
+        assert shape(e.stats()) == want
+        e.infer_device(y.data_ptr(), rows, f.data_ptr())
+        assert shape(e.stats()) != want
