@@ -1637,8 +1637,9 @@ int run(sdnn_engine* e, int64_t rows, const float* d_in, int32_t* d_flags) {
   e->launches = e->run_launches;
   // (the weights may be gone or others by the time the stats are asked for)
   const bool resident = resident_on(e, e->L - 1);
-  e->last_tile = resident ? e->dl[e->L - 1].res.T : e->key.T;
-  e->last_threads = resident ? 512 : e->threads;
+  const DevLayer& d = e->dl[e->L - 1];
+  e->last_tile = resident ? d.res.T : e->key.T;
+  e->last_threads = resident ? 512 : d.constw ? e->threads : e->threads_general;
   e->have_run = true;
   e->pending_stats = 1;
   return SDNN_OK;

@@ -79,3 +79,20 @@ def test_stats_of_a_run_whose_weights_were_replaced(tmp_path):
         assert shape(e.stats()) == want
         e.infer_device(y.data_ptr(), rows, f.data_ptr())
         assert shape(e.stats()) != want
+
+
+@pytest.mark.parametrize("values,threads", [(False, 1024), (True, 512)])
+def test_stats_name_the_threads_of_the_launch(values, threads):
+    """Layers with a value per edge run 512 threads where rows are split into
+    input chunks, layers with one value 1024."""
+    N, rows = 49152, 3
+    j = np.arange(N)
+    v = np.full(N, 0.5, np.float32)
+    if values:
+        v[::2] = 0.25
+    with sg.Engine(N, 1, mode="SNIG", batch=rows, bias=0.0) as e:
+        e.set_layer_coo(0, j, j[::-1].copy(), v)
+        Y = np.random.default_rng(1).integers(0, 8, (rows, N)).astype(np.float32)
+        e.infer(Y)
+        assert e.stats()["threads"] == threads
+        assert np.array_equal(e.activations(rows), (Y * v)[:, ::-1])
