@@ -661,8 +661,9 @@ int upload_layer(sdnn_engine* e, int l, const PackedView& p, std::string& err) {
   };
   const size_t none = ~(size_t)0;
   size_t o_val = none, o_bias = none, o_sums = none, o_tr_off = none, o_tr_out = none, o_tr_val = none;
-  image.reserve(nslot * (p.constw ? 2 : 6) + ngrp * 12 +
-                (e->sparse_built ? (size_t)p.nnz * (p.constw ? 2 : 6) : 0) + (size_t)e->N * 8 + 4096);
+  // (edges are at most the slots; a file's own count of them is not relied on)
+  image.reserve(nslot * (p.constw ? 2 : 6) * (e->sparse_built ? 2 : 1) + ngrp * 12 +
+                (size_t)e->N * 8 + 4096);
   const size_t o_idx = put(p.idx, nslot * 2);
   const size_t o_grp = put(p.grp_blk, ngrp * 4);
   const int32_t scale = slot_index_in_bytes(e->Q) ? 4 : 1;

@@ -96,3 +96,23 @@ def test_stats_name_the_threads_of_the_launch(values, threads):
         e.infer(Y)
         assert e.stats()["threads"] == threads
         assert np.array_equal(e.activations(rows), (Y * v)[:, ::-1])
+
+
+@pytest.mark.parametrize("nnz", [-1, 1 << 62])
+def test_packed_file_with_a_wrong_edge_count(tmp_path, nnz):
+    """The count of edges in a layer's header is for the statistics alone: a
+    wrong one changes neither the upload nor the results."""
+    N, rows = 1024, 20
+    path = tmp_path / "w.sdnnw"
+    Y = sg.generate_inputs(N, 1, 0, rows)
+    with sg.Engine(N, 2, mode="SNIG", batch=rows, bias=-0.3) as e:
+        e.generate_weights(1)
+        e.save_packed(path)
+        want, _ = e.infer(Y)
+    image = bytearray(path.read_bytes())
+    image[64 + 8:64 + 16] = nnz.to_bytes(8, "little", signed=True)
+    path.write_bytes(image)
+    with sg.Engine(N, 2, mode="SNIG", batch=rows, bias=-0.3) as e:
+        e.load_packed(path)
+        got, _ = e.infer(Y)
+    assert 0 < want.sum() < rows and np.array_equal(got, want)
