@@ -335,6 +335,7 @@ void free_buffers(sdnn_engine* e) {
   if (e->h_flags) cudaFreeHost(e->h_flags);
   e->h_ctl = e->h_flags = nullptr;
   e->report_valid = false;
+  e->have_run = false;  // the last inference's rows and counters went with them
   e->cap = 0;
 }
 

@@ -116,3 +116,26 @@ def test_packed_file_with_a_wrong_edge_count(tmp_path, nnz):
         e.load_packed(path)
         got, _ = e.infer(Y)
     assert 0 < want.sum() < rows and np.array_equal(got, want)
+
+
+def test_reads_after_buffers_that_did_not_fit():
+    """A call whose row buffers cannot be allocated leaves no inference to read
+    from; the next one that fits works."""
+    torch = pytest.importorskip("torch")
+    N, rows = 1024, 8
+    Y = sg.generate_inputs(N, 1, 0, rows)
+    y = torch.from_numpy(Y).cuda()
+    f = torch.zeros(rows, dtype=torch.int32, device="cuda")
+    with sg.Engine(N, 2, mode="SNIG", batch=rows, bias=-0.3) as e:
+        e.generate_weights(1)
+        want, _ = e.infer(Y)
+        act = e.activations(rows)
+        with pytest.raises(sg.SdnnError) as ei:
+            e.infer_device(y.data_ptr(), 1 << 30, f.data_ptr())  # 4 TB a buffer
+        assert ei.value.code == 3
+        for read in (lambda: e.activations(rows), e.layer_rows):
+            with pytest.raises(sg.SdnnError):
+                read()
+        got, _ = e.infer(Y)
+        assert np.array_equal(got, want)
+        assert np.array_equal(e.activations(rows).view(np.uint32), act.view(np.uint32))
