@@ -403,18 +403,30 @@ int choose_kernel(sdnn_engine* e) {
     if (req_T > 0 && k.T != req_T) continue;
     const size_t smem = (size_t)k.T * (size_t)(e->Q + 32) * 4;
     if (smem > kMaxSmem) continue;
-    if (!layer_instance_exists(k)) continue;
     // a tile that leaves room for one CTA per SM wants all its warps: 6000 rows
     // of 16384 neurons took 832 us with 512 threads (T = 2), 572 with 1024 (T = 3)
     if (e->cfg.threads == 0 && k.kg == 1) threads = smem > kMaxSmem / 2 ? 1024 : 512;
     LayerKernelKey kc = k, kg = k;
     kc.constw = true;
     kg.constw = false;
+    if (k.kg == 1 && smem > kMaxSmem / 2 && k.T <= 2) {
+      // One CTA per SM and few gathers a list to hide the next list's round
+      // trip: lists as one stream.  3000 rows, us in batches -> as a stream:
+      // 16384 neurons at 2 rows x 512 threads 617 -> 559 with values, 440 -> 427
+      // with one value; with values also at 1024 threads, 28672 at 2 rows 780 ->
+      // 757, 32768 at 1 row 1383 -> 1250, but with one value 847 -> 964.  From 3
+      // rows on, and where CTAs share an SM, batches win (fewer registers): 354
+      // -> 385 (16384, values, 3 x 1024), 138 -> 257 (60000 rows of 256, values),
+      // 339 -> 520 (of 1024, values, 16 x 512).
+      kg.ahead = true;
+      kc.ahead = threads <= 512;
+    }
     int threads_general = threads;
     if (e->cfg.threads == 0 && k.kg == 8) {
       kg.kg = 16;
       threads_general = 512;
     }
+    if (!layer_instance_exists(kc) || !layer_instance_exists(kg)) continue;
     const int b1 = layer_blocks_per_sm(kc, threads, smem);
     const int b2 = layer_blocks_per_sm(kg, threads_general, smem);
     if (b1 <= 0 || b2 <= 0) continue;

@@ -29,7 +29,9 @@ static const std::vector<LayerInstance>& registry() {
 
 static const LayerInstance* find(const LayerKernelKey& k) {
   for (const auto& e : registry())
-    if (e.T == k.T && e.rsw == k.rsw && e.kg == k.kg && e.constw == k.constw) return &e;
+    if (e.T == k.T && e.rsw == k.rsw && e.kg == k.kg && e.constw == k.constw &&
+        e.ahead == k.ahead)
+      return &e;
   return nullptr;
 }
 

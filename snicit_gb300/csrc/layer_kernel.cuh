@@ -116,23 +116,24 @@ __device__ __forceinline__ void apply_block(float (&acc)[T], uint2 iv, const flo
 }
 
 // Blocks of a list held in registers ahead of their use (per lane 2 registers
-// a block, 4 more for per-edge values).
-template <int T, bool CONSTW>
-constexpr int kAhead = CONSTW ? (T <= 8 ? 4 : 2) : (T <= 4 ? 2 : 1);
+// a block, 4 more for per-edge values); tiles of one or two rows.
+template <bool CONSTW>
+constexpr int kAhead = CONSTW ? 4 : 2;
 
 // The groups gbeg + warp, + nwarps, ... below gend of a tile in shared memory:
 // accumulates each group's list and hands (acc, group) to done().  The slot
 // lists are walked as one stream: a block's registers are refilled with the
 // block NB further on -- of this group or the next -- as soon as it has been
 // applied, so a warp never waits for a round trip to L2 between batches or
-// groups (the kernel before this one did, and shared memory stood idle a
-// quarter of the time).  A list ends at its last used slot, not at the end of
-// its last block of 4 (1.5 of 38 slots).
+// groups.  That costs registers (64 a thread against 32 to 64 in batches): it
+// pays where a CTA has its SM to itself and a list is few gathers, tiles of one
+// or two rows (choose_kernel has the times).  A list ends at its last used slot,
+// not at the end of its last block of 4 (1.5 of 38 slots).
 template <int T, int RSW, bool CONSTW, typename Done>
 __device__ __forceinline__ void walk_groups(const LayerDev& wl, const float* __restrict__ ys, int RS,
                                             int gbeg, int gend, int warp, int nwarps, int lane,
                                             Done done) {
-  constexpr int NB = kAhead<T, CONSTW>;
+  constexpr int NB = kAhead<CONSTW>;
   const float wc = wl.wconst;
   const uint2* __restrict__ idx = wl.idx + lane;
   const float4* __restrict__ val = CONSTW ? nullptr : wl.val + lane;
@@ -217,6 +218,41 @@ __device__ __forceinline__ void load_blocks(uint2 (&iv)[NB], float4 (&vv)[CONSTW
   for (int k = 0; k < NB; ++k) {
     iv[k] = __ldg(ip + (size_t)(b + k) * 32);
     if constexpr (!CONSTW) vv[k] = __ldg(vp + (size_t)(b + k) * 32);
+  }
+}
+
+// Accumulates the in-edges of group g from input chunk q into acc[T].
+// Slot blocks are fetched in batches of 8, then 2, then 1 (no predicated
+// tail): all indices of a batch are in registers before the first is used,
+// so a warp waits for one memory round trip per batch.
+template <int T, int RSW, bool CONSTW>
+__device__ __forceinline__ void accumulate_group(float (&acc)[T], const LayerDev& wl, int nq,
+                                                 const float* __restrict__ ys, int RS, int g,
+                                                 int q, int lane) {
+  const int32_t b0 = __ldg(wl.grp_blk + g * nq + q);
+  const int32_t b1 = __ldg(wl.grp_blk + g * nq + q + 1);
+  const uint2* __restrict__ ip = wl.idx + (size_t)b0 * 32 + lane;
+  const float4* __restrict__ vp = CONSTW ? nullptr : wl.val + (size_t)b0 * 32 + lane;
+  const float wc = wl.wconst;
+  const int nb = b1 - b0;
+  int b = 0;
+  for (; b + 8 <= nb; b += 8) {
+    uint2 iv[8];
+    float4 vv[CONSTW ? 1 : 8];
+    load_blocks<CONSTW, 8>(iv, vv, ip, vp, b);
+    apply_blocks<T, RSW, CONSTW, 8>(acc, iv, vv, wc, ys, RS);
+  }
+  for (; b + 2 <= nb; b += 2) {
+    uint2 iv[2];
+    float4 vv[CONSTW ? 1 : 2];
+    load_blocks<CONSTW, 2>(iv, vv, ip, vp, b);
+    apply_blocks<T, RSW, CONSTW, 2>(acc, iv, vv, wc, ys, RS);
+  }
+  if (b < nb) {
+    uint2 iv[1];
+    float4 vv[1];
+    load_blocks<CONSTW, 1>(iv, vv, ip, vp, b);
+    apply_blocks<T, RSW, CONSTW, 1>(acc, iv, vv, wc, ys, RS);
   }
 }
 
@@ -414,28 +450,38 @@ __device__ __forceinline__ Cut make_cut(int count, int G, int nwarps) {
 }
 
 // One piece of a tile: groups [gbeg, gend) of the rows in shared memory.
-template <int T, int RSW, bool CONSTW>
+template <int T, int RSW, bool CONSTW, bool AHEAD>
 __device__ __forceinline__ uint32_t run_piece(const LayerArgs& a, const float* ys, int RS,
                                               const int32_t* rows, int nrows, int gbeg, int gend,
                                               int warp, int nwarps, int lane) {
   uint32_t m = 0;
-  walk_groups<T, RSW, CONSTW>(a.w, ys, RS, gbeg, gend, warp, nwarps, lane,
-                              [&](const float (&acc)[T], int g) {
-                                m |= epilogue_group<T>(acc, a, rows, nrows, g, lane);
-                              });
+  if constexpr (AHEAD) {
+    walk_groups<T, RSW, CONSTW>(a.w, ys, RS, gbeg, gend, warp, nwarps, lane,
+                                [&](const float (&acc)[T], int g) {
+                                  m |= epilogue_group<T>(acc, a, rows, nrows, g, lane);
+                                });
+  } else {
+    for (int g = gbeg + warp; g < gend; g += nwarps) {
+      float acc[T];
+#pragma unroll
+      for (int t = 0; t < T; ++t) acc[t] = 0.f;
+      accumulate_group<T, RSW, CONSTW>(acc, a.w, 1, ys, RS, g, 0, lane);
+      m |= epilogue_group<T>(acc, a, rows, nrows, g, lane);
+    }
+  }
   return m;
 }
 // ... with the code of the smallest tile size that holds TE rows.
-template <int T, int P2, int RSW, bool CONSTW>
+template <int T, int P2, int RSW, bool CONSTW, bool AHEAD>
 __device__ __forceinline__ uint32_t run_sized(int TE, const LayerArgs& a, const float* ys, int RS,
                                               const int32_t* rows, int nrows, int gbeg, int gend,
                                               int warp, int nwarps, int lane) {
   if constexpr (P2 >= 1) {
     if (TE <= P2)
-      return run_sized<P2, P2 / 2, RSW, CONSTW>(TE, a, ys, RS, rows, nrows, gbeg, gend, warp,
-                                                nwarps, lane);
+      return run_sized<P2, P2 / 2, RSW, CONSTW, AHEAD>(TE, a, ys, RS, rows, nrows, gbeg, gend, warp,
+                                                       nwarps, lane);
   }
-  return run_piece<T, RSW, CONSTW>(a, ys, RS, rows, nrows, gbeg, gend, warp, nwarps, lane);
+  return run_piece<T, RSW, CONSTW, AHEAD>(a, ys, RS, rows, nrows, gbeg, gend, warp, nwarps, lane);
 }
 __host__ __device__ constexpr int pow2_below(int t) {
   int p = 1;
@@ -443,8 +489,8 @@ __host__ __device__ constexpr int pow2_below(int t) {
   return t > 1 ? p : 0;
 }
 
-template <int T, int RSW, bool CONSTW>
-__global__ void __launch_bounds__(1024, 1) layer_rows_kernel(const LayerArgs a) {
+template <int T, int RSW, bool CONSTW, bool AHEAD>
+__device__ __forceinline__ void layer_rows(const LayerArgs& a) {
   extern __shared__ __align__(128) float ys[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ int32_t s_rows[2][32];
@@ -519,8 +565,8 @@ __global__ void __launch_bounds__(1024, 1) layer_rows_kernel(const LayerArgs a) 
     if (s_fail) return;
     mbar_try_wait(&bar, phase);
     phase ^= 1u;
-    uint32_t m = run_sized<T, pow2_below(T), RSW, CONSTW>(cut.TE, a, ys, RS, s_rows[buf], nrows,
-                                                          gbeg, gend, warp, nwarps, lane);
+    uint32_t m = run_sized<T, pow2_below(T), RSW, CONSTW, AHEAD>(
+        cut.TE, a, ys, RS, s_rows[buf], nrows, gbeg, gend, warp, nwarps, lane);
     m = __reduce_or_sync(0xffffffffu, m);
     if (lane == 0 && m) atomicOr(&s_mask[buf], m);
     pending = true;
@@ -533,6 +579,22 @@ __global__ void __launch_bounds__(1024, 1) layer_rows_kernel(const LayerArgs a) 
   __syncthreads();
   if (warp == nwarps - 1)
     publish_rows(a, s_mask[buf ^ 1], pending_shared, s_rows[buf ^ 1], lane);
+}
+
+// Registers.  Where rows are short several CTAs share an SM, and half of them
+// at 64 registers a thread cost up to 1.7 times the time (60000 rows of 1024 with
+// values, 24 x 256: 447 -> 769 us; of 96: 142 -> 218); the compiler, left alone,
+// takes 32 to 64.  With one value and tiles of 4 to 8 rows it takes 32 and spills,
+// or leaves too few loads in flight: those have 48 (600 rows of 992, 8 x 512:
+// 16.5 -> 14.2 us; 20000 of 8192: 928 -> 895), or 32 without its spills at the
+// stride of 1024 (60000 rows, 8 x 1024: 373 -> 358).
+template <int T, int RSW, bool CONSTW, bool AHEAD>
+__global__ void __launch_bounds__(1024, AHEAD ? 1 : 0) layer_rows_kernel(const LayerArgs a) {
+  layer_rows<T, RSW, CONSTW, AHEAD>(a);
+}
+template <int T, int RSW, bool CONSTW>
+__global__ void __maxnreg__(RSW == 1056 ? 32 : 48) layer_rows_regs_kernel(const LayerArgs a) {
+  layer_rows<T, RSW, CONSTW, false>(a);
 }
 
 // ---------------------------------------------------------------------------
@@ -650,16 +712,26 @@ __global__ void __launch_bounds__(KG <= 8 ? 1024 : 512, 1) layer_chunk_kernel(co
   if (last_warp && s_ppending) publish_rows(a, s_pmask, sp.spl > 1, s_rows[s_pbuf], lane);
 }
 
-#define SDNN_ROWS_INSTANCE(T, RSW, CW) \
-  template __global__ void layer_rows_kernel<T, RSW, CW>(const LayerArgs);
 #define SDNN_CHUNK_INSTANCE(T, RSW, KG, CW) \
   template __global__ void layer_chunk_kernel<T, RSW, KG, CW>(const LayerArgs);
 
 // Registry entry used by the dispatcher.
 struct LayerInstance {
   int T, rsw, kg;
-  bool constw;
+  bool constw, ahead;
   const void* fn;
 };
+
+template <int T, int RSW, bool CONSTW, bool AHEAD>
+LayerInstance rows_instance() {
+  if constexpr (CONSTW && !AHEAD && T >= 4 && T <= 8)
+    return {T, RSW, 1, CONSTW, AHEAD, (const void*)&layer_rows_regs_kernel<T, RSW, CONSTW>};
+  else
+    return {T, RSW, 1, CONSTW, AHEAD, (const void*)&layer_rows_kernel<T, RSW, CONSTW, AHEAD>};
+}
+// ... for layers with a value per edge and with one value.
+#define SDNN_ROWS_INSTANCES(v, T, RSW, AHEAD)          \
+  v.push_back(rows_instance<T, RSW, false, AHEAD>()); \
+  v.push_back(rows_instance<T, RSW, true, AHEAD>())
 
 }  // namespace sdnn

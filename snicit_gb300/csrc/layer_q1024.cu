@@ -5,24 +5,11 @@
 
 namespace sdnn {
 
-SDNN_ROWS_INSTANCE(8, 1056, false)
-SDNN_ROWS_INSTANCE(8, 1056, true)
-SDNN_ROWS_INSTANCE(12, 1056, false)
-SDNN_ROWS_INSTANCE(12, 1056, true)
-SDNN_ROWS_INSTANCE(16, 1056, false)
-SDNN_ROWS_INSTANCE(16, 1056, true)
-SDNN_ROWS_INSTANCE(24, 1056, false)
-SDNN_ROWS_INSTANCE(24, 1056, true)
-
 void register_layer_q1024(std::vector<LayerInstance>& v) {
-  v.push_back({8, 1056, 1, false, (const void*)&layer_rows_kernel<8, 1056, false>});
-  v.push_back({8, 1056, 1, true, (const void*)&layer_rows_kernel<8, 1056, true>});
-  v.push_back({12, 1056, 1, false, (const void*)&layer_rows_kernel<12, 1056, false>});
-  v.push_back({12, 1056, 1, true, (const void*)&layer_rows_kernel<12, 1056, true>});
-  v.push_back({16, 1056, 1, false, (const void*)&layer_rows_kernel<16, 1056, false>});
-  v.push_back({16, 1056, 1, true, (const void*)&layer_rows_kernel<16, 1056, true>});
-  v.push_back({24, 1056, 1, false, (const void*)&layer_rows_kernel<24, 1056, false>});
-  v.push_back({24, 1056, 1, true, (const void*)&layer_rows_kernel<24, 1056, true>});
+  SDNN_ROWS_INSTANCES(v, 8, 1056, false);
+  SDNN_ROWS_INSTANCES(v, 12, 1056, false);
+  SDNN_ROWS_INSTANCES(v, 16, 1056, false);
+  SDNN_ROWS_INSTANCES(v, 24, 1056, false);
 }
 
 }  // namespace sdnn

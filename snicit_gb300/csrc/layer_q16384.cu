@@ -5,12 +5,6 @@
 
 namespace sdnn {
 
-SDNN_ROWS_INSTANCE(1, 16416, false)
-SDNN_ROWS_INSTANCE(1, 16416, true)
-SDNN_ROWS_INSTANCE(2, 16416, false)
-SDNN_ROWS_INSTANCE(2, 16416, true)
-SDNN_ROWS_INSTANCE(3, 16416, false)
-SDNN_ROWS_INSTANCE(3, 16416, true)
 SDNN_CHUNK_INSTANCE(1, 16416, 16, false)
 SDNN_CHUNK_INSTANCE(1, 16416, 16, true)
 SDNN_CHUNK_INSTANCE(2, 16416, 16, false)
@@ -27,26 +21,24 @@ SDNN_CHUNK_INSTANCE(1, 32800, 16, false)
 SDNN_CHUNK_INSTANCE(1, 32800, 16, true)
 
 void register_layer_q16384(std::vector<LayerInstance>& v) {
-  v.push_back({1, 16416, 1, false, (const void*)&layer_rows_kernel<1, 16416, false>});
-  v.push_back({1, 16416, 1, true, (const void*)&layer_rows_kernel<1, 16416, true>});
-  v.push_back({2, 16416, 1, false, (const void*)&layer_rows_kernel<2, 16416, false>});
-  v.push_back({2, 16416, 1, true, (const void*)&layer_rows_kernel<2, 16416, true>});
-  v.push_back({3, 16416, 1, false, (const void*)&layer_rows_kernel<3, 16416, false>});
-  v.push_back({3, 16416, 1, true, (const void*)&layer_rows_kernel<3, 16416, true>});
-  v.push_back({1, 16416, 16, false, (const void*)&layer_chunk_kernel<1, 16416, 16, false>});
-  v.push_back({1, 16416, 16, true, (const void*)&layer_chunk_kernel<1, 16416, 16, true>});
-  v.push_back({2, 16416, 16, false, (const void*)&layer_chunk_kernel<2, 16416, 16, false>});
-  v.push_back({2, 16416, 16, true, (const void*)&layer_chunk_kernel<2, 16416, 16, true>});
-  v.push_back({3, 16416, 16, false, (const void*)&layer_chunk_kernel<3, 16416, 16, false>});
-  v.push_back({3, 16416, 16, true, (const void*)&layer_chunk_kernel<3, 16416, 16, true>});
-  v.push_back({1, 16416, 8, false, (const void*)&layer_chunk_kernel<1, 16416, 8, false>});
-  v.push_back({1, 16416, 8, true, (const void*)&layer_chunk_kernel<1, 16416, 8, true>});
-  v.push_back({2, 16416, 8, false, (const void*)&layer_chunk_kernel<2, 16416, 8, false>});
-  v.push_back({2, 16416, 8, true, (const void*)&layer_chunk_kernel<2, 16416, 8, true>});
-  v.push_back({3, 16416, 8, false, (const void*)&layer_chunk_kernel<3, 16416, 8, false>});
-  v.push_back({3, 16416, 8, true, (const void*)&layer_chunk_kernel<3, 16416, 8, true>});
-  v.push_back({1, 32800, 16, false, (const void*)&layer_chunk_kernel<1, 32800, 16, false>});
-  v.push_back({1, 32800, 16, true, (const void*)&layer_chunk_kernel<1, 32800, 16, true>});
+  SDNN_ROWS_INSTANCES(v, 1, 16416, false);
+  SDNN_ROWS_INSTANCES(v, 2, 16416, false);
+  SDNN_ROWS_INSTANCES(v, 2, 16416, true);
+  SDNN_ROWS_INSTANCES(v, 3, 16416, false);
+  v.push_back({1, 16416, 16, false, false, (const void*)&layer_chunk_kernel<1, 16416, 16, false>});
+  v.push_back({1, 16416, 16, true, false, (const void*)&layer_chunk_kernel<1, 16416, 16, true>});
+  v.push_back({2, 16416, 16, false, false, (const void*)&layer_chunk_kernel<2, 16416, 16, false>});
+  v.push_back({2, 16416, 16, true, false, (const void*)&layer_chunk_kernel<2, 16416, 16, true>});
+  v.push_back({3, 16416, 16, false, false, (const void*)&layer_chunk_kernel<3, 16416, 16, false>});
+  v.push_back({3, 16416, 16, true, false, (const void*)&layer_chunk_kernel<3, 16416, 16, true>});
+  v.push_back({1, 16416, 8, false, false, (const void*)&layer_chunk_kernel<1, 16416, 8, false>});
+  v.push_back({1, 16416, 8, true, false, (const void*)&layer_chunk_kernel<1, 16416, 8, true>});
+  v.push_back({2, 16416, 8, false, false, (const void*)&layer_chunk_kernel<2, 16416, 8, false>});
+  v.push_back({2, 16416, 8, true, false, (const void*)&layer_chunk_kernel<2, 16416, 8, true>});
+  v.push_back({3, 16416, 8, false, false, (const void*)&layer_chunk_kernel<3, 16416, 8, false>});
+  v.push_back({3, 16416, 8, true, false, (const void*)&layer_chunk_kernel<3, 16416, 8, true>});
+  v.push_back({1, 32800, 16, false, false, (const void*)&layer_chunk_kernel<1, 32800, 16, false>});
+  v.push_back({1, 32800, 16, true, false, (const void*)&layer_chunk_kernel<1, 32800, 16, true>});
 }
 
 }  // namespace sdnn

@@ -5,28 +5,12 @@
 
 namespace sdnn {
 
-SDNN_ROWS_INSTANCE(2, 4128, false)
-SDNN_ROWS_INSTANCE(2, 4128, true)
-SDNN_ROWS_INSTANCE(3, 4128, false)
-SDNN_ROWS_INSTANCE(3, 4128, true)
-SDNN_ROWS_INSTANCE(4, 4128, false)
-SDNN_ROWS_INSTANCE(4, 4128, true)
-SDNN_ROWS_INSTANCE(5, 4128, false)
-SDNN_ROWS_INSTANCE(5, 4128, true)
-SDNN_ROWS_INSTANCE(6, 4128, false)
-SDNN_ROWS_INSTANCE(6, 4128, true)
-
 void register_layer_q4096(std::vector<LayerInstance>& v) {
-  v.push_back({2, 4128, 1, false, (const void*)&layer_rows_kernel<2, 4128, false>});
-  v.push_back({2, 4128, 1, true, (const void*)&layer_rows_kernel<2, 4128, true>});
-  v.push_back({3, 4128, 1, false, (const void*)&layer_rows_kernel<3, 4128, false>});
-  v.push_back({3, 4128, 1, true, (const void*)&layer_rows_kernel<3, 4128, true>});
-  v.push_back({4, 4128, 1, false, (const void*)&layer_rows_kernel<4, 4128, false>});
-  v.push_back({4, 4128, 1, true, (const void*)&layer_rows_kernel<4, 4128, true>});
-  v.push_back({5, 4128, 1, false, (const void*)&layer_rows_kernel<5, 4128, false>});
-  v.push_back({5, 4128, 1, true, (const void*)&layer_rows_kernel<5, 4128, true>});
-  v.push_back({6, 4128, 1, false, (const void*)&layer_rows_kernel<6, 4128, false>});
-  v.push_back({6, 4128, 1, true, (const void*)&layer_rows_kernel<6, 4128, true>});
+  SDNN_ROWS_INSTANCES(v, 2, 4128, false);
+  SDNN_ROWS_INSTANCES(v, 3, 4128, false);
+  SDNN_ROWS_INSTANCES(v, 4, 4128, false);
+  SDNN_ROWS_INSTANCES(v, 5, 4128, false);
+  SDNN_ROWS_INSTANCES(v, 6, 4128, false);
 }
 
 }  // namespace sdnn

@@ -32,42 +32,6 @@ namespace sdnn {
 
 constexpr int kChainCluster = 8;
 
-// Accumulates the in-edges of group g from input chunk q into acc[T].
-// Slot blocks are fetched in batches of 8, then 2, then 1 (no predicated
-// tail): all indices of a batch are in registers before the first is used,
-// so a warp waits for one memory round trip per batch (a chain layer has one
-// or two groups per warp and nothing else to hide that latency).
-template <int T, int RSW, bool CONSTW>
-__device__ __forceinline__ void accumulate_group(float (&acc)[T], const LayerDev& wl, int nq,
-                                                 const float* __restrict__ ys, int RS, int g,
-                                                 int q, int lane) {
-  const int32_t b0 = __ldg(wl.grp_blk + g * nq + q);
-  const int32_t b1 = __ldg(wl.grp_blk + g * nq + q + 1);
-  const uint2* __restrict__ ip = wl.idx + (size_t)b0 * 32 + lane;
-  const float4* __restrict__ vp = CONSTW ? nullptr : wl.val + (size_t)b0 * 32 + lane;
-  const float wc = wl.wconst;
-  const int nb = b1 - b0;
-  int b = 0;
-  for (; b + 8 <= nb; b += 8) {
-    uint2 iv[8];
-    float4 vv[CONSTW ? 1 : 8];
-    load_blocks<CONSTW, 8>(iv, vv, ip, vp, b);
-    apply_blocks<T, RSW, CONSTW, 8>(acc, iv, vv, wc, ys, RS);
-  }
-  for (; b + 2 <= nb; b += 2) {
-    uint2 iv[2];
-    float4 vv[CONSTW ? 1 : 2];
-    load_blocks<CONSTW, 2>(iv, vv, ip, vp, b);
-    apply_blocks<T, RSW, CONSTW, 2>(acc, iv, vv, wc, ys, RS);
-  }
-  if (b < nb) {
-    uint2 iv[1];
-    float4 vv[1];
-    load_blocks<CONSTW, 1>(iv, vv, ip, vp, b);
-    apply_blocks<T, RSW, CONSTW, 1>(acc, iv, vv, wc, ys, RS);
-  }
-}
-
 template <int RSW, int KC>
 __global__ void __launch_bounds__(1024, 1) chain_kernel(const ChainArgs a) {
   extern __shared__ __align__(128) float rows[];  // [2][KC][RSW]

@@ -71,6 +71,7 @@ struct LayerKernelKey {
   int rsw;     // compile-time smem row stride in floats (0 = runtime)
   int kg;      // groups per warp held across chunks (1 = no chunking)
   bool constw;
+  bool ahead;  // whole rows: lists fetched ahead as one stream (else in batches)
 };
 
 // Launches the layer kernel instance matching key; returns cudaErrorInvalidValue

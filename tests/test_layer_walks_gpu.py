@@ -1,0 +1,61 @@
+"""The streamed-list kernel's two ways through a list -- in batches, and as one
+stream where a CTA of few rows has its SM to itself -- at the widths and shapes
+on both sides of the rule between them.
+
+Both add an output's products in slot order: the rows must agree bit for bit,
+and lie within the rounding bound of a sum of n products in FP32,
+(n + 2) * 2^-24 * (sum |w y| + |b|), of FP64.
+"""
+import numpy as np
+import pytest
+
+import snicit_gb300 as sg
+
+pytestmark = pytest.mark.gpu
+
+
+def _net(N, nnz, values, seed):
+    rng = np.random.default_rng([seed, N, nnz])
+    width = N // nnz
+    cols = rng.integers(0, width, (N, nnz)) + np.arange(nnz) * width
+    vals = rng.standard_normal(N * nnz) * 0.3 if values else np.full(N * nnz, 0.0625)
+    return np.repeat(np.arange(N), nnz), cols.reshape(-1), vals.astype(np.float32)
+
+
+@pytest.mark.parametrize("values", [False, True])
+@pytest.mark.parametrize("N,shapes", [
+    (32, [(0, 0), (1, 256), (8, 1024)]), (96, [(0, 0), (2, 512)]), (992, [(0, 0), (4, 1024)]),
+    (1024, [(16, 512), (24, 256), (12, 512), (8, 1024)]),
+    (4096, [(2, 1024), (3, 512), (4, 512), (5, 512), (6, 512)]),
+    (8192, [(0, 0), (2, 512), (1, 256)]),            # 4 rows; 2: two CTAs on an SM
+    (16384, [(0, 0), (2, 512), (2, 1024), (1, 512)]),  # stream at 2 x 512 only
+    (20480, [(0, 0), (2, 512), (1, 512)]),
+    (32768, [(0, 0), (1, 512), (1, 256)]),           # stream with values, and below 1024 threads
+])
+def test_lists_in_batches_and_as_a_stream_agree(N, shapes, values):
+    nnz = min(32, N // 2)
+    r, c, v = _net(N, nnz, values, 12)
+    bias = -0.2
+    rng = np.random.default_rng(N + values)
+    order = np.argsort(c, kind="stable")
+    n = np.bincount(c, minlength=N)
+    start = np.concatenate([[0], np.cumsum(n)])[:-1]
+    for rows in (1, 5, 333):
+        Y = np.where(rng.random((rows, N)) < 0.4, rng.random((rows, N)) * 3, 0).astype(np.float32)
+        got = []
+        for tile, threads in shapes:
+            with sg.Engine(N, 1, mode="SNIG", batch=rows, bias=bias, tile_rows=tile,
+                           threads=threads) as e:
+                e.set_layer_coo(0, r, c, v)
+                flags, _ = e.infer(Y)
+                got.append((flags, e.activations(rows)))
+        for flags, act in got[1:]:
+            assert np.array_equal(flags, got[0][0])
+            assert np.array_equal(act.view(np.uint32), got[0][1].view(np.uint32))
+        some = np.unique(np.linspace(0, rows - 1, 12).astype(int))  # FP64: a dozen of the rows
+        P = Y[some][:, r[order]].astype(np.float64) * v[order]
+        at = np.minimum(start, P.shape[1] - 1)
+        S, A = (np.where(n > 0, np.add.reduceat(x, at, axis=1), 0) for x in (P, np.abs(P)))
+        b = float(np.float32(bias))
+        bound = (n + 2) * 2.0 ** -24 * (A + abs(b))
+        assert np.all(np.abs(got[0][1][some] - np.clip(S + b, 0, 32)) <= bound)
