@@ -951,9 +951,11 @@ int finalize_weights(sdnn_engine* e) {
 
 // Whether layer l runs on the kernel that keeps its slot lists in tensor
 // memory: wherever that kernel applies, unless the caller asked for a tile
-// shape (tile_rows, threads) of the streaming kernel.
-bool resident_on(const sdnn_engine* e, int l) {
-  return e->cfg.tile_rows == 0 && e->cfg.threads == 0 && e->dl[l].res.fn;
+// shape (tile_rows, threads) of the streaming kernel.  `rows`: as many as there
+// may be (an inference's graph serves every count that its buffers hold).
+bool resident_on(const sdnn_engine* e, int l, int64_t rows) {
+  const ResidentPlan& p = e->dl[l].res;
+  return e->cfg.tile_rows == 0 && e->cfg.threads == 0 && p.fn && rows <= p.most_rows;
 }
 
 int layer_launch(sdnn_engine* e, int l, int epi, const float* in, float* out, const int32_t* lin,
@@ -993,7 +995,7 @@ int layer_launch(sdnn_engine* e, int l, int epi, const float* in, float* out, co
     a.next = e->dl[l + 1].idx;
     a.next_bytes = e->dl[l + 1].list_bytes;
   }
-  if (resident_on(e, l)) {
+  if (resident_on(e, l, e->cap)) {
     CK(launch_layer_resident(d.res, a, e->stream));
   } else {
     CK(launch_layer(d.constw ? e->key : e->key_general, a, d.constw ? e->grid : e->grid_general,
@@ -1650,7 +1652,7 @@ int run(sdnn_engine* e, int64_t rows, const float* d_in, int32_t* d_flags) {
   }
   e->launches = e->run_launches;
   // (the weights may be gone or others by the time the stats are asked for)
-  const bool resident = resident_on(e, e->L - 1);
+  const bool resident = resident_on(e, e->L - 1, e->cap);
   const DevLayer& d = e->dl[e->L - 1];
   e->last_tile = resident ? d.res.T : e->key.T;
   e->last_threads = resident ? 512 : d.constw ? e->threads : e->threads_general;
@@ -2522,10 +2524,10 @@ void engine_set_merge(sdnn_engine* e, int start, int every, bool on) {
 sdnn_config engine_config(const sdnn_engine* e) { return e->cfg; }
 
 // Fills the weight/shape part of the layer-kernel arguments of `layer` and the
-// launch shape, without allocating anything: the weights must already be on
+// launch shape for `rows` rows, without allocating anything: the weights must already be on
 // the device (sdnn_finalize_weights or an earlier inference).
-int engine_layer_setup(sdnn_engine* e, int layer, LayerArgs* a, LayerKernelKey* key, int* grid,
-                       int* threads, size_t* smem, ResidentPlan* res) {
+int engine_layer_setup(sdnn_engine* e, int layer, int64_t rows, LayerArgs* a, LayerKernelKey* key,
+                       int* grid, int* threads, size_t* smem, ResidentPlan* res) {
   if (layer < 0 || layer >= e->L) return fail(e, SDNN_ERR_INVALID, "bad layer");
   if (!e->stream || e->weights_dirty || (int)e->dl.size() != e->L)
     return fail(e, SDNN_ERR_STATE, "weights are not on the device: call sdnn_finalize_weights first");
@@ -2536,7 +2538,7 @@ int engine_layer_setup(sdnn_engine* e, int layer, LayerArgs* a, LayerKernelKey* 
   }
   const DevLayer& d = e->dl[layer];
   const LayerKernelKey k = d.constw ? e->key : e->key_general;
-  *res = resident_on(e, layer) ? d.res : ResidentPlan{};
+  *res = resident_on(e, layer, rows) ? d.res : ResidentPlan{};
   if (res->fn) CK(resident_prepare(*res));
   else CK(layer_prepare(k));
   *a = LayerArgs{};

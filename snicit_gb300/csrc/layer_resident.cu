@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1)
   __shared__ int2 s_lists[kWarps][kGroups<CONSTW>];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int RS = RSW > 0 ? RSW : a.Q + 32;
+  constexpr int RS = RSW;  // (the zero columns are at a.Q, whatever the stride)
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (tid == kWarps * 32 - 32) fetch_next_lists(a);
   // Engines that work side by side take a share of the SMs each: a CTA fills
@@ -452,6 +452,10 @@ __global__ void __launch_bounds__(kWarps * 32, 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
+// Row strides of the widths without one of their own (their indices are in
+// floats), each for the widths that it holds with the zero columns.
+constexpr int kStride1536 = 1568, kStride2368 = 2400, kStride4064 = 4096;
+
 struct Instance {
   int T, rsw;
   bool constw;
@@ -460,8 +464,9 @@ struct Instance {
 #define SDNN_RESIDENT(T, RSW) \
   {T, RSW, true, (const void*)&layer_resident_kernel<T, RSW, true>}, \
       {T, RSW, false, (const void*)&layer_resident_kernel<T, RSW, false>}
-const Instance kInstances[] = {SDNN_RESIDENT(8, 1056), SDNN_RESIDENT(6, 4128), SDNN_RESIDENT(8, 0),
-                               SDNN_RESIDENT(6, 0)};
+const Instance kInstances[] = {SDNN_RESIDENT(8, 1056), SDNN_RESIDENT(8, kStride1536),
+                               SDNN_RESIDENT(8, kStride2368), SDNN_RESIDENT(6, kStride4064),
+                               SDNN_RESIDENT(6, 4128)};
 
 const void* find_instance(int T, int rsw, bool constw) {
   for (const Instance& e : kInstances)
@@ -506,17 +511,33 @@ ResidentPlan resident_plan(int N, bool constw, int max_depth, int num_sms) {
   const int held = 4 * (constw ? kResBlocks<true> : kResBlocks<false>);
   if (N % 32 != 0 || N < 1024 || N > 4096 || max_depth > 2 * held) return p;
   p.split = (G + per_cta - 1) / per_cta;
-  p.rsw = N == 1024 ? 1056 : N == 4096 ? 4128 : 0;
-  const size_t row = (size_t)(N + 32) * 4;
-  // 8 rows where three stages of them fit (N <= 2300), else two stages of 6:
-  // at N = 4096 three stages of 4 rows took 1208 us for 60000 rows, two of 6
-  // 1119 (fewer list words and group turns per row); at N = 1024 16 rows are no
-  // faster than 8 (285 against 290 us) and leave more of the last round empty
-  // (10000 rows: 76 against 64 us).
+  // Strides are known when compiling: every gather then has its row's offset as
+  // an immediate (60000 rows, us, stride N + 32 at run time -> one of these:
+  // 2048 neurons 563 -> 531, 4064 1168 -> 1094, with values 1509 -> 1380; 3072
+  // with values 1147 -> 1040, where lists streamed per tile took 1084).
+  p.rsw = N == 1024 ? 1056
+          : N == 4096 ? 4128
+          : N <= kStride1536 - 32 ? kStride1536
+          : N <= kStride2368 - 32 ? kStride2368
+                                  : kStride4064;
+  const size_t row = (size_t)p.rsw * 4;
+  // 8 rows where three stages of them fit, else two stages of 6: at N = 4096
+  // three stages of 4 rows took 1208 us for 60000 rows, two of 6 1119 (fewer
+  // list words and group turns per row); at N = 1024 16 rows are no faster than
+  // 8 (285 against 290 us) and leave more of the last round empty (10000 rows:
+  // 76 against 64 us).
   p.T = 3 * 8 * row <= kResSmem ? 8 : 6;
   p.stages = (int)std::min<size_t>(kMaxStages, kResSmem / (p.T * row));
   p.smem = p.stages * p.T * row;
   p.fn = find_instance(p.T, p.rsw, constw);
+  // A warp with one group more than the others holds up its CTA: just past a
+  // width that fills the warps' turns, lists streamed per tile are faster for
+  // many rows (60000 rows, us, streamed against kept: 1056 neurons with values
+  // 411 against 507, 1088 429 against 477; 2080 with one value 660 against 707,
+  // but 1056 361 against 363).  Up to 4096 rows they are level or slower (300
+  // rows, 40 layers: 366 against 303).
+  const int turns = p.split * kWarps * ((G + p.split * kWarps - 1) / (p.split * kWarps));
+  if (G < (constw ? 0.68 : 0.55) * turns) p.most_rows = 4096;
   p.few = few_rows(p, N, constw, num_sms);
   return p;
 }

@@ -24,8 +24,8 @@
 #include "snicit_gb300.h"
 
 namespace sdnn {
-int engine_layer_setup(sdnn_engine* e, int layer, LayerArgs* a, LayerKernelKey* key, int* grid,
-                       int* threads, size_t* smem, ResidentPlan* res);
+int engine_layer_setup(sdnn_engine* e, int layer, int64_t rows, LayerArgs* a, LayerKernelKey* key,
+                       int* grid, int* threads, size_t* smem, ResidentPlan* res);
 cudaStream_t engine_stream(const sdnn_engine* e);
 void engine_set_error(sdnn_engine* e, const std::string& msg);
 }  // namespace sdnn
@@ -133,7 +133,7 @@ extern "C" int sdnn_layer_noalloc(sdnn_engine* e, int32_t layer, const float* d_
   sdnn::ResidentPlan res;
   int grid = 0, threads = 0;
   size_t smem = 0;
-  int rc = sdnn::engine_layer_setup(e, layer, &a, &key, &grid, &threads, &smem, &res);
+  int rc = sdnn::engine_layer_setup(e, layer, rows, &a, &key, &grid, &threads, &smem, &res);
   if (rc) return rc;
   // CTAs that share a tile write one row's outputs while others may still be
   // loading that row: input and output must not overlap
@@ -194,7 +194,7 @@ extern "C" int sdnn_selftest_noalloc_timeout(sdnn_engine* e, int32_t* d_alive, i
   sdnn::ResidentPlan res;
   int grid = 0, threads = 0;
   size_t smem = 0;
-  int rc = sdnn::engine_layer_setup(e, 0, &a, &key, &grid, &threads, &smem, &res);  // engine's device
+  int rc = sdnn::engine_layer_setup(e, 0, rows, &a, &key, &grid, &threads, &smem, &res);  // engine's device
   if (rc) return rc;
   NoAllocScratch* scratch = nullptr;
   rc = scratch_address(e, &scratch);

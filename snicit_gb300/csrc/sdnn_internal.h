@@ -126,6 +126,7 @@ struct ResidentPlan {
   int T, rsw, split, stages;
   size_t smem;
   FewRows few;
+  int64_t most_rows = INT32_MAX;  // for more, lists streamed per tile are faster
 };
 ResidentPlan resident_plan(int N, bool constw, int max_depth, int num_sms);
 cudaError_t resident_prepare(const ResidentPlan& p);

@@ -33,14 +33,48 @@ def _net(N, nnz, values, seed):
     (32768, [(0, 0), (1, 512), (1, 256)]),           # stream with values, and below 1024 threads
 ])
 def test_lists_in_batches_and_as_a_stream_agree(N, shapes, values):
-    nnz = min(32, N // 2)
+    _same_rows(N, min(32, N // 2), values, shapes, (1, 5, 333))
+
+
+@pytest.mark.parametrize("values", [False, True])
+@pytest.mark.parametrize("N,nnz", [
+    (1056, 32), (1088, 32), (1536, 32), (1568, 32), (2080, 32), (2368, 32), (2400, 32), (3072, 32),
+    (4064, 32), (1536, 72), (2368, 44), (3072, 72)])  # 72, 44: past the slots that a warp keeps
+def test_kept_lists_at_every_stride(N, nnz, values):
+    """Widths on both sides of the strides that the kernel with kept lists is
+    built for, against lists streamed per tile."""
+    _same_rows(N, nnz, values, [(0, 0), (8 if N < 2400 else 4, 512)], (1, 7, 401))
+
+
+@pytest.mark.parametrize("N,values", [(1056, True), (2080, False)])
+def test_many_rows_of_widths_that_fill_the_turns_badly(N, values):
+    """Widths where buffers for more than 4096 rows take the other kernel: the
+    same bits from an engine with small buffers and from one with large."""
+    r, c, v = _net(N, 32, values, 13)
+    rng = np.random.default_rng(N)
+    Y = np.where(rng.random((4200, N)) < 0.4, rng.random((4200, N)) * 3, 0).astype(np.float32)
+    out = []
+    for batch in (4096, 4097):
+        with sg.Engine(N, 2, mode="SNIG", batch=batch, bias=-0.3) as e:
+            for l in range(2):
+                e.set_layer_coo(l, r, c, v)
+            flags, _ = e.infer(Y[:batch])
+            out.append((flags[:4000], e.activations(4000)))
+            f, _ = e.infer(Y[:77])
+            assert np.array_equal(f, flags[:77])
+            assert np.array_equal(e.activations(77).view(np.uint32), out[-1][1][:77].view(np.uint32))
+    assert np.array_equal(out[0][0], out[1][0])
+    assert np.array_equal(out[0][1].view(np.uint32), out[1][1].view(np.uint32))
+
+
+def _same_rows(N, nnz, values, shapes, counts):
     r, c, v = _net(N, nnz, values, 12)
     bias = -0.2
     rng = np.random.default_rng(N + values)
     order = np.argsort(c, kind="stable")
     n = np.bincount(c, minlength=N)
     start = np.concatenate([[0], np.cumsum(n)])[:-1]
-    for rows in (1, 5, 333):
+    for rows in counts:
         Y = np.where(rng.random((rows, N)) < 0.4, rng.random((rows, N)) * 3, 0).astype(np.float32)
         got = []
         for tile, threads in shapes:
@@ -53,9 +87,9 @@ def test_lists_in_batches_and_as_a_stream_agree(N, shapes, values):
             assert np.array_equal(flags, got[0][0])
             assert np.array_equal(act.view(np.uint32), got[0][1].view(np.uint32))
         some = np.unique(np.linspace(0, rows - 1, 12).astype(int))  # FP64: a dozen of the rows
-        P = Y[some][:, r[order]].astype(np.float64) * v[order]
-        at = np.minimum(start, P.shape[1] - 1)
-        S, A = (np.where(n > 0, np.add.reduceat(x, at, axis=1), 0) for x in (P, np.abs(P)))
+        P = np.zeros((len(some), len(c) + 1))  # (the last column: outputs without edges)
+        P[:, :-1] = Y[some][:, r[order]].astype(np.float64) * v[order]
+        S, A = (np.where(n > 0, np.add.reduceat(x, start, axis=1), 0) for x in (P, np.abs(P)))
         b = float(np.float32(bias))
         bound = (n + 2) * 2.0 ** -24 * (A + abs(b))
         assert np.all(np.abs(got[0][1][some] - np.clip(S + b, 0, 32)) <= bound)
