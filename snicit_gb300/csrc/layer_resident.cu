@@ -56,6 +56,9 @@ template <bool CONSTW>
 constexpr int kGroupCols = kCols / kGroups<CONSTW>;
 constexpr size_t kResSmem = 225 * 1024;
 
+__device__ __forceinline__ void tmem_free(uint32_t base) {
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(base) : "memory");
+}
 __device__ __forceinline__ void tmem_st2(uint32_t addr, uint2 v) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(v.x), "r"(v.y)
                : "memory");
@@ -258,7 +261,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1)
   __shared__ uint32_t s_mask[kMaxStages];
   __shared__ int32_t s_done[kMaxStages];
   __shared__ uint32_t s_tmem;
-  __shared__ int32_t s_count;
+  __shared__ int32_t s_count, s_share;
   __shared__ bool s_many;
   __shared__ int2 s_lists[kWarps][kGroups<CONSTW>];
 
@@ -271,30 +274,51 @@ __global__ void __launch_bounds__(kWarps * 32, 1)
   // and all.  (The number is set before the inference's first launch.)  A
   // server of 4 slots at 2000 requests a second: median latency 12.2 -> 7.8 ms
   // with merging, 11.9 -> 5.8 without.
-  const unsigned share = a.share ? (unsigned)__ldcg(a.share) : 1u;
-  const unsigned grid = max((unsigned)f.teams / share, 1u) * plan_split;
-  if (blockIdx.x >= grid) return;
-  const unsigned few = (unsigned)f.few / share;
-  // ---- before the previous launch has ended: nothing it writes is read
+  auto grid_of = [&](unsigned share) { return max((unsigned)f.teams / share, 1u) * plan_split; };
+  // ---- before the previous launch has ended: nothing it writes is relied on.
+  // Each warp sets up a part, the loads beside the taking of tensor memory (0.8
+  // us): one after the other, a layer that no row reaches -- every one after the
+  // last row has died -- took 2.65 us, now 1.9; the kernel with lists streamed
+  // per tile takes 1.55.  (Taking it only once rows are known to come: 1.8, but
+  // 0.8 more where they do.  A warp more to read the count meanwhile: 1.75, but
+  // 96 registers a thread, 2 % of a layer of many rows.)
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
-                     smem_u32(&s_tmem))
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    // Where there are many rows, the lists are kept before the previous launch
+    // has ended.  That is then known only roughly (the counts may still grow): a
+    // wrong guess costs time, not results.
+    int rows = a.rows, share = 1;
+    if (a.hint) rows = max(__ldcg(a.hint), __ldcg(a.count_in));
+    if (a.share) share = __ldcg(a.share);
+    if (lane == 0) {
+      s_many = rows > f.few / share;
+      s_share = share;
+    }
+  } else if (warp == 1) {
+    if (!a.share || blockIdx.x < grid_of(__ldcg(a.share))) {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+                       smem_u32(&s_tmem))
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+  } else if (warp == 2) {
+    if (lane < kMaxStages) {
+      mbar_init(&full[lane], 1);
+      s_mask[lane] = 0;
+      s_done[lane] = 0;
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  } else {
+    for (int i = warp - 3; i < T * stages; i += kWarps - 3) ring[(size_t)i * RS + a.Q + lane] = 0.f;
   }
-  for (int i = warp; i < T * stages; i += kWarps) ring[(size_t)i * RS + a.Q + lane] = 0.f;
-  if (tid < kMaxStages) {
-    mbar_init(&full[tid], 1);
-    s_mask[tid] = 0;
-    s_done[tid] = 0;
-  }
-  if (tid == 0) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  // the warp's columns: its quarter of the lanes, 128 of the 512 columns
   const uint32_t tmem = s_tmem;
+  const unsigned share = (unsigned)s_share, grid = grid_of(share);
+  if (blockIdx.x >= grid) return;
+  const unsigned few = (unsigned)f.few / share;
+  // the warp's columns: its quarter of the lanes, 128 of the 512 columns
   const uint32_t col = tmem + ((uint32_t)(warp & 3) << 21) + (uint32_t)(warp >> 2) * kCols;
   // The CTAs of a tile (its "split"), and with it the groups of this warp.
   int split = 0, part, team, teams, first_grp, step0, step1, n = 0;
@@ -352,27 +376,18 @@ __global__ void __launch_bounds__(kWarps * 32, 1)
     cur.load(col, 0);
     cur.wait();
   };
-  // Where there are many rows, the lists are kept before the previous launch
-  // has ended.  That is then known only roughly (the counts may still grow): a
-  // wrong guess costs time, not results.
-  if (warp == 0) {
-    bool many = a.rows > (int)few;
-    if (a.hint) many = max(__ldcg(a.hint), __ldcg(a.count_in)) > (int)few;
-    if (lane == 0) s_many = many;
-  }
-  __syncthreads();
   if (s_many) {
     assign(plan_split);
     keep_lists();
   }
-
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (warp == 0) {
-    const int c = __ldcg(a.count_in);
-    if (lane == 0) s_count = c;
-  }
+  if (tid == 0) s_count = __ldcg(a.count_in);
   __syncthreads();
   const unsigned count = (unsigned)s_count;
+  if (count == 0) {
+    if (warp == 1) tmem_free(tmem);
+    return;
+  }
   unsigned TE, tiles;
   int sp = plan_split;
   if (count > few) {
@@ -448,8 +463,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1)
     }
   }
   __syncthreads();
-  if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+  if (warp == 1) tmem_free(tmem);
 }
 
 // Row strides of the widths without one of their own (their indices are in

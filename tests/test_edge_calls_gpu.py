@@ -139,3 +139,25 @@ def test_reads_after_buffers_that_did_not_fit():
         got, _ = e.infer(Y)
         assert np.array_equal(got, want)
         assert np.array_equal(e.activations(rows).view(np.uint32), act.view(np.uint32))
+
+
+@pytest.mark.parametrize("N", [992, 1024, 1088, 2400, 4096, 65536])
+@pytest.mark.parametrize("mode", ["SNIG", "SNICIT"])
+def test_layers_that_no_row_reaches(N, mode):
+    """Every row dies in the first layer; the layers after it find none, and the
+    next call is as if that one had not been."""
+    rows = 70
+    Y = sg.generate_inputs(N, 8, 0, rows)
+    with sg.Engine(N, 6, mode=mode, threshold=4, batch=rows, bias=-0.01) as e:
+        e.generate_weights(3)
+        want, _ = e.infer(Y)
+        act = e.activations(rows)
+        assert want.any()
+        for n in (1, rows):
+            flags, ids = e.infer(np.zeros((n, N), np.float32))
+            assert not flags.any() and len(ids) == 0
+            assert not e.activations(n).any()
+            assert list(e.layer_rows()) == [n] + [0] * 5
+        flags, _ = e.infer(Y)
+        assert np.array_equal(flags, want)
+        assert np.array_equal(e.activations(rows).view(np.uint32), act.view(np.uint32))
