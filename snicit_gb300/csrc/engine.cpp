@@ -182,8 +182,8 @@ struct sdnn_engine {
   int32_t* d_mcounts = nullptr;        // [L + 4] ... and their number
   uint32_t mmask = 0;
   bool bits_on = false;            // layer 0 of 0/1 inputs by counting
-  bool slot = false;               // one of several of a server
-  int share = 1;                   // engines that work side by side now (servers)
+  bool shares = false;             // a server's pass beside others (resident launches take a share)
+  int share = 1;                   // ... of the SMs: one in so many
   bool bit_rows = false;           // ... from d_inbits (the call's rows came as bits)
 
   cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -220,9 +220,9 @@ struct sdnn_engine {
 
   // graph cache: one captured graph per phase of an inference (slots 5 and 6:
   // PH_ALL and PH_PRE starting after the layers run piece by piece, 7 and 8: from
-  // rows that came as bits)
-  GraphSlot graphs[9];
-  FullGraph full[3];       // SNICIT whole-inference graphs (pipe_start 0 / > 0, bit rows)
+  // rows that came as bits, 9 to 13: of passes that share the SMs)
+  GraphSlot graphs[14];
+  FullGraph full[4];       // SNICIT whole-inference graphs (pipe_start 0 / > 0, bit rows, sharing)
   bool full_off = false;   // building one failed: the host picks the post path
   bool in_body = false;    // capturing a conditional body (no event records)
   int last_full = 0;       // 1 + slot of the whole-inference graph that ran last, 0: none
@@ -974,7 +974,7 @@ int layer_launch(sdnn_engine* e, int l, int epi, const float* in, float* out, co
   a.list_in = lin;
   a.count_in = cin;
   a.hint = hint;
-  a.share = e->slot ? e->d_rows + 1 : nullptr;
+  a.share = e->shares ? e->d_rows + 1 : nullptr;
   a.list_out = lout;
   a.count_out = cout;
   a.stamp = e->d_stamp;
@@ -1400,7 +1400,7 @@ int run_phase(sdnn_engine* e, int slot, int phase, int64_t rows, const float* d_
   }
   const bool reads_in = phase == PH_ALL || phase == PH_PRE;
   const bool streamed = e->pipe_start > 0 && reads_in, bit_rows = e->bit_rows && reads_in;
-  GraphSlot& g = e->graphs[streamed ? 5 + slot : bit_rows ? 7 + slot : slot];
+  GraphSlot& g = e->graphs[streamed ? 5 + slot : bit_rows ? 7 + slot : e->shares ? 9 + slot : slot];
   const GraphKey key{0, reads_in ? d_in : nullptr, d_flags, effective_threshold(e),
                      std::max(1, e->cfg.num_centroids), e->cfg.mode, e->key.T, e->threads,
                      phase == PH_POST_CHAIN ? e->chain_kc * 4 + e->chain_kind : 0,
@@ -1556,7 +1556,7 @@ int build_full_graph(sdnn_engine* e, FullGraph& fg, int64_t rows, const float* d
 // SDNN_ERR_UNSUPPORTED when the graph cannot be built (the caller then lets
 // the host choose the post-threshold path, for this and every later call).
 int run_full(sdnn_engine* e, int64_t rows, const float* d_in, int32_t* d_flags) {
-  const int slot = e->pipe_start > 0 ? 1 : e->bit_rows ? 2 : 0;
+  const int slot = e->pipe_start > 0 ? 1 : e->bit_rows ? 2 : e->shares ? 3 : 0;
   FullGraph& fg = e->full[slot];
   const GraphKey key{0, d_in, d_flags, effective_threshold(e), std::max(1, e->cfg.num_centroids), e->cfg.mode,
                      e->key.T, e->threads, 0, e->pipe_start};
@@ -2596,9 +2596,11 @@ float* engine_input(sdnn_engine* e) { return e->d_in; }
 int32_t* engine_flags(sdnn_engine* e) { return e->d_flags; }
 // One of several slots: `at_work` of them run now.  Passes of few tiles per CTA
 // share the SMs, as one alone would wait for round trips most of the time; from
-// 8 rounds of tiles on a pass takes them all.
-int engine_run(sdnn_engine* e, int64_t rows, int slots, int at_work) {
-  e->slot = slots > 1;
+// 8 rounds of tiles on a pass takes them all.  A pass that finds no other at work
+// runs as on an engine of its own, launches overlapped: a lone row on a server of
+// 4 slots of 1024 neurons 150 us, 204 with the launches of a pass that shares.
+int engine_run(sdnn_engine* e, int64_t rows, int at_work) {
+  e->shares = at_work > 1;
   const int64_t all = std::max<int64_t>(1, 8ll * 8 * e->num_sms / std::max<int64_t>(1, rows));
   e->share = (int)std::clamp<int64_t>(all, 1, std::max(1, at_work));
   return run(e, rows, e->d_in, e->d_flags);

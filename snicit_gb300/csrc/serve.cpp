@@ -46,7 +46,7 @@ sdnn_config engine_config(const sdnn_engine* e);
 cudaStream_t engine_stream(const sdnn_engine* e);
 float* engine_input(sdnn_engine* e);
 int32_t* engine_flags(sdnn_engine* e);
-int engine_run(sdnn_engine* e, int64_t rows, int slots, int at_work);
+int engine_run(sdnn_engine* e, int64_t rows, int at_work);
 int engine_check(sdnn_engine* e);
 std::vector<int32_t> engine_final_positions(const sdnn_engine* e);
 bool engine_head(sdnn_engine* e, const float* Hp, const float* hb, int32_t H, int64_t rows,
@@ -184,7 +184,7 @@ void run_pass(sdnn_server* sv, Slot& slot) {
   if (cudaMemcpyAsync(sdnn::engine_input(e), slot.h_in, sizeof(float) * (size_t)total * N,
                       cudaMemcpyHostToDevice, s) != cudaSuccess)
     rc = SDNN_ERR_CUDA;
-  if (rc == SDNN_OK) rc = sdnn::engine_run(e, total, (int)sv->slots.size(), at_work);
+  if (rc == SDNN_OK) rc = sdnn::engine_run(e, total, at_work);
   if (rc == SDNN_OK && H > 0 &&
       !sdnn::engine_head(e, sv->d_head, sv->d_hb, H, total, slot.d_logits, slot.d_argmax))
     rc = SDNN_ERR_UNSUPPORTED;
