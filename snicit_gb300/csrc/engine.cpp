@@ -529,11 +529,6 @@ int ensure_buffers(sdnn_engine* e, int64_t rows) {
   // grid chain rows: a fresh buffer per layer (wide layouts only, where it runs)
   if (e->N >= 16384) T(A(&e->d_gscratch, grid_chain_scratch_floats(e->L, e->nq, e->Q) * 4));
   T(A(&e->d_gbar, 16));
-  if (bits_possible(e)) {
-    const size_t tiles = (size_t)(cap + 31) / 32;
-    T(A(&e->d_bits, tiles * (size_t)N * 4));
-    T(A(&e->d_tile_state, tiles * 4));
-  }
   {
     uint64_t P = 1024;
     while (P < 2 * (uint64_t)cap) P <<= 1;
@@ -556,6 +551,17 @@ int ensure_buffers(sdnn_engine* e, int64_t rows) {
     free_buffers(e);
     cudaGetLastError();
     return fail(e, SDNN_ERR_OOM, std::string("device allocation failed: ") + cudaGetErrorString(rc));
+  }
+  // last, and only where there is room: without the bit words of a binary first
+  // layer (1 % of the rows) that layer runs on the float kernels
+  if (bits_possible(e)) {
+    const size_t tiles = (size_t)(cap + 31) / 32;
+    if (A(&e->d_bits, tiles * (size_t)N * 4) != cudaSuccess ||
+        A(&e->d_tile_state, tiles * 4) != cudaSuccess) {
+      cudaGetLastError();
+      dfree(e->d_bits);
+      dfree(e->d_tile_state);
+    }
   }
   e->cap = cap;
   CK(cudaMemsetAsync(e->d_ctl, 0, (size_t)e->ctl_size * 4, e->stream));
@@ -1693,8 +1699,9 @@ int prepare(sdnn_engine* e, int64_t rows) {
     if (e->sparse_built) CK(sparse_residue_prepare(e->N));
     e->kernels_ready = true;
   }
-  e->bits_on = bits_possible(e) && !(e->cfg.flags & SDNN_FLAG_NO_BINARY_FIRST_LAYER);
-  return ensure_buffers(e, rows);
+  rc = ensure_buffers(e, rows);
+  e->bits_on = e->d_bits && e->d_tile_state && !(e->cfg.flags & SDNN_FLAG_NO_BINARY_FIRST_LAYER);
+  return rc;
 }
 
 // The error word among the counters read back last.
@@ -2148,7 +2155,19 @@ int infer_host(sdnn_engine* e, const float* Y0, const uint64_t* bits, int64_t ro
   const int64_t W = (N + 63) / 64;
   if (bits && e->inbits_cap < e->cap) {
     dfree(e->d_inbits);
-    CK(cudaMalloc((void**)&e->d_inbits, (size_t)e->cap * W * 8));
+    e->inbits_cap = 0;
+    const size_t bytes = (size_t)e->cap * W * 8;
+    cudaError_t ce = cudaMalloc((void**)&e->d_inbits, bytes);
+    if (ce == cudaErrorMemoryAllocation && e->d_bits) {
+      // the bit words of the first layer give way
+      cudaGetLastError();
+      drop_graph(e);
+      dfree(e->d_bits);
+      dfree(e->d_tile_state);
+      e->bits_on = false;
+      ce = cudaMalloc((void**)&e->d_inbits, bytes);
+    }
+    CK(ce);
     e->inbits_cap = e->cap;
   }
   int64_t total = 0;

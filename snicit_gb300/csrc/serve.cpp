@@ -370,9 +370,10 @@ int sdnn_server_create(sdnn_engine* model, const sdnn_server_config* cfg, const 
     delete sv;
     return SDNN_ERR_CUDA;
   }
-  // device bytes per row of a slot: input and its bit words, two layer buffers (the
-  // materialise scratch is one of them), row lists/state (~64 B), logits
-  sv->per_row = (int64_t)sv->N * 4 * 3 + sv->N / 8 + 64 + (int64_t)sv->H * 4;
+  // device bytes per row of a slot: input, two layer buffers (the materialise
+  // scratch is one of them), row lists/state (~64 B), logits (the input's bit
+  // words, 1 % more, are taken where there is room)
+  sv->per_row = (int64_t)sv->N * 4 * 3 + 64 + (int64_t)sv->H * 4;
   sv->cap = cfg->max_rows > 0 ? std::min<int64_t>(cfg->max_rows, 1 << 20) : (1 << 20);
   sv->model = model;
   sdnn_config ec = mc;

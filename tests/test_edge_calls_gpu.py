@@ -161,3 +161,44 @@ def test_layers_that_no_row_reaches(N, mode):
         flags, _ = e.infer(Y)
         assert np.array_equal(flags, want)
         assert np.array_equal(e.activations(rows).view(np.uint32), act.view(np.uint32))
+
+
+@pytest.mark.parametrize("as_bits", [False, True])
+def test_rows_fit_a_full_device_without_the_bit_words(as_bits):
+    """A device with room for all of an engine's buffers but the bit words of
+    the binary first layer (and, for rows that come as bits, of those): the rows
+    run all the same, with the same results."""
+    torch = pytest.importorskip("torch")
+    N, rows = 16384, 8192
+    bits = rows // 32 * N * 4
+    Y = np.zeros((rows, N), np.float32)
+    Y[:64] = sg.generate_inputs(N, 4, 0, 64)
+
+    def run():
+        with sg.Engine(N, 2, mode="SNIG", batch=rows, bias=-0.3, streamed_input=False) as e:
+            e.generate_weights(4)
+            flags, _ = e.infer(Y)
+            act = e.activations(64)
+            if not as_bits:
+                return flags, act, flags, torch.cuda.mem_get_info()[0]
+            f2, _ = e.infer_bits(sg.pack_bits(Y[:70]))
+            return flags, act, f2, torch.cuda.mem_get_info()[0]
+
+    torch.zeros(1, device="cuda")
+    run()  # (kernels and the context are loaded)
+    before = torch.cuda.mem_get_info()[0]
+    want = run()
+    used = before - want[3]
+    leave = used - bits // 2
+    filler = []
+    for keep in (256 << 20, 0):  # (sizes that the allocator passes on as they are)
+        room = torch.cuda.mem_get_info()[0] - leave - keep
+        filler.append(torch.empty(room // (2 << 20) * (2 << 20), dtype=torch.uint8, device="cuda"))
+    if not leave <= torch.cuda.mem_get_info()[0] < leave + (4 << 20):
+        pytest.skip("free device memory cannot be set this closely here")
+    got = run()
+    del filler
+    torch.cuda.empty_cache()
+    for a, b in zip(want[:3], got[:3]):
+        assert np.array_equal(np.ascontiguousarray(a).view(np.uint32), np.ascontiguousarray(b).view(np.uint32))
+    assert want[0].any()
