@@ -285,6 +285,12 @@ int sdnn_load_packed_weights(sdnn_engine* e, const char* path);
  * out as it must; the engine stays usable afterwards. */
 int sdnn_selftest_wait_timeout(sdnn_engine* e, int64_t limit_us);
 
+/* Self-test of passes that share the SMs (no reference counterpart): the
+ * following inferences of this engine take one in `share` of the SMs, like a
+ * server's pass beside share - 1 others (share >= 1; 0: as an engine of its
+ * own again).  Results do not depend on it. */
+int sdnn_selftest_share(sdnn_engine* e, int32_t share);
+
 /* Switches the mode (and threshold) of an engine without repacking its
  * weights, e.g. to time the plain path and SNICIT on one resident copy of W.
  * (The reference picks the engine class once, main/SDGC.cu:104-110.) */

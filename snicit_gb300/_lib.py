@@ -111,6 +111,7 @@ SIGNATURES = [
     ("sdnn_set_mode", ctypes.c_int, [P, I32, I32]),
     ("sdnn_set_input_streaming", ctypes.c_int, [P, I32]),
     ("sdnn_selftest_wait_timeout", ctypes.c_int, [P, I64]),
+    ("sdnn_selftest_share", ctypes.c_int, [P, I32]),
     ("sdnn_save_packed_weights", ctypes.c_int, [P, ctypes.c_char_p]),
     ("sdnn_load_packed_weights", ctypes.c_int, [P, ctypes.c_char_p]),
     ("sdnn_layer_noalloc", ctypes.c_int, [P, I32, P, P, I64, P, P]),

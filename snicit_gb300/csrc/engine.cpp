@@ -2451,6 +2451,13 @@ int sdnn_selftest_wait_timeout(sdnn_engine* e, int64_t limit_us) {
   return check_device_error(e);  // SDNN_ERR_TIMEOUT expected; resets the error word
 }
 
+int sdnn_selftest_share(sdnn_engine* e, int32_t share) {
+  if (!e || share < 0) return SDNN_ERR_INVALID;
+  e->shares = share > 0;
+  e->share = std::max(1, share);
+  return SDNN_OK;
+}
+
 int sdnn_set_mode(sdnn_engine* e, int32_t mode, int32_t threshold) {
   if (!e || mode < SDNN_MODE_BF || mode > SDNN_MODE_SNICIT || threshold < 0) return SDNN_ERR_INVALID;
   e->cfg.mode = mode;

@@ -202,3 +202,72 @@ def test_rows_fit_a_full_device_without_the_bit_words(as_bits):
     for a, b in zip(want[:3], got[:3]):
         assert np.array_equal(np.ascontiguousarray(a).view(np.uint32), np.ascontiguousarray(b).view(np.uint32))
     assert want[0].any()
+
+
+@pytest.mark.parametrize("N", [1024, 4096, 49152])
+@pytest.mark.parametrize("degree", [63, 64, 120])
+def test_counting_at_the_limits_of_its_planes(N, degree):
+    """A binary first layer whose largest in-degree is the last that six planes
+    hold, the first that needs seven, and near the most that is counted: rows of
+    ones reach that count, and every output is that of the float kernels."""
+    rng = np.random.default_rng([N, degree])
+    far = np.arange(0, N, 37)  # these outputs have `degree` edges, the others 9
+    n = np.full(N, 9)
+    n[far] = degree
+    cols = np.repeat(np.arange(N), n)
+    ins = np.concatenate([rng.permutation(N // 32)[np.arange(k) // 32] * 32 + np.arange(k) % 32
+                          for k in n])  # an output's inputs take the banks in turn
+    rows = 75
+    Y = (rng.random((rows, N)) < np.linspace(0, 1, rows)[:, None]).astype(np.float32)
+    Y[-2:] = 1
+    got = []
+    for counts in (True, False):
+        with sg.Engine(N, 1, mode="SNIG", batch=rows, bias=-1.4, binary_first_layer=counts,
+                       placement=False) as e:
+            e.set_layer_coo(0, ins, cols, np.full(len(ins), 0.0625, np.float32))
+            flags, _ = e.infer(Y)
+            got.append((flags, e.activations(rows), e.stats()["launches"]))
+            if counts:
+                f2, _ = e.infer_bits(sg.pack_bits(Y))
+                assert np.array_equal(f2, flags)
+                assert np.array_equal(e.activations(rows).view(np.uint32), got[0][1].view(np.uint32))
+    assert got[0][2] > got[1][2]  # the counting kernels ran
+    assert np.array_equal(got[0][0], got[1][0])
+    assert np.array_equal(got[0][1].view(np.uint32), got[1][1].view(np.uint32))
+    assert got[0][1][-1].max() == np.float32(degree * 0.0625) + np.float32(-1.4)
+
+
+@pytest.mark.parametrize("N,nnz,values,L,K", [
+    (1024, 32, False, 70, 1), (1024, 3, False, 35, 3),
+    (1024, 80, False, 40, 8),   # lists longer than one batch of 16 blocks
+    (1024, 50, True, 36, 2),    # ... than one of 8 with their values
+    (4096, 32, False, 67, 1), (4096, 32, False, 10, 4), (4096, 20, True, 36, 1),
+    (16384, 20, False, 40, 1),  # one weight buffer
+])
+def test_streamed_chain_carries_every_centroid(N, nnz, values, L, K):
+    """K prototypes far apart, four copies of each: they are the centroids, no
+    residue is left, and the streamed chain runs the layers after the threshold,
+    with the bits of a launch per layer and of the chain that reads weights from
+    L2."""
+    rng = np.random.default_rng([N, nnz, K])
+    width = N // nnz
+    c = (rng.integers(0, width, (N, nnz)) + np.arange(nnz) * width).reshape(-1)
+    r = np.repeat(np.arange(N), nnz)
+    v = np.abs(rng.standard_normal(N * nnz)).astype(np.float32) if values else np.ones(N * nnz, np.float32)
+    v *= np.float32(0.9 / (nnz * v.mean()))
+    protos = np.stack([np.where(rng.random(N) < 0.5, rng.random(N) * 3 * (k + 1), 0)
+                       for k in range(K)]).astype(np.float32)
+    Y = np.tile(protos, (4, 1))
+    out = []
+    for kw, kernel in (({}, 3), ({"chain_stream": False}, 2), ({"chain": False}, 1)):
+        with sg.Engine(N, L, mode="SNICIT", threshold=3, batch=4 * K, bias=0.1, num_centroids=50,
+                       merge_start=1, **kw) as e:
+            for l in range(L):
+                e.set_layer_coo(l, r, c, v)
+            flags, _ = e.infer(Y)
+            st = e.stats()
+            assert (st["residue_rows"], st["centroids"], st["post_kernel"]) == (0, K, kernel), st
+            out.append((flags, e.activations(4 * K)))
+    for flags, act in out[1:]:
+        assert np.array_equal(flags, out[0][0])
+        assert np.array_equal(act.view(np.uint32), out[0][1].view(np.uint32))

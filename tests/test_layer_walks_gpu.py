@@ -93,3 +93,27 @@ def _same_rows(N, nnz, values, shapes, counts):
         b = float(np.float32(bias))
         bound = (n + 2) * 2.0 ** -24 * (A + abs(b))
         assert np.all(np.abs(got[0][1][some] - np.clip(S + b, 0, 32)) <= bound)
+
+
+@pytest.mark.parametrize("N,values", [(1024, False), (1024, True), (1568, True), (3072, False),
+                                      (4096, False), (4096, True)])
+def test_shares_of_the_sms_change_no_bit(N, values):
+    """Passes that take one in 1, 2, 3, 16 or (no CTA left over) 1000 of the SMs,
+    few rows and several rounds of tiles, in both modes; launches without rows
+    among them."""
+    r, c, v = _net(N, 24, values, 14)
+    rng = np.random.default_rng(N)
+    Y = np.where(rng.random((900, N)) < 0.4, rng.random((900, N)) * 3, 0).astype(np.float32)
+    Y[::7] = 0
+    for mode in ("SNIG", "SNICIT"):
+        with sg.Engine(N, 6, mode=mode, threshold=4, batch=900, bias=-0.1) as e:
+            for l in range(6):
+                e.set_layer_coo(l, r, c, v)
+            for rows in (1, 2, 40, 333, 900):
+                want, _ = e.infer(Y[:rows])
+                act = e.activations(rows)
+                for share in (1, 2, 3, 16, 1000, 0):
+                    assert sg.load().sdnn_selftest_share(e._h, share) == 0
+                    flags, _ = e.infer(Y[:rows])
+                    assert np.array_equal(flags, want), (mode, rows, share)
+                    assert np.array_equal(e.activations(rows).view(np.uint32), act.view(np.uint32))
