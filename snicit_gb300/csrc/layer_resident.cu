@@ -200,6 +200,31 @@ __device__ __forceinline__ uint32_t plain_outputs(const float (&acc)[T], const L
   return m;
 }
 
+// ... in residue mode: every row's pre-activation is on its way before the first
+// is used (each is two loads, one after the other, and a CTA has its SM's only
+// 16 warps).  14 post layers of some 21000 residue rows of 1024 neurons
+// 2533 -> 2078 us (2416 with lists streamed per tile, of which 48 warps share an
+// SM).
+template <int T>
+__device__ __forceinline__ uint32_t residue_outputs(const float (&acc)[T], const LayerArgs& a,
+                                                    const int32_t* rows, int nrows, int g, int lane) {
+  const int c = g * 32 + lane;
+  float pc[T];
+#pragma unroll
+  for (int t = 0; t < T; ++t)
+    pc[t] = t < nrows ? a.pre_in[(size_t)a.cslot[rows[t]] * a.N + c] : 0.f;
+  uint32_t m = 0;
+#pragma unroll
+  for (int t = 0; t < T; ++t) {
+    if (t < nrows) {
+      const float y = clampf(pc[t] + acc[t], a.clampv) - clampf(pc[t], a.clampv);
+      a.y_out[(size_t)rows[t] * a.N + c] = y;
+      if (y != 0.f) m |= 1u << t;
+    }
+  }
+  return m;
+}
+
 // One warp's groups over the rows of a stage; returns the lane's row mask.
 template <int T, int RSW, bool CONSTW>
 __device__ __forceinline__ uint32_t run_groups(const LayerArgs& a, const float* ys, int RS,
@@ -230,8 +255,9 @@ __device__ __forceinline__ uint32_t run_groups(const LayerArgs& a, const float* 
       if constexpr (!CONSTW) vv = __ldg(a.w.val + at);
       apply_block<T, RSW, CONSTW>(acc, iv, vv, a.w.wconst, ys, RS, min(4, list.y - s));
     }
-    m |= plain ? plain_outputs<T>(acc, a, dst, g, lane)
-               : epilogue_group<T>(acc, a, rows, nrows, g, lane);
+    if (plain) m |= plain_outputs<T>(acc, a, dst, g, lane);
+    else if (a.epi == EPI_RESIDUE) m |= residue_outputs<T>(acc, a, rows, nrows, g, lane);
+    else m |= epilogue_group<T>(acc, a, rows, nrows, g, lane);
     g += (i & 1) ? step1 : step0;
   }
   return m;
@@ -552,10 +578,11 @@ ResidentPlan resident_plan(int N, bool constw, int max_depth, int num_sms) {
   // width that fills the warps' turns, lists streamed per tile are faster for
   // many rows (60000 rows, us, streamed against kept: 1056 neurons with values
   // 411 against 507, 1088 429 against 477; 2080 with one value 660 against 707,
-  // but 1056 361 against 363).  Up to 4096 rows they are level or slower (300
-  // rows, 40 layers: 366 against 303).
+  // with values 719 against 751; 1056 with one value 361 against 363, but its
+  // residue layers 2543 against 2631).  Up to 4096 rows they are level or slower
+  // (300 rows, 40 layers: 366 against 303).
   const int turns = p.split * kWarps * ((G + p.split * kWarps - 1) / (p.split * kWarps));
-  if (G < (constw ? 0.68 : 0.55) * turns) p.most_rows = 4096;
+  if (G < 0.7 * turns) p.most_rows = 4096;
   p.few = few_rows(p, N, constw, num_sms);
   return p;
 }

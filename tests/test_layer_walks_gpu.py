@@ -117,3 +117,30 @@ def test_shares_of_the_sms_change_no_bit(N, values):
                     flags, _ = e.infer(Y[:rows])
                     assert np.array_equal(flags, want), (mode, rows, share)
                     assert np.array_equal(e.activations(rows).view(np.uint32), act.view(np.uint32))
+
+
+@pytest.mark.parametrize("N,values", [(1024, False), (1024, True), (1568, True), (2400, False),
+                                      (4096, False), (4096, True)])
+def test_residue_layers_on_either_kernel(N, values):
+    """Rows that keep residues to the end (no merging), full and part-filled
+    tiles: the kernel with kept lists and the one with lists per tile give the
+    same activations, centroids and residue rows."""
+    r, c, v = _net(N, 24, values, 15)
+    v = np.abs(v)
+    v *= np.float32(1.1 / (24 * v.mean()))
+    rng = np.random.default_rng(N)
+    Y = np.where(rng.random((700, N)) < 0.4, rng.random((700, N)) * 3, 0).astype(np.float32)
+    for rows in (40, 700):
+        out = []
+        for kw in ({}, {"tile_rows": 8 if N < 2400 else 4, "threads": 512}):
+            with sg.Engine(N, 5, mode="SNICIT", threshold=2, batch=rows, bias=-0.05, merge=False,
+                           sparse_residue=False, num_centroids=4, **kw) as e:
+                for l in range(5):
+                    e.set_layer_coo(l, r, c, v)
+                flags, _ = e.infer(Y[:rows])
+                st = e.stats()
+                assert st["residue_rows"] > rows // 3 and st["post_kernel"] == 1
+                out.append((flags, e.activations(rows), e.layer_rows()))
+        for a, b in zip(*out):
+            assert np.array_equal(np.ascontiguousarray(a).view(np.uint32),
+                                  np.ascontiguousarray(b).view(np.uint32))
