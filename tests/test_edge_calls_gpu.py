@@ -271,3 +271,36 @@ def test_streamed_chain_carries_every_centroid(N, nnz, values, L, K):
     for flags, act in out[1:]:
         assert np.array_equal(flags, out[0][0])
         assert np.array_equal(act.view(np.uint32), out[0][1].view(np.uint32))
+
+
+@pytest.mark.parametrize("N,rows", [(256, 6200), (1024, 5300), (1056, 300)])
+def test_split_of_many_residue_rows(N, rows):
+    """Residue rows of 1 to 4 times as many nonzeros as a list holds (and, for the
+    larger counts, more rows than the split gives a CTA each): as many become
+    lists as must, whichever row is the centroid, and all keep their values."""
+    cap = max(32, N // 32)
+    rng = np.random.default_rng(N)
+    Y = np.tile(rng.integers(1, 200, N).astype(np.float32) / 64, (rows, 1))
+    k = rng.integers(0, 4 * cap + 1, rows)  # row r differs from a row s in |k[r] - k[s]| entries
+    Y[np.arange(N) < k[:, None]] += np.float32(1 / 256)
+    Y = np.ascontiguousarray(Y[:, rng.permutation(N)])
+    apart = np.abs(k[:, None] - np.arange(4 * cap + 1))
+    expected = list(zip((apart > 0).sum(axis=0), ((apart > 0) & (apart <= cap)).sum(axis=0)))
+    out = []
+    for sparse in (True, False):
+        with sg.Engine(N, 3, mode="SNICIT", threshold=1, batch=rows, bias=0.0, merge=False,
+                       num_centroids=1, sparse_residue=sparse) as e:
+            for l in range(3):
+                e.set_layer_coo(l, *_identity(N, 1.0))
+            flags, _ = e.infer(Y)
+            st = e.stats()
+            out.append((flags, e.activations(rows), list(e.layer_rows())))
+            lists = st["sparse_residue_rows"]
+            if sparse:
+                assert (st["residue_rows"], lists) in expected, (st, k[:5])
+                assert 0 < lists < st["residue_rows"] and st["sparse_row_layers"] == 2 * lists
+    want = Y
+    for flags, act, _ in out:
+        assert flags.all()
+        assert np.array_equal(act, want)
+    assert out[0][2] == out[1][2]
