@@ -203,7 +203,7 @@ __device__ __forceinline__ uint32_t plain_outputs(const float (&acc)[T], const L
 // ... in residue mode: every row's pre-activation is on its way before the first
 // is used (each is two loads, one after the other, and a CTA has its SM's only
 // 16 warps).  14 post layers of some 21000 residue rows of 1024 neurons
-// 2533 -> 2078 us (2416 with lists streamed per tile, of which 48 warps share an
+// 2533 -> 1955 us (2416 with lists streamed per tile, of which 48 warps share an
 // SM).
 template <int T>
 __device__ __forceinline__ uint32_t residue_outputs(const float (&acc)[T], const LayerArgs& a,
@@ -225,14 +225,16 @@ __device__ __forceinline__ uint32_t residue_outputs(const float (&acc)[T], const
   return m;
 }
 
-// One warp's groups over the rows of a stage; returns the lane's row mask.
-template <int T, int RSW, bool CONSTW>
+// One warp's groups over the rows of a stage; returns the lane's row mask.  (A
+// loop of its own in residue mode: as a branch in the one loop it cost plain
+// layers 1 %.)
+template <int T, int RSW, bool CONSTW, bool RESIDUE>
 __device__ __forceinline__ uint32_t run_groups(const LayerArgs& a, const float* ys, int RS,
                                                const int32_t* rows, int nrows, uint32_t col,
                                                Batch<CONSTW>& cur, const int2* lists, int first_grp,
                                                int step0, int step1, int n, int lane) {
   constexpr int kHeld = 4 * kResBlocks<CONSTW>;
-  const bool plain = a.epi == EPI_PLAIN && nrows == T;
+  const bool plain = !RESIDUE && a.epi == EPI_PLAIN && nrows == T;
   float* dst[T];
 #pragma unroll
   for (int t = 0; t < T; ++t) dst[t] = plain ? a.y_out + (size_t)rows[t] * a.N : nullptr;
@@ -255,9 +257,11 @@ __device__ __forceinline__ uint32_t run_groups(const LayerArgs& a, const float* 
       if constexpr (!CONSTW) vv = __ldg(a.w.val + at);
       apply_block<T, RSW, CONSTW>(acc, iv, vv, a.w.wconst, ys, RS, min(4, list.y - s));
     }
-    if (plain) m |= plain_outputs<T>(acc, a, dst, g, lane);
-    else if (a.epi == EPI_RESIDUE) m |= residue_outputs<T>(acc, a, rows, nrows, g, lane);
-    else m |= epilogue_group<T>(acc, a, rows, nrows, g, lane);
+    if constexpr (RESIDUE)
+      m |= residue_outputs<T>(acc, a, rows, nrows, g, lane);
+    else
+      m |= plain ? plain_outputs<T>(acc, a, dst, g, lane)
+                 : epilogue_group<T>(acc, a, rows, nrows, g, lane);
     g += (i & 1) ? step1 : step0;
   }
   return m;
@@ -274,8 +278,11 @@ __device__ __forceinline__ uint32_t run_stage(int TE, const LayerArgs& a, const 
       return run_stage<pow2_below(T), RSW, CONSTW>(TE, a, ys, RS, rows, nrows, col, cur, lists, first_grp,
                                            step0, step1, n, lane);
   }
-  return run_groups<T, RSW, CONSTW>(a, ys, RS, rows, nrows, col, cur, lists, first_grp, step0, step1,
-                                    n, lane);
+  if (a.epi == EPI_RESIDUE)
+    return run_groups<T, RSW, CONSTW, true>(a, ys, RS, rows, nrows, col, cur, lists, first_grp, step0,
+                                            step1, n, lane);
+  return run_groups<T, RSW, CONSTW, false>(a, ys, RS, rows, nrows, col, cur, lists, first_grp, step0,
+                                           step1, n, lane);
 }
 
 template <int T, int RSW, bool CONSTW>
