@@ -157,7 +157,7 @@ int tune(sdnn_engine* e, const Sample& smp, const char* record_path) {
     if (merge_on && bs.ms < 1e30f) {
       // first layer after which identical rows are merged: early merging finds
       // duplicates sooner, late merging skips hashing rows that are all distinct;
-      // and the spacing of the later merge steps (each costs three launches)
+      // and the spacing of the later merge steps (each costs two launches)
       Trial bm = bs;
       int best_every = cfg0.merge_every;
       for (int every : {1, 2, 4, 8}) {

@@ -403,8 +403,8 @@ int choose_kernel(sdnn_engine* e) {
     if (req_T > 0 && k.T != req_T) continue;
     const size_t smem = (size_t)k.T * (size_t)(e->Q + 32) * 4;
     if (smem > kMaxSmem) continue;
-    // a tile that leaves room for one CTA per SM wants all its warps: 6000 rows
-    // of 16384 neurons took 832 us with 512 threads (T = 2), 572 with 1024 (T = 3)
+    // a tile that leaves room for one CTA per SM wants all its warps: 3000 rows
+    // of 16384 neurons take 427 us with 512 threads (T = 2), 282 with 1024 (T = 3)
     if (e->cfg.threads == 0 && k.kg == 1) threads = smem > kMaxSmem / 2 ? 1024 : 512;
     LayerKernelKey kc = k, kg = k;
     kc.constw = true;
@@ -515,7 +515,7 @@ int ensure_buffers(sdnn_engine* e, int64_t rows) {
   T(A(&e->d_pre, (size_t)K * N * 4));
   T(A(&e->d_fallback, (size_t)cap * 4));
   if (e->sparse_built) {
-    // a sparse row's update runs on one warp, entry after entry: rows with
+    // a sparse row's scatter runs on one warp, entry after entry: rows with
     // more than N / 32 nonzeros stay dense (the gather kernel's throughput)
     e->sp_cap = std::max(32, e->N / 32);
     for (int i = 0; i < 2; ++i) {
@@ -1625,8 +1625,8 @@ int run(sdnn_engine* e, int64_t rows, const float* d_in, int32_t* d_flags) {
               centroids = e->host(e->d_ccount)[0];
     e->report_valid = false;  // (the post-threshold layers are still to come)
     // no residue left: one chain launch carries the centroid rows -- the
-    // cluster kernel where the rows fit shared memory (measured faster: 1.6
-    // and 7.2 us per layer at N = 4096 and 16384 against 13.8 and 11.8 for the
+    // cluster kernel where the rows fit shared memory (measured faster: 1.0
+    // and 4.2 us per layer at N = 4096 and 16384 against 13.8 and 11.8 for the
     // grid kernel), else the grid kernel
     int kind = 0, variant = 0;
     if (residues == 0 && centroids >= 1 && !(e->cfg.flags & SDNN_FLAG_NO_CHAIN)) {

@@ -30,10 +30,13 @@
 //    stream of an inference, of 4096 12.0 -> 5.4; 60 layers of 2048 with 600
 //    rows at first 717 -> 573.
 //
-// One layer, us with lists streamed per tile (best tile) -> kept: 60000 rows of
-// 1024 neurons 334 -> 290, of 4096 1292 -> 1119 (the gathers alone need 239
-// and 956 at one wavefront per clock); 3001 rows of 4096 with values 104 -> 93.
-// The port is then 85 % busy, tile copies and stores included.
+// One layer through the one-layer entry point, us with lists streamed per tile
+// (best tile) -> kept: 60000 rows of 1024 neurons 307 -> 299, of 4096 1240 ->
+// 1116, of 2048 651 -> 531 (the gathers alone need 239, 956 and 478 at one
+// wavefront per clock).  The port is then 85 % busy, tile copies and stores
+// included.  With a value per edge the two are level for many rows (1024: 333 ->
+// 346, 4096: 1427 -> 1457) and the kept lists ahead in layer after layer of a few
+// hundred (40 of 300 rows of 1536: 416 -> 301).
 #include <algorithm>
 #include <climits>
 #include <cstdint>
